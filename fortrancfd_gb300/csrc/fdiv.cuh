@@ -24,6 +24,8 @@
 
 #include <cuda_runtime.h>
 
+#include "idiv.h"
+
 namespace gbmg {
 
 __device__ __forceinline__ int fdiv_exp(double x) {

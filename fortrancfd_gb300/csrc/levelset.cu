@@ -14,10 +14,24 @@
 // The faces are reconstructed once each (k_ls_faces, one thread per face,
 // both split parts), then k_ls_stage forms L(phi) per cell in the
 // reference's order and applies the stage.  All arithmetic is FP64 with every
-// product rounded on its own (no fused multiply-add), so the results equal
-// the FP64 oracle bit for bit.  GB300 runs FP64 at about 1/57 of its FP32
-// rate and a face costs two reconstructions of about 20 divisions each, so
-// these kernels are bound by the FP64 pipe, not by memory.
+// product rounded on its own (a fused multiply-add only where one factor is a
+// power of two, which rounds the same), so the results equal the FP64 oracle
+// bit for bit.  GB300's FP64 pipe runs at about 1/57 of its FP32 rate and
+// these kernels are bound by it, not by memory; what is kept off it:
+//   - every division and most multiplications: correctly rounded quotients and
+//     products in integer and FP32 arithmetic (idiv.h), one reciprocal per
+//     divisor;
+//   - what neighbouring faces share: the smoothness indicators and weights of
+//     a three-cell stencil are formed once per cell and handed along the line
+//     through shared memory, where they were formed once per face and side;
+//   - the side the flow does not come from: a split flux that is zero on a
+//     stencil has constant weights, and a face value of zeros is a zero.
+// Measured: a 256^3 advection step with a smooth velocity 92.8 -> 17.7 ms (with
+// the divisions alone off the pipe 22.9), one redistancing call of 13
+// iterations on 143x127x101 cells 139.0 -> 28.7 ms (37.1).  The face kernel
+// issues 46 FP64 warp instructions per 32 cells of a 128^3 case (about 355
+// before) and runs at 59% of the FP64 pipe and 46% of the issue slots: the
+// integer work that replaced the rest now takes about as long.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -26,118 +40,238 @@
 #include "gbmg.h"
 #include "fdiv.cuh"
 #include "gbmg_internal.h"
+#include "idiv.h"
 
 namespace gbmg {
 
 namespace {
 
-__device__ __forceinline__ double dsq(double x) { return __dmul_rn(x, x); }
 __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double dvd(double a, double b) { return __ddiv_rn(a, b); }
-// Quotients by the run-time spacing come from its correctly rounded
-// reciprocal without dividing (fdiv.cuh): the same doubles, cheaper where a
-// kernel divides by h often (the redistancing gradient: 6 per cell and
-// axis).  Divisions by literal constants and the WENO weights (a divisor
-// used three times, whose reciprocal would cost a division of its own) stay
-// IEEE divisions: measured faster so (advection step 96.5 against 106 ms).
-__device__ __forceinline__ double by3(double a) { return dvd(a, 3.0); }
-__device__ __forceinline__ double by6(double a) { return dvd(a, 6.0); }
-__device__ __forceinline__ double by12(double a) { return dvd(a, 12.0); }
+__device__ __forceinline__ double by3(double a) { return div_3(a, 0); }
+__device__ __forceinline__ double by6(double a) { return div_3(a, 1); }
+__device__ __forceinline__ double by12(double a) { return div_3(a, 2); }
 __device__ __forceinline__ double by4(double a) { return mul(a, 0.25); }  // exact
+// a + c b with c b exact (c a power of two): the sum's one rounding
+__device__ __forceinline__ double fma2(double c, double b, double a) { return __fma_rn(c, b, a); }
 
-// value at face i+1/2 of g(i-2..i+2) = g0..g4, biased to the left
-__device__ double weno_left(double g0, double g1, double g2, double g3, double g4, double eps) {
-  const double b1 = add(mul(13.0, dsq(add(sub(g0, mul(2.0, g1)), g2))),
-                        mul(3.0, dsq(add(sub(g0, mul(4.0, g1)), mul(3.0, g2)))));
-  const double b2 = add(mul(13.0, dsq(add(sub(g1, mul(2.0, g2)), g3))), mul(3.0, dsq(sub(g1, g3))));
-  const double b3 = add(mul(13.0, dsq(add(sub(g2, mul(2.0, g3)), g4))),
-                        mul(3.0, dsq(add(sub(mul(3.0, g2), mul(4.0, g3)), g4))));
-  const double a1 = dvd(1.0, dsq(add(eps, b1)));
-  const double a2 = dvd(6.0, dsq(add(eps, b2)));
-  const double a3 = dvd(3.0, dsq(add(eps, b3)));
-  const double s = add(add(a1, a2), a3);
-  const double w1 = dvd(a1, s), w2 = dvd(a2, s), w3 = dvd(a3, s);
-  double v = mul(by3(w1), g0);
-  v = sub(v, mul(by6(add(mul(7.0, w1), w2)), g1));
-  v = add(v, mul(by6(add(add(mul(11.0, w1), mul(5.0, w2)), mul(2.0, w3))), g2));
-  v = add(v, mul(by6(add(mul(2.0, w2), mul(5.0, w3))), g3));
-  v = sub(v, mul(by6(w3), g4));
+__device__ __forceinline__ double isq(double x) { return mul_int(x, x); }
+
+// eps + b1, eps + b2, eps + b3 squared for the three-cell stencil (ga, gb, gc):
+// the indicators of a left-biased face two cells to the right of ga (x[0]),
+// right of gb (x[1]) and left of gc (x[2]).  ta = 3 ga, tc = 3 gc.
+__device__ __forceinline__ void weno_stencil(double ga, double gb, double gc, double ta, double tc,
+                                             double eps, double (&x)[3]) {
+  const double d = mul_k<13>(isq(add(fma2(-2.0, gb, ga), gc)));
+  x[0] = isq(add(eps, add(d, mul_k<3>(isq(add(fma2(-4.0, gb, ga), tc))))));
+  x[1] = isq(add(eps, add(d, mul_k<3>(isq(sub(ga, gc))))));
+  x[2] = isq(add(eps, add(d, mul_k<3>(isq(add(fma2(-4.0, gb, ta), gc))))));
+}
+
+// value at face i+1/2 of g(i-2..i+2) = g0..g4, biased to the left, from the
+// unnormalised weights a1, a2, a3
+__device__ __forceinline__ double weno_left(double a1, double a2, double a3, double g0, double g1,
+                                            double g2, double g3, double g4) {
+  const RcpInt s = rcp_int(add(add(a1, a2), a3));
+  const double w1 = div_int(a1, s), w2 = div_int(a2, s), w3 = div_int(a3, s);
+  double v = mul_int(by3(w1), g0);
+  v = sub(v, mul_int(by6(add(mul_k<7>(w1), w2)), g1));
+  v = add(v, mul_int(by6(fma2(2.0, w3, add(mul_k<11>(w1), mul_k<5>(w2)))), g2));
+  v = add(v, mul_int(by6(fma2(2.0, w2, mul_k<5>(w3))), g3));
+  v = sub(v, mul_int(by6(w3), g4));
   return v;
 }
 
 // value at face i+1/2 of f(i-1..i+3) = f0..f4, biased to the right
-__device__ double weno_right(double f0, double f1, double f2, double f3, double f4, double eps) {
-  const double b3 = add(mul(13.0, dsq(add(sub(f0, mul(2.0, f1)), f2))),
-                        mul(3.0, dsq(add(sub(f0, mul(4.0, f1)), mul(3.0, f2)))));
-  const double b2 = add(mul(13.0, dsq(add(sub(f1, mul(2.0, f2)), f3))), mul(3.0, dsq(sub(f1, f3))));
-  const double b1 = add(mul(13.0, dsq(add(sub(f2, mul(2.0, f3)), f4))),
-                        mul(3.0, dsq(add(sub(mul(3.0, f2), mul(4.0, f3)), f4))));
-  const double a1 = dvd(1.0, dsq(add(eps, b1)));
-  const double a2 = dvd(6.0, dsq(add(eps, b2)));
-  const double a3 = dvd(3.0, dsq(add(eps, b3)));
-  const double s = add(add(a1, a2), a3);
-  const double w1 = dvd(a1, s), w2 = dvd(a2, s), w3 = dvd(a3, s);
-  double v = by6(mul(w3, add(add(-f0, mul(5.0, f1)), mul(2.0, f2))));
-  v = add(v, by6(mul(w2, sub(add(mul(2.0, f1), mul(5.0, f2)), f3))));
-  v = add(v, by6(mul(w1, add(sub(mul(11.0, f2), mul(7.0, f3)), mul(2.0, f4)))));
+__device__ __forceinline__ double weno_right(double a1, double a2, double a3, double f0, double f1,
+                                             double f2, double f3, double f4) {
+  const RcpInt s = rcp_int(add(add(a1, a2), a3));
+  const double w1 = div_int(a1, s), w2 = div_int(a2, s), w3 = div_int(a3, s);
+  double v = by6(mul_int(w3, fma2(2.0, f2, sub(mul_k<5>(f1), f0))));
+  v = add(v, by6(mul_int(w2, sub(fma2(2.0, f1, mul_k<5>(f2)), f3))));
+  v = add(v, by6(mul_int(w1, fma2(2.0, f4, sub(mul_k<11>(f2), mul_k<7>(f3))))));
   return v;
+}
+
+__device__ __forceinline__ bool is_zero(double x) {
+  return ((unsigned long long)__double_as_longlong(x) << 1) == 0ull;
+}
+// a zero as a float of the same sign
+__device__ __forceinline__ float zero_f(double x) {
+  return __int_as_float(__double2hiint(x) & (int)0x80000000);
+}
+__device__ __forceinline__ double zero_d(float z) {
+  return __hiloint2double(__float_as_int(z), 0);
+}
+// weno_left and weno_right of five zeros: a zero, its sign from the same sums
+__device__ __forceinline__ double weno_left_zero(double g0, double g1, double g2, double g3,
+                                                 double g4) {
+  return zero_d(__fsub_rn(
+      __fadd_rn(__fadd_rn(__fsub_rn(zero_f(g0), zero_f(g1)), zero_f(g2)), zero_f(g3)), zero_f(g4)));
+}
+__device__ __forceinline__ double weno_right_zero(double d0, double d1, double d2, double d3,
+                                                  double d4) {
+  const float f0 = zero_f(d0), f1 = zero_f(d1), f2 = zero_f(d2), f3 = zero_f(d3), f4 = zero_f(d4);
+  float v = __fadd_rn(__fadd_rn(-f0, f1), f2);
+  v = __fadd_rn(v, __fsub_rn(__fadd_rn(f1, f2), f3));
+  return zero_d(__fadd_rn(v, __fadd_rn(__fsub_rn(f2, f3), f4)));
 }
 
 __device__ __forceinline__ int clampi(int i, int n) { return i < 0 ? 0 : (i >= n ? n - 1 : i); }
 
 struct LsGrid {
   int nx, ny, nz;
-  double dx, dy, dz;
-  double rdx, rdy, rdz;  // RN(1/dx) ...; fast = 1 when all three allow div_known
-  int fast;
+  ConstDiv h[3];
 };
 
 LsGrid ls_grid(const gbmg_grid& g) {
-  LsGrid G{g.nx, g.ny, g.nz, g.dx, g.dy, g.dz, 1.0 / g.dx, 1.0 / g.dy, 1.0 / g.dz, 1};
-  G.fast = fdiv_divisor_ok(g.dx) && fdiv_divisor_ok(g.dy) && fdiv_divisor_ok(g.dz);
-  return G;
+  return LsGrid{g.nx, g.ny, g.nz, {const_div(g.dx), const_div(g.dy), const_div(g.dz)}};
 }
 
-// a / h along an axis with the reciprocal from the grid
-__device__ __forceinline__ double by_h(const LsGrid& g, double a, double h, double rh) {
-  return g.fast ? div_known(a, h, rh) : __ddiv_rn(a, h);
+// A block works on kLines lines of kSeg consecutive cells along an axis, one
+// thread per cell; what a cell's face needs of its neighbours goes through
+// shared memory.  The face right of a cell needs three-cell stencils up to two
+// cells away, so kFaces = kSeg - 5 faces of a segment are complete.  A warp is
+// 8 lines by 4 cells for every axis: the lines are adjacent along x (64-byte
+// accesses), or along y for the x axis (32-byte accesses), where it keeps the
+// ends of segments from idling half a warp (the kernels are bound by
+// arithmetic, with DRAM at a few percent).
+constexpr int kSeg = 64, kLines = 8, kLsThreads = kSeg * kLines, kFaces = kSeg - 5;
+
+struct LsLine {
+  int c;         // the thread's cell along the axis (may lie outside the grid)
+  int a;         // position in the segment
+  int n;         // cells along the axis
+  int l1, l2;    // the line: its two other indices
+  bool live;     // the line exists
+  size_t stride, base;
+};
+
+// The unit of a block: count = (segments) x (line groups) x (other axis)
+template <int kAxis>
+__device__ __forceinline__ LsLine ls_line(const LsGrid& g, int faces) {
+  LsLine L;
+  L.a = threadIdx.x / kLines;
+  const int l = threadIdx.x % kLines;
+  L.n = kAxis == 0 ? g.nx : (kAxis == 1 ? g.ny : g.nz);
+  const int n1 = kAxis == 0 ? g.ny : g.nx;
+  const int segs = (faces + kFaces - 1) / kFaces, groups = (n1 + kLines - 1) / kLines;
+  const unsigned b = blockIdx.x;
+  const int seg = (int)(b % (unsigned)segs);
+  const unsigned r = b / (unsigned)segs;
+  L.l1 = (int)(r % (unsigned)groups) * kLines + l;
+  L.l2 = (int)(r / (unsigned)groups);
+  L.live = L.l1 < n1;
+  const int l1 = L.live ? L.l1 : n1 - 1;
+  L.c = seg * kFaces - 3 + L.a;
+  L.stride = kAxis == 0 ? 1 : (kAxis == 1 ? (size_t)g.nx : (size_t)g.nx * g.ny);
+  L.base = kAxis == 0   ? ((size_t)L.l2 * g.ny + l1) * g.nx
+           : kAxis == 1 ? (size_t)L.l2 * g.ny * g.nx + l1
+                        : (size_t)L.l2 * g.nx + l1;
+  return L;
 }
+
+unsigned ls_blocks(const LsGrid& g, int axis, int faces) {
+  const int n1 = axis == 0 ? g.ny : g.nx, n2 = axis == 2 ? g.ny : g.nz;
+  return (unsigned)((faces + kFaces - 1) / kFaces) * (unsigned)((n1 + kLines - 1) / kLines) *
+         (unsigned)n2;
+}
+
+// weights of a stencil of zeros: 1, 6 and 3 over eps^2
+struct LsZero {
+  double w1, w6, w3;
+};
+
+LsZero ls_zero(double eps) {
+  const double x = eps * eps;
+  return LsZero{1.0 / x, 6.0 / x, 3.0 / x};
+}
+
+constexpr double kAdvEps = 1.0e-13, kRedisEps = 1.0e-10;
 
 // Faces of one axis: face f (0..n) is the reference's face i+1/2 with
 // i = f - 1; ss1 = left-biased WENO of u+ phi, ss2 = right-biased of u- phi.
 // The face arrays are laid out like cell arrays with n+1 entries along the
 // axis.
-__global__ void __launch_bounds__(256) k_ls_faces(LsGrid g, int axis, const double* __restrict__ phi,
-                                                  const double* __restrict__ vel,
-                                                  double* __restrict__ ss1,
-                                                  double* __restrict__ ss2) {
-  const int ex = g.nx + (axis == 0), ey = g.ny + (axis == 1), ez = g.nz + (axis == 2);
-  const size_t nf = (size_t)ex * ey * ez;
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nf) return;
-  const int a = (int)(t % ex);
-  const size_t r = t / ex;
-  const int b = (int)(r % ey), c = (int)(r / ey);
-  // position of the face along the axis and the line through it
-  const int f = axis == 0 ? a : (axis == 1 ? b : c);
-  const int n = axis == 0 ? g.nx : (axis == 1 ? g.ny : g.nz);
-  const size_t stride = axis == 0 ? 1 : (axis == 1 ? (size_t)g.nx : (size_t)g.nx * g.ny);
-  const int i0 = axis == 0 ? 0 : a, j0 = axis == 1 ? 0 : b, k0 = axis == 2 ? 0 : c;
-  const size_t base = ((size_t)k0 * g.ny + j0) * g.nx + i0;
-  const int fi = f - 1;
-  double gp[6], gm[6];  // u+ phi and u- phi of cells fi-2 .. fi+3
-#pragma unroll
-  for (int m = 0; m < 6; ++m) {
-    const size_t q = base + (size_t)clampi(fi - 2 + m, n) * stride;
+template <int kAxis>
+__global__ void __launch_bounds__(kLsThreads, 2)
+    k_ls_faces(LsGrid g, LsZero z, const double* __restrict__ phi, const double* __restrict__ vel,
+               double* __restrict__ ss1, double* __restrict__ ss2) {
+  constexpr int S = kLines;  // neighbour along the line
+  __shared__ double gp[kLsThreads], gm[kLsThreads], tp[kLsThreads], tm[kLsThreads];
+  __shared__ double p1[kLsThreads], p3[kLsThreads], m1[kLsThreads], m2[kLsThreads];
+  const int t = threadIdx.x;
+  const LsLine L = ls_line<kAxis>(g, (kAxis == 0 ? g.nx : kAxis == 1 ? g.ny : g.nz) + 1);
+  const bool used = L.live && L.c <= L.n + 2;  // cells that some face reads
+  if (used) {
+    const size_t q = L.base + (size_t)clampi(L.c, L.n) * L.stride;
     const double u = vel[q], p = phi[q];
-    gp[m] = mul(mul(0.5, add(u, fabs(u))), p);
-    gm[m] = mul(mul(0.5, sub(u, fabs(u))), p);
+    double a, b;
+    const long long ub = __double_as_longlong(u);
+    if ((ub & 0x7ff0000000000000ll) < 0x7fe0000000000000ll &&
+        (__double_as_longlong(p) & 0x7ff0000000000000ll) < 0x7ff0000000000000ll) {
+      // (u + |u|)/2 and (u - |u|)/2 are u and +0, or +0 and u (-0 keeps its
+      // sign in the second): one product, the other a zero of p's sign
+      const double v = mul_int(u, p);
+      const double zp = __hiloint2double(__double2hiint(p) & (int)0x80000000, 0);
+      const bool neg = ub < 0, nz = (ub << 1) != 0;
+      a = !neg && nz ? v : zp;
+      b = neg ? v : zp;
+    } else {
+      a = mul(mul(0.5, add(u, fabs(u))), p);
+      b = mul(mul(0.5, sub(u, fabs(u))), p);
+    }
+    gp[t] = a;
+    gm[t] = b;
+    tp[t] = mul_k<3>(a);
+    tm[t] = mul_k<3>(b);
   }
-  const double eps = 1.0e-13;
-  ss1[t] = weno_left(gp[0], gp[1], gp[2], gp[3], gp[4], eps);
-  ss2[t] = weno_right(gm[1], gm[2], gm[3], gm[4], gm[5], eps);
+  __syncthreads();
+  double p2 = z.w6, m3 = z.w3;
+  if (used && L.a >= 1 && L.a <= kSeg - 2 && L.c <= L.n + 1) {
+    double x[3], w1 = z.w1, w3 = z.w3;
+    if (!(is_zero(gp[t - S]) && is_zero(gp[t]) && is_zero(gp[t + S]))) {
+      weno_stencil(gp[t - S], gp[t], gp[t + S], tp[t - S], tp[t + S], kAdvEps, x);
+      w1 = div_int(1.0, rcp_int(x[0]));
+      p2 = div_int(6.0, rcp_int(x[1]));
+      w3 = div_int(3.0, rcp_int(x[2]));
+    }
+    p1[t] = w1;
+    p3[t] = w3;
+    w1 = z.w1;
+    double w2 = z.w6;
+    if (!(is_zero(gm[t - S]) && is_zero(gm[t]) && is_zero(gm[t + S]))) {
+      weno_stencil(gm[t - S], gm[t], gm[t + S], tm[t - S], tm[t + S], kAdvEps, x);
+      w1 = div_int(1.0, rcp_int(x[2]));
+      w2 = div_int(6.0, rcp_int(x[1]));
+      m3 = div_int(3.0, rcp_int(x[0]));
+    }
+    m1[t] = w1;
+    m2[t] = w2;
+  }
+  __syncthreads();
+  const int f = L.c + 1;
+  if (!L.live || L.a < 2 || L.a > kSeg - 4 || f > L.n) return;
+  const int ex = g.nx + (kAxis == 0), ey = g.ny + (kAxis == 1);
+  const size_t o = kAxis == 0   ? ((size_t)L.l2 * ey + L.l1) * ex + f
+                   : kAxis == 1 ? ((size_t)L.l2 * ey + f) * ex + L.l1
+                                : ((size_t)f * ey + L.l2) * ex + L.l1;
+  {
+    const double g0 = gp[t - 2 * S], g1 = gp[t - S], g2 = gp[t], g3 = gp[t + S], g4 = gp[t + 2 * S];
+    if (is_zero(g0) && is_zero(g1) && is_zero(g2) && is_zero(g3) && is_zero(g4))
+      ss1[o] = weno_left_zero(g0, g1, g2, g3, g4);
+    else
+      ss1[o] = weno_left(p1[t - S], p2, p3[t + S], g0, g1, g2, g3, g4);
+  }
+  {
+    const double f0 = gm[t - S], f1 = gm[t], f2 = gm[t + S], f3 = gm[t + 2 * S], f4 = gm[t + 3 * S];
+    if (is_zero(f0) && is_zero(f1) && is_zero(f2) && is_zero(f3) && is_zero(f4))
+      ss2[o] = weno_right_zero(f0, f1, f2, f3, f4);
+    else
+      ss2[o] = weno_right(m1[t + 2 * S], m2[t + S], m3, f0, f1, f2, f3, f4);
+  }
 }
 
 // One stage: l = L(phi) per cell, then phi += src * dt with the stage's
@@ -161,13 +295,13 @@ __global__ void __launch_bounds__(256) k_ls_stage(LsGrid g, int stage, double dt
   const size_t fy = ((size_t)k * (g.ny + 1) + j) * g.nx + i;
   const size_t fz = ((size_t)k * g.ny + j) * g.nx + i;
   double d = sub(sub(add(x1[fx + 1], x2[fx + 1]), x1[fx]), x2[fx]);
-  double src = -by_h(g, d, g.dx, g.rdx);
+  double src = -div_const(g.h[0], d);
   d = sub(sub(add(y1[fy + g.nx], y2[fy + g.nx]), y1[fy]), y2[fy]);
-  src = sub(src, by_h(g, d, g.dy, g.rdy));
+  src = sub(src, div_const(g.h[1], d));
   if (g.nz > 1) {
     const size_t pz = (size_t)g.nx * g.ny;
     d = sub(sub(add(z1[fz + pz], z2[fz + pz]), z1[fz]), z2[fz]);
-    src = sub(src, by_h(g, d, g.dz, g.rdz));
+    src = sub(src, div_const(g.h[2], d));
   }
   double s;
   if (stage == 1) {
@@ -175,11 +309,11 @@ __global__ void __launch_bounds__(256) k_ls_stage(LsGrid g, int stage, double dt
     s = src;
   } else if (stage == 2) {
     l2[q] = src;
-    s = by4(add(mul(-3.0, l1[q]), src));
+    s = by4(sub(src, mul_k<3>(l1[q])));
   } else {
-    s = by12(add(sub(-l1[q], l2[q]), mul(8.0, src)));
+    s = by12(fma2(8.0, src, sub(-l1[q], l2[q])));
   }
-  phi[q] = add(phi[q], mul(s, dt));
+  phi[q] = add(phi[q], mul_int(s, dt));
 }
 
 // ---- redistancing: level_set_rk3_redis ("Two phase flows/newOpenMP/2D/src/
@@ -188,11 +322,38 @@ __global__ void __launch_bounds__(256) k_ls_stage(LsGrid g, int stage, double dt
 constexpr double kPi = 3.141592653589793;  // acos(-1) in double
 
 // ls_funs ("Two phase flows/newOpenMP/3D+IBM/src/interface_solver/
-// others.f90:1-37"): smoothed Heaviside, its derivative and the sign 2H - 1
-__device__ __forceinline__ void ls_funs1(double phi, double ls_wid, double& heavy, double& delta,
-                                         double& sgn) {
+// others.f90:1-37"): smoothed Heaviside, its derivative and the sign 2H - 1.
+// Beyond `out` (slightly above ls_wid (1 - 1e-12), from the host) phi/ls_wid
+// lands past the clipping threshold, so H is 0 or 1 without the division; the
+// test compares bit patterns (NaN takes the formula).
+struct LsWidth {
+  double wid;
+  long long out;
+};
+
+LsWidth ls_width(double ls_wid) {
+  LsWidth w{ls_wid, 0};
+  const double out = ls_wid * (1.0 - 1e-12) * (1.0 + 1e-15);
+  std::memcpy(&w.out, &out, sizeof out);
+  return w;
+}
+
+__device__ __forceinline__ bool ls_outside(const LsWidth& w, double phi) {
+  const long long m = __double_as_longlong(phi) & 0x7fffffffffffffffll;
+  return m > w.out && m <= 0x7ff0000000000000ll;
+}
+
+__device__ __forceinline__ void ls_funs1(double phi, const LsWidth& w, double& heavy,
+                                         double& delta, double& sgn) {
+  if (ls_outside(w, phi)) {
+    const bool neg = __double_as_longlong(phi) < 0;
+    heavy = neg ? 0.0 : 1.0;
+    delta = 0.0;
+    sgn = neg ? -1.0 : 1.0;
+    return;
+  }
   const double eps = 1.0e-12;
-  const double x = dvd(phi, ls_wid);
+  const double x = dvd(phi, w.wid);
   double h, hp;
   if (x > 1.0 - eps) {
     h = 1.0;
@@ -202,7 +363,7 @@ __device__ __forceinline__ void ls_funs1(double phi, double ls_wid, double& heav
     hp = 0.0;
   } else {
     h = mul(0.5, add(add(1.0, x), dvd(sin(mul(kPi, x)), kPi)));
-    hp = dvd(mul(0.5, add(1.0, cos(mul(kPi, x)))), ls_wid);
+    hp = dvd(mul(0.5, add(1.0, cos(mul(kPi, x)))), w.wid);
   }
   h = h < 1.0 ? h : 1.0;
   h = h > 0.0 ? h : 0.0;
@@ -214,7 +375,8 @@ __device__ __forceinline__ void ls_funs1(double phi, double ls_wid, double& heav
 // s = the sign held fixed through the call: 2H - 1, or phi itself for the
 // first redistancing (level_set_redis_stable, btn = 0)
 __global__ void __launch_bounds__(256) k_ls_sign(size_t n, const double* __restrict__ phi,
-                                                 double ls_wid, int btn, double* __restrict__ s) {
+                                                 LsWidth ls_wid, int btn,
+                                                 double* __restrict__ s) {
   const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   if (btn == 0) {
@@ -226,69 +388,107 @@ __global__ void __launch_bounds__(256) k_ls_sign(size_t n, const double* __restr
   }
 }
 
-__device__ __forceinline__ double dmin(double a, double b) { return a < b ? a : b; }
 __device__ __forceinline__ double dmax(double a, double b) { return a > b ? a : b; }
+
+// max(x, 0) and max(-x, 0), 0 for NaN, and the larger of two such values, by
+// their bit patterns (FP64 comparisons run on the FP64 pipe)
+__device__ __forceinline__ double pos_part(double x) {
+  const long long b = __double_as_longlong(x);
+  return b > 0 && b <= 0x7ff0000000000000ll ? x : 0.0;
+}
+__device__ __forceinline__ double neg_part(double x) {
+  return pos_part(__hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x)));
+}
+__device__ __forceinline__ double larger(double a, double b) {
+  return __double_as_longlong(a) > __double_as_longlong(b) ? a : b;
+}
+__device__ __forceinline__ bool at_least_zero(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  return b <= 0x7ff0000000000000ull || b == 0x8000000000000000ull;
+}
 
 // |grad phi| by Godunov upwinding on the sign s (level_set_redis_gradient):
 // the WENO-JS one-sided values (EPS = 1e-10) of the backward differences
-// (phi_i - phi_{i-1})/h, zero-gradient ghosts by index clamping
-__global__ void __launch_bounds__(256) k_ls_grad(LsGrid g, const double* __restrict__ phi,
-                                                 const double* __restrict__ s,
-                                                 double* __restrict__ grad) {
-  const size_t n = (size_t)g.nx * g.ny * g.nz;
-  const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const int i = (int)(q % g.nx);
-  const size_t r = q / g.nx;
-  const int j = (int)(r % g.ny), k = (int)(r / g.ny);
-  const int naxes = g.nz > 1 ? 3 : 2;
-  const bool pos = s[q] >= 0.0;
-  double sum = 0.0;
-  for (int a = 0; a < naxes; ++a) {
-    const int n_a = a == 0 ? g.nx : (a == 1 ? g.ny : g.nz);
-    const int c = a == 0 ? i : (a == 1 ? j : k);
-    const size_t stride = a == 0 ? 1 : (a == 1 ? (size_t)g.nx : (size_t)g.nx * g.ny);
-    const double h = a == 0 ? g.dx : (a == 1 ? g.dy : g.dz);
-    const double rh = a == 0 ? g.rdx : (a == 1 ? g.rdy : g.rdz);
-    const size_t base = q - (size_t)c * stride;
-    double f[6];
-#pragma unroll
-    for (int m = 0; m < 6; ++m) {
-      const int cc = clampi(c - 2 + m, n_a);
-      const int cm = cc > 0 ? cc - 1 : 0;
-      f[m] = by_h(g, sub(phi[base + (size_t)cc * stride], phi[base + (size_t)cm * stride]), h, rh);
-    }
-    const double s1 = weno_right(f[1], f[2], f[3], f[4], f[5], 1.0e-10);
-    const double s2 = weno_left(f[0], f[1], f[2], f[3], f[4], 1.0e-10);
-    const double pm = -dmin(s1, 0.0), pp = dmax(s1, 0.0);
-    const double mm = -dmin(s2, 0.0), mp = dmax(s2, 0.0);
-    const double t = pos ? dmax(pm, mp) : dmax(pp, mm);
-    sum = a == 0 ? mul(t, t) : add(sum, mul(t, t));
+// (phi_i - phi_{i-1})/h, zero-gradient ghosts by index clamping.  One launch
+// per axis, which adds its square to grad; both sides' weights of a stencil
+// come from the same three indicators.  The last axis takes the root and, with
+// kLambda, forms s2 = lam s (|grad| - 1) and s3 = |grad| delta lam
+// (level_set_redis_lambda; delta and both are 0 outside the band) and raises
+// *odd when one of them is not finite.
+template <int kAxis, bool kLast, bool kLambda>
+__global__ void __launch_bounds__(kLsThreads, 2)
+    k_ls_grad(LsGrid g, const double* __restrict__ phi, const double* __restrict__ s,
+              double* __restrict__ grad, LsWidth wid, double rho12, double* __restrict__ s2,
+              double* __restrict__ s3, unsigned long long* odd) {
+  constexpr int S = kLines;
+  __shared__ double d[kLsThreads], td[kLsThreads];
+  __shared__ double l1[kLsThreads], l3[kLsThreads], r1[kLsThreads], r2[kLsThreads];
+  const int t = threadIdx.x;
+  const LsLine L = ls_line<kAxis>(g, (kAxis == 0 ? g.nx : kAxis == 1 ? g.ny : g.nz) + 1);
+  const bool used = L.live && L.c <= L.n + 2;
+  if (used) {
+    const int cc = clampi(L.c, L.n), cm = cc > 0 ? cc - 1 : 0;
+    const double v = div_const(g.h[kAxis], sub(phi[L.base + (size_t)cc * L.stride],
+                                               phi[L.base + (size_t)cm * L.stride]));
+    d[t] = v;
+    td[t] = mul_k<3>(v);
   }
-  grad[q] = __dsqrt_rn(sum);
-}
-
-// s2 = lam s (|grad| - 1), s3 = |grad| delta lam (level_set_redis_lambda)
-__global__ void __launch_bounds__(256) k_ls_lambda(size_t n, int three, double ls_wid,
-                                                   double rho12, const double* __restrict__ phi,
-                                                   const double* __restrict__ s,
-                                                   const double* __restrict__ grad,
-                                                   double* __restrict__ s2,
-                                                   double* __restrict__ s3) {
-  const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  double hv, dl, sg;
-  ls_funs1(phi[q], ls_wid, hv, dl, sg);
-  const double lam = three ? mul(add(mul(mul(2.0, sub(1.0, rho12)), hv), rho12), dl) : dl;
-  s2[q] = mul(mul(lam, s[q]), sub(grad[q], 1.0));
-  s3[q] = mul(mul(grad[q], dl), lam);
+  __syncthreads();
+  double w2 = 0.0, w3 = 0.0;
+  if (used && L.a >= 1 && L.a <= kSeg - 2 && L.c <= L.n + 1) {
+    double x[3];
+    weno_stencil(d[t - S], d[t], d[t + S], td[t - S], td[t + S], kRedisEps, x);
+    const RcpInt x0 = rcp_int(x[0]);
+    l1[t] = div_int(1.0, x0);
+    w3 = div_int(3.0, x0);
+    w2 = div_int(6.0, rcp_int(x[1]));
+    r2[t] = w2;
+    const RcpInt x2 = rcp_int(x[2]);
+    r1[t] = div_int(1.0, x2);
+    l3[t] = div_int(3.0, x2);
+  }
+  __syncthreads();
+  if (!L.live || L.a < 2 || L.a > kSeg - 4 || L.c < 0 || L.c >= L.n) return;
+  const size_t q = L.base + (size_t)L.c * L.stride;
+  const double sq = s[q];
+  const double v1 = weno_right(r1[t + 2 * S], r2[t + S], w3, d[t - S], d[t], d[t + S], d[t + 2 * S],
+                               d[t + 3 * S]);
+  const double v2 = weno_left(l1[t - S], w2, l3[t + S], d[t - 2 * S], d[t - S], d[t], d[t + S],
+                              d[t + 2 * S]);
+  const double v = at_least_zero(sq) ? larger(neg_part(v1), pos_part(v2))
+                                     : larger(pos_part(v1), neg_part(v2));
+  double sum = isq(v);
+  if (kAxis > 0) sum = add(grad[q], sum);
+  if (kLast) sum = __dsqrt_rn(sum);
+  grad[q] = sum;
+  if (kLast && kLambda) {
+    const double p = phi[q];
+    double a = 0.0, b = 0.0;
+    if (!ls_outside(wid, p) ||
+        (__double_as_longlong(sum) & 0x7ff0000000000000ll) == 0x7ff0000000000000ll) {
+      double hv, dl, sg;
+      ls_funs1(p, wid, hv, dl, sg);
+      const double lam = g.nz > 1 ? mul(add(mul(mul(2.0, sub(1.0, rho12)), hv), rho12), dl) : dl;
+      a = mul(mul(lam, sq), sub(sum, 1.0));
+      b = mul(mul(sum, dl), lam);
+      const long long e = 0x7ff0000000000000ll;
+      if ((__double_as_longlong(a) & e) == e || (__double_as_longlong(b) & e) == e)
+        atomicOr(odd, 1ull);
+    }
+    s2[q] = a;
+    s3[q] = b;
+  }
 }
 
 // One pseudo-time stage: s1 = the correction (block sums of s2 and s3 with
 // weight 16 (2D) or 51 (3D) on the cell, btn = 1; 0 for btn = 0),
-// l = (s - s1)|grad| - s, phi -= rdt * (the stage's combination of l1..l3)
+// l = (s - s1)|grad| - s, phi -= rdt * (the stage's combination of l1..l3).
+// s1 carries the factor delta, so it is 0 outside the band and only the
+// band's cells add the 54 neighbours (unless one of s2, s3 is not finite
+// somewhere, *odd).
 __global__ void __launch_bounds__(256) k_ls_redis_stage(LsGrid g, int stage, int btn, double rdt,
-                                                        double ls_wid,
+                                                        LsWidth ls_wid,
+                                                        const unsigned long long* odd,
                                                         const double* __restrict__ s,
                                                         const double* __restrict__ grad,
                                                         const double* __restrict__ s2,
@@ -298,7 +498,7 @@ __global__ void __launch_bounds__(256) k_ls_redis_stage(LsGrid g, int stage, int
   const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   double s1 = 0.0;
-  if (btn != 0) {
+  if (btn != 0 && (!ls_outside(ls_wid, phi[q]) || *odd != 0ull)) {
     const int i = (int)(q % g.nx);
     const size_t r = q / g.nx;
     const int j = (int)(r % g.ny), k = (int)(r / g.ny);
@@ -318,18 +518,18 @@ __global__ void __launch_bounds__(256) k_ls_redis_stage(LsGrid g, int stage, int
     ls_funs1(phi[q], ls_wid, hv, dl, sg);
     s1 = fabs(b) > 1.0e-12 ? mul(dvd(a, b), dl) : 0.0;
   }
-  const double l = sub(mul(sub(s[q], s1), grad[q]), s[q]);
+  const double l = sub(mul_int(sub(s[q], s1), grad[q]), s[q]);
   double src;
   if (stage == 1) {
     l1[q] = l;
     src = l;
   } else if (stage == 2) {
     l2[q] = l;
-    src = by4(add(mul(-3.0, l1[q]), l));
+    src = by4(sub(l, mul_k<3>(l1[q])));
   } else {
-    src = by12(add(sub(-l1[q], l2[q]), mul(8.0, l)));
+    src = by12(fma2(8.0, l, sub(-l1[q], l2[q])));
   }
-  phi[q] = sub(phi[q], mul(rdt, src));
+  phi[q] = sub(phi[q], mul_int(rdt, src));
 }
 
 // *out = max over cells of |a - b| (b == nullptr: max of a, a >= 0); the
@@ -375,7 +575,7 @@ struct gbmg_ls {
   bool own_stream = false;
   double *phi = nullptr, *u = nullptr, *v = nullptr, *w = nullptr, *l1 = nullptr, *l2 = nullptr;
   double* face[6] = {};
-  unsigned long long* red = nullptr;  // one max-reduction slot
+  unsigned long long* red = nullptr;  // a max-reduction slot and a flag
   unsigned long long* host_red = nullptr;
   int64_t launches = 0;
   std::string err;
@@ -504,7 +704,7 @@ int gbmg_ls_create(const gbmg_grid* grid, int device, void* stream, gbmg_ls** ou
       return GBMG_OUT_OF_MEMORY;
     }
   }
-  if (cudaMalloc((void**)&ls->red, sizeof(unsigned long long)) != cudaSuccess ||
+  if (cudaMalloc((void**)&ls->red, 2 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMallocHost((void**)&ls->host_red, sizeof(unsigned long long)) != cudaSuccess) {
     cudaGetLastError();
     ls_free(ls);
@@ -552,15 +752,17 @@ int gbmg_ls_advect(gbmg_ls* ls, gbmg_field phi, gbmg_field u, gbmg_field v, gbmg
   const LsGrid G = ls_grid(g);
   const size_t n = ls_cells(g);
   const double* vel[3] = {ls->u, ls->v, ls->w};
-  const size_t nf[3] = {(size_t)(g.nx + 1) * g.ny * g.nz, (size_t)g.nx * (g.ny + 1) * g.nz,
-                        (size_t)g.nx * g.ny * (g.nz + 1)};
+  const LsZero Z = ls_zero(kAdvEps);
   for (int s = 0; s < steps; ++s)
     for (int stage = 1; stage <= 3; ++stage) {
-      for (int a = 0; a < (three ? 3 : 2); ++a) {
-        k_ls_faces<<<blocks_for(nf[a]), 256, 0, ls->stream>>>(G, a, ls->phi, vel[a],
-                                                              ls->face[2 * a], ls->face[2 * a + 1]);
-        ls->launches += 1;
-      }
+      k_ls_faces<0><<<ls_blocks(G, 0, g.nx + 1), kLsThreads, 0, ls->stream>>>(
+          G, Z, ls->phi, vel[0], ls->face[0], ls->face[1]);
+      k_ls_faces<1><<<ls_blocks(G, 1, g.ny + 1), kLsThreads, 0, ls->stream>>>(
+          G, Z, ls->phi, vel[1], ls->face[2], ls->face[3]);
+      if (three)
+        k_ls_faces<2><<<ls_blocks(G, 2, g.nz + 1), kLsThreads, 0, ls->stream>>>(
+            G, Z, ls->phi, vel[2], ls->face[4], ls->face[5]);
+      ls->launches += three ? 3 : 2;
       k_ls_stage<<<blocks_for(n), 256, 0, ls->stream>>>(
           G, stage, dt, ls->face[0], ls->face[1], ls->face[2], ls->face[3], ls->face[4],
           ls->face[5], ls->l1, ls->l2, ls->phi);
@@ -573,6 +775,30 @@ int gbmg_ls_advect(gbmg_ls* ls, gbmg_field phi, gbmg_field u, gbmg_field v, gbmg
 }
 
 namespace {
+// |grad phi| of ls->phi, one launch per axis; with lambda also s2 and s3
+void ls_gradient(gbmg_ls* ls, const LsGrid& G, const double* s, double* grad, bool lambda,
+                 const LsWidth& wid, double rho_12, double* s2, double* s3) {
+  const bool three = G.nz > 1;
+  unsigned long long* odd = ls->red + 1;
+  const unsigned b0 = ls_blocks(G, 0, G.nx + 1), b1 = ls_blocks(G, 1, G.ny + 1);
+  const cudaStream_t st = ls->stream;
+  const double* p = ls->phi;
+  k_ls_grad<0, false, false><<<b0, kLsThreads, 0, st>>>(G, p, s, grad, wid, rho_12, s2, s3, odd);
+  if (three) {
+    const unsigned b2 = ls_blocks(G, 2, G.nz + 1);
+    k_ls_grad<1, false, false><<<b1, kLsThreads, 0, st>>>(G, p, s, grad, wid, rho_12, s2, s3, odd);
+    if (lambda)
+      k_ls_grad<2, true, true><<<b2, kLsThreads, 0, st>>>(G, p, s, grad, wid, rho_12, s2, s3, odd);
+    else
+      k_ls_grad<2, true, false><<<b2, kLsThreads, 0, st>>>(G, p, s, grad, wid, rho_12, s2, s3, odd);
+  } else if (lambda) {
+    k_ls_grad<1, true, true><<<b1, kLsThreads, 0, st>>>(G, p, s, grad, wid, rho_12, s2, s3, odd);
+  } else {
+    k_ls_grad<1, true, false><<<b1, kLsThreads, 0, st>>>(G, p, s, grad, wid, rho_12, s2, s3, odd);
+  }
+  ls->launches += three ? 3 : 2;
+}
+
 // max over cells of |a - b| (or of a), read back to the host
 int ls_max(gbmg_ls* ls, const double* a, const double* b, double* out) {
   const size_t n = ls_cells(ls->grid);
@@ -622,11 +848,12 @@ int gbmg_ls_redistance(gbmg_ls* ls, gbmg_field phi, double ls_wid, double rdt, d
   int rc;
   if ((rc = ls_in(ls, phi, mem, ls->phi)) != GBMG_OK) return rc;
   // level_set_redis_init (+ level_set_redis_stable for btn = 0)
-  k_ls_sign<<<nb, 256, 0, ls->stream>>>(n, ls->phi, ls_wid, btn, s);
+  const LsWidth wid = ls_width(ls_wid);
+  LS_CUDA(ls, cudaMemsetAsync(ls->red + 1, 0, sizeof(unsigned long long), ls->stream));
+  k_ls_sign<<<nb, 256, 0, ls->stream>>>(n, ls->phi, wid, btn, s);
   ls->launches += 1;
   if (btn == 0) {
-    k_ls_grad<<<nb, 256, 0, ls->stream>>>(G, ls->phi, s, grad);
-    ls->launches += 1;
+    ls_gradient(ls, G, s, grad, false, wid, rho_12, s2, s3);
     LS_CUDA(ls, cudaMemsetAsync(ls->red, 0, sizeof(unsigned long long), ls->stream));
     unsigned blocks = nb > 1024 ? 1024 : nb;
     k_ls_maxabs<<<blocks, 256, 0, ls->stream>>>(n, grad, nullptr, ls->red);
@@ -646,14 +873,8 @@ int gbmg_ls_redistance(gbmg_ls* ls, gbmg_field phi, double ls_wid, double rdt, d
     LS_CUDA(ls, cudaMemcpyAsync(tmp, ls->phi, n * sizeof(double), cudaMemcpyDeviceToDevice,
                                 ls->stream));
     for (int stage = 1; stage <= 3; ++stage) {
-      k_ls_grad<<<nb, 256, 0, ls->stream>>>(G, ls->phi, s, grad);
-      ls->launches += 1;
-      if (btn != 0) {
-        k_ls_lambda<<<nb, 256, 0, ls->stream>>>(n, three ? 1 : 0, ls_wid, rho_12, ls->phi, s,
-                                                grad, s2, s3);
-        ls->launches += 1;
-      }
-      k_ls_redis_stage<<<nb, 256, 0, ls->stream>>>(G, stage, btn, rdt, ls_wid, s, grad, s2, s3,
+      ls_gradient(ls, G, s, grad, btn != 0, wid, rho_12, s2, s3);
+      k_ls_redis_stage<<<nb, 256, 0, ls->stream>>>(G, stage, btn, rdt, wid, ls->red + 1, s, grad, s2, s3,
                                                    ls->l1, ls->l2, ls->phi);
       ls->launches += 1;
     }
