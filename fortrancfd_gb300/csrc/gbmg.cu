@@ -263,7 +263,7 @@ int free_all(gbmg_handle* h) {
   dfree(h->pw[0]); dfree(h->pw[1]); dfree(h->bw); dfree(h->cxw); dfree(h->cyw); dfree(h->czw);
   for (int a = 0; a < 3; ++a) dfree(h->vel[a]);
   dfree(h->aux[0]); dfree(h->aux[1]); dfree(h->r0);
-  dfree(h->kr); dfree(h->kz); dfree(h->kzold); dfree(h->kd); dfree(h->kq);
+  dfree(h->kdiag); dfree(h->kr); dfree(h->kz); dfree(h->kzold); dfree(h->kd); dfree(h->kq);
   dfree(h->gmV); dfree(h->gmZ); dfree(h->gmPart); dfree(h->gmDev);
   if (h->gmHost) cudaFreeHost(h->gmHost);
   dfree(h->minv); dfree(h->adense); dfree(h->cwork); dfree(h->minv32); dfree(h->adense32); dfree(h->derr);
@@ -389,8 +389,9 @@ int allocate(gbmg_handle* h) {
   // the FP64 increment rule keeps the previous cycle's p
   if (h->prm.stop_rule == GBMG_STOP_INCREMENT && !h->mixed) GB_TRY(dmalloc(h, &h->r0, h->n0));
   if (h->prm.krylov) {
+    GB_TRY(dmalloc(h, &h->kdiag, h->n0));
     GB_TRY(dmalloc(h, &h->kr, h->n0));
-    GB_TRY(dmalloc(h, &h->kz, h->n0));
+    if (!h->mixed || h->prm.krylov == 2) GB_TRY(dmalloc(h, &h->kz, h->n0));
     GB_TRY(dmalloc(h, &h->kzold, h->n0));
     GB_TRY(dmalloc(h, &h->kd, h->n0));
     GB_TRY(dmalloc(h, &h->kq, h->n0));
@@ -457,6 +458,7 @@ int build_hierarchy(gbmg_handle* h) {
   }
   LAUNCH(h, GBMG_PROF_SETUP,
          launch_coarse_invert(s, v64(h->lv[h->L - 1]), h->minv, h->adense, h->minv32, h->adense32, h->cwork));
+  if (h->kdiag) LAUNCH(h, GBMG_PROF_SETUP, launch_diag(s, v64(h->lv[0]), h->kdiag));
   if (h->mixed && !h->fine_copies) {
     const Level& f = h->lv[0];
     LAUNCH(h, GBMG_PROF_SETUP, launch_to_dw(s, f.cx, h->cxw, f.n));
@@ -580,6 +582,30 @@ int read_result(gbmg_handle* h, int slot, double* v) {
   return GBMG_OK;
 }
 
+// kr = b - A p in FP64 and its norm (flexible CG: at the start, and where the
+// recursion's residual is about to be believed), with the FP32 copy that the
+// next mixed iteration's V-cycle reads.
+int pcg_residual(gbmg_handle* h) {
+  const cudaStream_t s = h->stream;
+  Level& f = h->lv[0];
+  f.sol = h->p; f.src = h->b;
+  LAUNCH(h, GBMG_PROF_RESIDUAL, launch_residual_norm<double>(s, v64(f), h->kr, h->red, kSlotNorm));
+  if (h->mixed && h->prm.krylov == 1) {
+    if (f.split)
+      LAUNCH(h, GBMG_PROF_VECTOR, launch_to_split(s, h->kr, f.src32, f.nx, f.ny, f.nz, f.hstride));
+    else
+      LAUNCH(h, GBMG_PROF_VECTOR, launch_double_to_float(s, h->kr, f.src32, h->n0));
+  }
+  return check_launch(h, "residual");
+}
+
+// Captured graphs come in two variants: the mixed iteration by the buffer that
+// holds p, flexible CG by how it gets its residual.
+int graph_par(const gbmg_handle* h, int kind) {
+  if (kind == kGraphMixed) return h->pcur;
+  return kind == kGraphFp64 ? 0 : (h->pcg_true ? 1 : 0);
+}
+
 // Enqueue the body of one solver iteration for the given kind.
 // cycles: FP32 V-cycles of a mixed iteration (one defect correction)
 int enqueue_iteration(gbmg_handle* h, int kind, bool first, bool to_host = true, int cycles = 1) {
@@ -614,23 +640,24 @@ int enqueue_iteration(gbmg_handle* h, int kind, bool first, bool to_host = true,
       f.sol = h->kz; f.src = h->kr;
       GB_TRY(enqueue_vcycle<double>(h, true, zg));
     } else {
-      if (f.split) LAUNCH(h, V, launch_to_split(s, h->kr, f.src32, f.nx, f.ny, f.nz, f.hstride));
-      else LAUNCH(h, V, launch_double_to_float(s, h->kr, f.src32, n));
-      if (!zg) GB_CUDA(h, cudaMemsetAsync(f.sol32, 0, n * sizeof(float), s));
+      // (src32 holds r: pcg_residual or the last iteration's step wrote it)
+      if (!zg) GB_CUDA(h, cudaMemsetAsync(f.sol32, 0, (f.split ? n / 2 + f.hstride : n) * sizeof(float), s));
       GB_TRY(enqueue_vcycle<float>(h, true, zg));
-      if (f.split)
-        LAUNCH(h, V, launch_from_split(s, f.sol32, h->kz, f.nx, f.ny, f.nz, f.hstride));
-      else LAUNCH(h, V, launch_float_to_double(s, f.sol32, h->kz, n));
     }
-    LAUNCH(h, V, launch_sum(s, h->kz, n, h->red, kSlotSum));
-    LAUNCH(h, V, launch_shift_by_mean(s, h->kz, h->kz, n, h->red, kSlotSum, -1));
-    LAUNCH(h, V, launch_dot2(s, h->kr, h->kz, h->kzold, n, h->red, kSlotDot));
-    LAUNCH(h, V, launch_pcg_direction(s, h->kd, h->kzold, h->kz, n, h->red, first ? 1 : 0));
-    h->launches += 1;  // the one-thread rz bookkeeping kernel
+    const bool z64 = kind == kGraphPcg64;
+    const PcgVec z{z64 ? h->kz : nullptr, z64 ? nullptr : f.sol32, n, f.split ? f.hstride : 0,
+                   f.nx, f.ny};
+    LAUNCH(h, V, launch_pcg_sum(s, z, h->red, kSlotSum));
+    LAUNCH(h, V, launch_pcg_dots(s, z, h->kr, h->kzold, h->red));
+    LAUNCH(h, V, launch_pcg_direction(s, h->kd, h->kzold, n, h->red, first ? 1 : 0));
     f.sol = h->p; f.src = h->b;
-    LAUNCH(h, R, launch_apply_dot(s, v64(f), h->kd, h->kq, h->red, kSlotDot2));
-    LAUNCH(h, V, launch_pcg_step(s, h->p, h->kd, n, h->red));
-    LAUNCH(h, R, launch_residual_norm<double>(s, v64(f), h->kr, h->red, kSlotNorm));
+    LAUNCH(h, R, launch_apply_diag(s, v64(f), h->kdiag, h->kd, h->kq, h->red, kSlotDot2, true));
+    if (h->pcg_true) {
+      LAUNCH(h, V, launch_pcg_x(s, h->p, h->kd, n, h->red));
+      GB_TRY(pcg_residual(h));
+    } else {
+      LAUNCH(h, V, launch_pcg_step(s, h->p, h->kd, h->kr, h->kq, z64 ? nullptr : f.src32, z, h->red));
+    }
   }
   if (to_host)
     GB_CUDA(h, cudaMemcpyAsync(h->host_res, h->red.result, kRedSlots * sizeof(double),
@@ -646,7 +673,7 @@ int run_iteration(gbmg_handle* h, int kind, bool first, int cycles = 1) {
     GB_TRY(enqueue_iteration(h, kind, first, true, cycles));
     return GBMG_OK;
   }
-  const int par = kind == kGraphMixed ? h->pcur : 0;
+  const int par = graph_par(h, kind);
   cudaGraphExec_t& gx = tail ? h->tail_graph[cycles][par] : h->graph[kind][par];
   int64_t& gk = tail ? h->tail_kernels[cycles][par] : h->graph_kernels[kind][par];
   if (!gx) {
@@ -769,7 +796,7 @@ int build_loop(gbmg_handle* h, int kind, int par) {
 int run_loop(gbmg_handle* h, int kind, CycleCtl* c, bool* used) {
   *used = false;
   if (h->loop_off || h->prm.use_graph != 1 || h->prof || h->stag_mode) return GBMG_OK;
-  const int par = kind == kGraphMixed ? h->pcur : 0;
+  const int par = graph_par(h, kind);
   if (!h->loop_graph[kind][par]) {
     GB_TRY(build_loop(h, kind, par));
     if (!h->loop_graph[kind][par]) return GBMG_OK;
@@ -825,7 +852,8 @@ int gm_apply(gbmg_handle* h) {
   Level& f = h->lv[0];
   const auto enqueue = [&]() -> int {
     GB_TRY(precondition(h, h->kr, h->kz));
-    LAUNCH(h, GBMG_PROF_RESIDUAL, launch_apply_dot(s, v64(f), h->kz, h->kq, h->red, kSlotDot2));
+    LAUNCH(h, GBMG_PROF_RESIDUAL,
+           launch_apply_diag(s, v64(f), h->kdiag, h->kz, h->kq, h->red, kSlotDot2, false));
     return check_launch(h, "preconditioned product");
   };
   if (!h->prm.use_graph || h->prof) return enqueue();
@@ -1046,10 +1074,16 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
   if (h->prm.stop_rule == GBMG_STOP_RMS) tol = tol * std::sqrt((double)n) / scale;
   const double rtol = by_inc ? 0.0 : tol;  // threshold of the residual tests
   bool shifted = false;
+  // Below 1e-11 flexible CG recomputes its residual every iteration: the
+  // recursion strays from b - A p by about 1e-15 |A||p| per iteration, up to
+  // some 1e-13 |b| over a solve, which a tolerance near the FP64 floor (a
+  // difference of two solves at 1e-13) can see.  At 1e-11 and above it is under
+  // a hundredth of the tolerance, and b - A p has the last word either way.
+  h->pcg_true = rtol < 1e-11;
   // initial residual
   f.sol = h->p; f.src = h->b;
   if (pcg) {
-    LAUNCH(h, GBMG_PROF_RESIDUAL, launch_residual_norm<double>(s, v64(f), h->kr, h->red, kSlotNorm));
+    GB_TRY(pcg_residual(h));
     GB_CUDA(h, cudaMemsetAsync(h->kzold, 0, n * sizeof(double), s));
   } else if (h->mixed) {
     GB_TRY(start_mixed(h, &shifted));
@@ -1171,6 +1205,17 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
         }
       }
     }
+    if (pcg && h->prm.krylov != 2 && cyc > 0 && !h->pcg_true) {
+      // the recursion's residual, restated as b - A p: accepted below the
+      // tolerance, else the iteration goes on from it
+      GB_TRY(pcg_residual(h));
+      GB_TRY(read_result(h, kSlotNorm, &r2));
+      rel = std::sqrt(r2) / scale;
+      if (status == GBMG_OK && !(rel < rtol)) {
+        status = std::isfinite(rel) ? GBMG_NOT_CONVERGED : GBMG_DIVERGED;
+        if (status == GBMG_NOT_CONVERGED && cyc < h->prm.max_cycles) continue;
+      }
+    }
     // mean projection of p (compatibility_sol on the finest level)
     if (kind == kGraphMixed) {
       GB_TRY(finish_mixed(h, shifted));
@@ -1258,8 +1303,10 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
   const int w = h->mixed ? 4 : 8;
   double per = vcycle_bytes(h, w);
   if (kind == kGraphMixed) per += (40.0 * n + 16.0 * n + 4.0 * n) / h->inner;
+  else if (h->prm.krylov == 1) per += (h->mixed ? 156.0 : 160.0) * n;  // pcg.cu's passes
   else per += 40.0 * n + (h->mixed ? 20.0 * n : 0.0);
-  if (pcg) per += (h->mixed ? 24.0 : 8.0) * n + 16.0 * n + 32.0 * n + 48.0 * n + 24.0 * n + 8.0 * n;
+  if (h->prm.krylov == 2)
+    per += (h->mixed ? 24.0 : 8.0) * n + 16.0 * n + 32.0 * n + 48.0 * n + 24.0 * n + 8.0 * n;
   st->bytes = per * cyc + 40.0 * n + 32.0 * n;
   return status;
 }

@@ -261,22 +261,38 @@ void launch_increment(cudaStream_t s, const T* x, const T* y, size_t n, size_t h
 void launch_zero_wall_faces(cudaStream_t s, int nx, int ny, int nz, double* u, int64_t usy,
                             int64_t usz, double* v, int64_t vsy, int64_t vsz, double* w,
                             int64_t wsy, int64_t wsz);
-// slot <- sum x, slot+1 <- sum x^2
+// slot <- sum x
 void launch_sum(cudaStream_t s, const double* x, size_t n, const ReduceScratch& R, int slot);
 // y = x - result[slot]/n ; result[slot2] <- sum y^2 (slot2 < 0: no norm)
 void launch_shift_by_mean(cudaStream_t s, const double* x, double* y, size_t n,
                           const ReduceScratch& R, int slot, int slot2);
 void launch_add_float(cudaStream_t s, double* p, const float* e, size_t n);
-// Flexible-CG helpers.  Slots: kSlotDot = r.z, kSlotDot+1 = r.z_old,
-// kSlotDot2 = d.(A d), kSlotDot2+1 = r.z of the previous iteration.
-void launch_dot2(cudaStream_t s, const double* a, const double* b, const double* c, size_t n,
-                 const ReduceScratch& R, int slot);
-void launch_pcg_direction(cudaStream_t s, double* d, double* zold, const double* z, size_t n,
+// Flexible-CG passes (pcg.cu).  Slots: kSlotSum = sum z, kSlotDot = r.z,
+// kSlotDot+1 = r.z_old, kSlotDot2 = d.(A d), kSlotDot2+1 = r.z of the previous
+// iteration, kSlotNorm = |r|^2.
+// The V-cycle's result z: z64 (FP64), or z32 (colour-split when hstride != 0).
+struct PcgVec {
+  const double* z64;
+  const float* z32;
+  size_t n, hstride;
+  int nx, ny;
+};
+void launch_pcg_sum(cudaStream_t s, const PcgVec& z, const ReduceScratch& R, int slot);
+// r.(z - mean), r.zold, then zold = z - mean
+void launch_pcg_dots(cudaStream_t s, const PcgVec& z, const double* r, double* zold,
+                     const ReduceScratch& R);
+void launch_pcg_direction(cudaStream_t s, double* d, const double* z, size_t n,
                           const ReduceScratch& R, int first);
-void launch_pcg_step(cudaStream_t s, double* x, const double* d, size_t n, const ReduceScratch& R);
-// q = A d on a level and d.q into slot (kernels_mg.cu)
-void launch_apply_dot(cudaStream_t s, const LevelView<double>& L, const double* d, double* q,
-                      const ReduceScratch& R, int slot);
+void launch_pcg_x(cudaStream_t s, double* x, const double* d, size_t n,
+                  const ReduceScratch& R);  // x += alpha d
+// x += alpha d, r -= alpha q, |r|^2; r32 (may be null): r rounded to float, in z's layout
+void launch_pcg_step(cudaStream_t s, double* x, const double* d, double* r, const double* q,
+                     float* r32, const PcgVec& z, const ReduceScratch& R);
+// sum of the face coefficients of each cell, and q = A d with it, d.q into
+// slot; keep_rz: kSlotDot2+1 <- kSlotDot (kernels_mg.cu)
+void launch_diag(cudaStream_t s, const LevelView<double>& L, double* diag);
+void launch_apply_diag(cudaStream_t s, const LevelView<double>& L, const double* diag,
+                       const double* d, double* q, const ReduceScratch& R, int slot, bool keep_rz);
 void launch_float_to_double(cudaStream_t s, const float* a, double* b, size_t n);
 // flexible GMRES vector kernels (krylov.cu): out[i] = V_i . w for i < cnt
 // (basis V_i at V + i*ld; partials: cnt * max_blocks doubles), w += sign *

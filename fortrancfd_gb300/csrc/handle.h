@@ -59,6 +59,10 @@ struct gbmg_handle {
   double* r0 = nullptr;  // initial FP64 residual of a warm-started mixed solve (first use)
   // flexible CG vectors (allocated when krylov = 1)
   double *kr = nullptr, *kz = nullptr, *kzold = nullptr, *kd = nullptr, *kq = nullptr;
+  // flexible CG recomputes b - A p every iteration (tight tolerances) instead
+  // of following the recursion
+  bool pcg_true = false;
+  double* kdiag = nullptr;  // sum of the finest level's face coefficients per cell
   // flexible GMRES (krylov = 2): basis V (restart + 1 vectors), preconditioned
   // vectors Z (restart), dot partials, device and pinned host coefficients
   double *gmV = nullptr, *gmZ = nullptr, *gmPart = nullptr, *gmDev = nullptr, *gmHost = nullptr;

@@ -368,12 +368,9 @@ __global__ void k_zero_wall_faces(int nx, int ny, int nz, double* u, int64_t usy
 
 __global__ void __launch_bounds__(kRedThreads) k_sum(const double* __restrict__ x, size_t n,
                                                      ReduceScratch R, int slot) {
-  double acc[2] = {0.0, 0.0};
-  stride4(n, [&](size_t q) { return x[q]; }, [&](size_t, double a) {
-    acc[0] += a;
-    acc[1] += a * a;
-  });
-  grid_sum_finish<2>(acc, R, slot);
+  double acc[1] = {0.0};
+  stride4(n, [&](size_t q) { return x[q]; }, [&](size_t, double a) { acc[0] += a; });
+  grid_sum_finish<1>(acc, R, slot);
 }
 
 __global__ void __launch_bounds__(kRedThreads) k_shift_by_mean(const double* __restrict__ x,
@@ -401,42 +398,6 @@ __global__ void k_f2d(const float* __restrict__ a, double* b, size_t n) {
 
 __global__ void k_d2f(const double* __restrict__ a, float* b, size_t n) {
   stride4(n, [&](size_t q) { return a[q]; }, [&](size_t q, double v) { b[q] = (float)v; });
-}
-
-// slot <- a.b, slot+1 <- a.c (c may be null)
-__global__ void __launch_bounds__(kRedThreads) k_dot2(const double* __restrict__ a,
-                                                      const double* __restrict__ b,
-                                                      const double* __restrict__ c, size_t n,
-                                                      ReduceScratch R, int slot) {
-  double acc[2] = {0.0, 0.0};
-  stride4(n, [&](size_t q) { return make_double3(a[q], b[q], c ? c[q] : 0.0); },
-          [&](size_t, double3 v) {
-            acc[0] += v.x * v.y;
-            if (c) acc[1] += v.x * v.z;
-          });
-  grid_sum_finish<2>(acc, R, slot);
-}
-
-// Flexible-CG direction: beta = (r.z - r.z_old)/rz_old (0 on the first
-// iteration), d = z + beta d, z_old = z.  rz_old lives in result[kSlotDot2+1].
-__global__ void k_pcg_direction(double* d, double* zold, const double* __restrict__ z, size_t n,
-                                ReduceScratch R, int first) {
-  const double rz = R.result[kSlotDot], rzo = R.result[kSlotDot + 1];
-  const double beta = first ? 0.0 : (rz - rzo) / R.result[kSlotDot2 + 1];
-  stride4(n, [&](size_t q) { return make_double2(z[q], first ? 0.0 : d[q]); },
-          [&](size_t q, double2 v) {
-            d[q] = first ? v.x : v.x + beta * v.y;
-            zold[q] = v.x;
-          });
-}
-
-__global__ void k_pcg_keep_rz(ReduceScratch R) { R.result[kSlotDot2 + 1] = R.result[kSlotDot]; }
-
-// x += alpha d with alpha = (r.z)/(d.q)
-__global__ void k_pcg_step(double* x, const double* __restrict__ d, size_t n, ReduceScratch R) {
-  const double alpha = R.result[kSlotDot] / R.result[kSlotDot2];
-  stride4(n, [&](size_t q) { return make_double2(x[q], d[q]); },
-          [&](size_t q, double2 v) { x[q] = v.x + alpha * v.y; });
 }
 
 }  // namespace
@@ -647,22 +608,6 @@ void launch_float_to_double(cudaStream_t s, const float* a, double* b, size_t n)
 
 void launch_double_to_float(cudaStream_t s, const double* a, float* b, size_t n) {
   k_d2f<<<stride_blocks(n) * 2, kRedThreads, 0, s>>>(a, b, n);
-}
-
-void launch_dot2(cudaStream_t s, const double* a, const double* b, const double* c, size_t n,
-                 const ReduceScratch& R, int slot) {
-  const unsigned bl = std::min<unsigned>(stride_blocks(n), (unsigned)R.max_blocks);
-  k_dot2<<<bl, kRedThreads, 0, s>>>(a, b, c, n, R, slot);
-}
-
-void launch_pcg_direction(cudaStream_t s, double* d, double* zold, const double* z, size_t n,
-                          const ReduceScratch& R, int first) {
-  k_pcg_direction<<<stride_blocks(n) * 2, kRedThreads, 0, s>>>(d, zold, z, n, R, first);
-  k_pcg_keep_rz<<<1, 1, 0, s>>>(R);
-}
-
-void launch_pcg_step(cudaStream_t s, double* x, const double* d, size_t n, const ReduceScratch& R) {
-  k_pcg_step<<<stride_blocks(n) * 2, kRedThreads, 0, s>>>(x, d, n, R);
 }
 
 }  // namespace gbmg

@@ -80,24 +80,47 @@ __global__ void __launch_bounds__(kRedThreads) k_residual_norm(LevelView<double>
   grid_sum_finish<1>(acc, R, slot);
 }
 
-// q = A d and sum d.q (the flexible-CG matrix product), rows as k_residual_norm.
-__global__ void __launch_bounds__(kRedThreads) k_apply_dot(LevelView<double> L,
-                                                           const double* __restrict__ dvec,
-                                                           double* qvec, ReduceScratch R,
-                                                           int slot) {
+// sum of the face coefficients (the order of stencil())
+__global__ void __launch_bounds__(256) k_diag(LevelView<double> L, double* diag) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int k = blockIdx.z;
+  if (i >= L.nx || j >= L.ny) return;
+  const size_t q = ((size_t)k * L.ny + j) * L.nx + i;
+  double s, d;
+  stencil(L, L.cx, i, j, k, q, s, d);  // d only
+  diag[q] = d;
+}
+
+// q = A d and sum d.q (the Krylov matrix product): a warp per row, the
+// diagonal read back instead of summed, 8 FP64 operations per cell for 13
+// (bound by the FP64 pipe: 512^3, 3.5 ms before)
+__global__ void __launch_bounds__(kRedThreads)
+    k_apply_diag(LevelView<double> L, const double* __restrict__ diag,
+                 const double* __restrict__ dvec, double* __restrict__ qvec, ReduceScratch R,
+                 int slot, int keep_rz) {
   double acc[1] = {0.0};
   const int rows = L.ny * L.nz;
-  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
+  const int lane = threadIdx.x & 31, warps = kRedThreads / 32;
+  const size_t sy = (size_t)L.nx, sz = (size_t)L.nx * L.ny;
+  for (int row = blockIdx.x * warps + (threadIdx.x >> 5); row < rows; row += gridDim.x * warps) {
     const int j = row % L.ny, k = row / L.ny;
-    for (int i = threadIdx.x; i < L.nx; i += blockDim.x) {
+    for (int i = lane; i < L.nx; i += 32) {
       const size_t q = ((size_t)k * L.ny + j) * L.nx + i;
-      double s, d;
-      stencil(L, dvec, i, j, k, q, s, d);
-      const double a = s - d * dvec[q];
+      double s = 0.0;
+      if (i > 0) s += L.cx[q] * dvec[q - 1];
+      if (i < L.nx - 1) s += L.cx[q + 1] * dvec[q + 1];
+      if (j > 0) s += L.cy[q] * dvec[q - sy];
+      if (j < L.ny - 1) s += L.cy[q + sy] * dvec[q + sy];
+      if (k > 0) s += L.cz[q] * dvec[q - sz];
+      if (k < L.nz - 1) s += L.cz[q + sz] * dvec[q + sz];
+      const double a = s - diag[q] * dvec[q];
       qvec[q] = a;
       acc[0] += dvec[q] * a;
     }
   }
+  if (keep_rz && blockIdx.x == 0 && threadIdx.x == 0)
+    R.result[kSlotDot2 + 1] = R.result[kSlotDot];
   grid_sum_finish<1>(acc, R, slot);
 }
 
@@ -444,10 +467,17 @@ void launch_residual_norm(cudaStream_t s, const LevelView<double>& L, TO* r,
   launch_pdl(k_residual_norm<TO>, dim3(blocks), dim3(kRedThreads), 0, s, L, r, R, slot);
 }
 
-void launch_apply_dot(cudaStream_t s, const LevelView<double>& L, const double* d, double* q,
-                      const ReduceScratch& R, int slot) {
-  const int blocks = std::min(reduce_blocks_for((size_t)L.ny * L.nz), R.max_blocks);
-  k_apply_dot<<<blocks, kRedThreads, 0, s>>>(L, d, q, R, slot);
+void launch_diag(cudaStream_t s, const LevelView<double>& L, double* diag) {
+  const dim3 blk(32, 8, 1);
+  const dim3 grd(cdiv((size_t)L.nx, 32), cdiv((size_t)L.ny, 8), (unsigned)L.nz);
+  k_diag<<<grd, blk, 0, s>>>(L, diag);
+}
+
+void launch_apply_diag(cudaStream_t s, const LevelView<double>& L, const double* diag,
+                       const double* d, double* q, const ReduceScratch& R, int slot,
+                       bool keep_rz) {
+  const int blocks = std::min(reduce_blocks_for(((size_t)L.ny * L.nz + 7) / 8), R.max_blocks);
+  k_apply_diag<<<blocks, kRedThreads, 0, s>>>(L, diag, d, q, R, slot, keep_rz ? 1 : 0);
 }
 
 template <typename T>
