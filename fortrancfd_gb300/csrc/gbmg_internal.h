@@ -7,6 +7,7 @@
 // has the same index map and alignment.
 #pragma once
 
+#include "idiv.h"
 #include "schedule.h"
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -355,12 +356,12 @@ struct NsArgs {
   int nx, ny, nz, g;
   int64_t sy, sz;
   double dx, dy, dz, dt, re, fr, we, mu_12, gx, gy, gz, btn_g, btn_sf;
-  // RN reciprocals of the constant divisors (dx, dy, dz, their squares, re)
-  // and fast = 1 when all of them allow the division-free quotient
-  // (fdiv.cuh); gterm = (g_d btn_g)/fr per axis, the gravity source
-  double rdx, rdy, rdz, rdx2, rdy2, rdz2, rre;
+  // the constant divisors: spacings, their squares and re (idiv.h); gterm =
+  // (g_d btn_g)/fr per axis, the gravity source; band = 1 when the parameters
+  // allow a cell without interface terms to skip them (k_ns_diffusion)
+  ConstDiv h[3], h2[3], rediv;
   double gterm[3];
-  int fast;
+  int band;
   int scheme;  // momentum advection: 0 second-order upwind, 1 QUICK
 };
 struct NsBc {

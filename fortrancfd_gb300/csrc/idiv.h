@@ -178,7 +178,7 @@ GB_HD double div_int(double a, const RcpInt& r) {
   const int ea = (int)((u >> 52) & 0x7ff);
   const int e = ea - r.e + 1022;  // biased exponent of the result, less one
   if ((unsigned)(ea - 1) >= 2046u || r.e == 0 || (unsigned)(e - 2) >= 2040u)
-    return idiv_ieee(a, r.b);
+    return (u << 1) == 0 && r.e != 0 ? a : idiv_ieee(a, r.b);  // (a zero over b > 0 is itself)
   const uint64_t ma = (u & 0xfffffffffffffull) | (1ull << 52);
   // q = floor-ish (a/b significands) 2^63, at most 5 units low
   const uint64_t q = idiv_mulhi(ma << 11, r.y);
@@ -214,8 +214,12 @@ GB_HD double mul_int(double a, double b) {
   const uint64_t u = idiv_bits(a), w = idiv_bits(b);
   const int ea = (int)((u >> 52) & 0x7ff), eb = (int)((w >> 52) & 0x7ff);
   const int e = ea + eb - 1023;
-  if ((unsigned)(ea - 1) >= 2046u || (unsigned)(eb - 1) >= 2046u || (unsigned)(e - 2) >= 2040u)
+  if ((unsigned)(ea - 1) >= 2046u || (unsigned)(eb - 1) >= 2046u || (unsigned)(e - 2) >= 2040u) {
+    // (a zero times a finite value is a zero)
+    if (((u << 1) == 0 || (w << 1) == 0) && ea < 2047 && eb < 2047)
+      return idiv_double((u ^ w) & 0x8000000000000000ull);
     return imul_ieee(a, b);
+  }
   const uint64_t ma = ((u & 0xfffffffffffffull) | (1ull << 52)) << 11;
   const uint64_t mb = ((w & 0xfffffffffffffull) | (1ull << 52)) << 11;
   const uint64_t q = idiv_mulhi(ma, mb);
@@ -236,13 +240,29 @@ GB_HD double mul_k(double a) {
   constexpr int B = K >= 8 ? 3 : (K >= 4 ? 2 : 1);  // 2^B <= K
   const uint64_t u = idiv_bits(a);
   const int ea = (int)((u >> 52) & 0x7ff);
-  if ((unsigned)(ea - 1) >= 2040u) return imul_ieee(a, (double)K);
+  if ((unsigned)(ea - 1) >= 2040u) return (u << 1) == 0 ? a : imul_ieee(a, (double)K);
   const uint64_t v = ((u & 0xfffffffffffffull) | (1ull << 52)) * (uint64_t)K;
   const int big = (int)(v >> (53 + B));
   const int sh = B + big;
   const uint64_t k = (v + (((1u << sh) >> 1) - 1u) + ((v >> sh) & 1u)) >> sh;
   const uint64_t r = ((uint64_t)(uint32_t)(ea - 1 + sh) << 52) + k;
   return idiv_double(r | (u & 0x8000000000000000ull));
+}
+
+// x 2^K by the exponent
+template <int K>
+GB_HD double scale2(double x) {
+  const uint64_t u = idiv_bits(x);
+  if ((unsigned)((int)((u >> 52) & 0x7ff) - 64) < 1900u)
+    return idiv_double(u + ((uint64_t)(int64_t)K << 52));
+  return (u << 1) == 0 ? x : imul_ieee(x, K < 0 ? 1.0 / (double)(1ll << -K) : (double)(1ll << K));
+}
+
+// Bits of a magnitude slightly above ls_wid (1 - 1e-12): |phi| beyond it gives
+// |RN(phi/ls_wid)| > 1 - 1e-12, the clipping threshold of ls_funs, whatever the
+// rounding (margin 1e-15).
+inline long long ls_outside_bits(double ls_wid) {
+  return (long long)idiv_bits(ls_wid * (1.0 - 1e-12) * (1.0 + 1e-15));
 }
 
 // ---- division by a constant known on the host --------------------------------
@@ -264,6 +284,7 @@ struct ConstDiv {
   double h, y, yl;
   int mode;
   int ex;  // kDivExact: log2 of 1/h
+  RcpInt r;
 };
 
 GB_HD double div_const(const ConstDiv& c, double x) {
@@ -282,8 +303,17 @@ GB_HD double div_const(const ConstDiv& c, double x) {
   return (u << 1) == 0 && (c.mode == kDivPair || c.mode == kDivExact) ? x : idiv_ieee(x, c.h);
 }
 
+// the same quotient on the integer pipes (kernels bound by the FP64 pipe: about
+// 30 instructions at one to two a cycle, against two at 16 cycles each)
+GB_HD double div_const_i(const ConstDiv& c, double x) {
+  const uint64_t u = idiv_bits(x);
+  if (c.mode == kDivExact && (unsigned)((int)((u >> 52) & 0x7ff) - 123) < 1800u)
+    return idiv_double(u + ((uint64_t)(int64_t)c.ex << 52));
+  return div_int(x, c.r);
+}
+
 inline ConstDiv const_div(double h) {
-  ConstDiv c{h, 1.0 / h, 0.0, kDivIeee, 0};
+  ConstDiv c{h, 1.0 / h, 0.0, kDivIeee, 0, rcp_int(h)};
   if (!(std::fabs(h) >= 0x1p-60 && std::fabs(h) <= 0x1p60)) return c;
   int ex;
   if (std::frexp(h, &ex) == 0.5) {

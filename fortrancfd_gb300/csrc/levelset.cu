@@ -332,10 +332,7 @@ struct LsWidth {
 };
 
 LsWidth ls_width(double ls_wid) {
-  LsWidth w{ls_wid, 0};
-  const double out = ls_wid * (1.0 - 1e-12) * (1.0 + 1e-15);
-  std::memcpy(&w.out, &out, sizeof out);
-  return w;
+  return LsWidth{ls_wid, ls_outside_bits(ls_wid)};
 }
 
 __device__ __forceinline__ bool ls_outside(const LsWidth& w, double phi) {

@@ -102,15 +102,18 @@ int ns_prepare(gbmg_handle* h, const gbmg_ns_params* prm, const gbmg_ns_fields* 
   a.dx = g.dx; a.dy = g.dy; a.dz = g.dz;
   a.dt = prm->dt; a.re = prm->re; a.fr = prm->fr; a.we = prm->we; a.mu_12 = prm->mu_12;
   a.gx = prm->gx; a.gy = prm->gy; a.gz = prm->gz; a.btn_g = prm->btn_g; a.btn_sf = prm->btn_sf;
-  // reciprocals of the constant divisors (IEEE divisions, so RN(1/b)), and
-  // the gravity source (g_d btn_g)/fr as the reference evaluates it per cell
-  const double dvs[7] = {g.dx, g.dy, g.dz, g.dx * g.dx, g.dy * g.dy, g.dz * g.dz, prm->re};
-  double* rcp[7] = {&a.rdx, &a.rdy, &a.rdz, &a.rdx2, &a.rdy2, &a.rdz2, &a.rre};
-  a.fast = 1;
-  for (int i = 0; i < 7; ++i) {
-    *rcp[i] = 1.0 / dvs[i];
-    if (!fdiv_divisor_ok(dvs[i])) a.fast = 0;
+  // the constant divisors and the gravity source (g_d btn_g)/fr as the reference evaluates it per cell
+  const double hs[3] = {g.dx, g.dy, g.dz};
+  a.band = 1;
+  for (int i = 0; i < 3; ++i) {
+    a.h[i] = const_div(hs[i]);
+    a.h2[i] = const_div(hs[i] * hs[i]);
+    if (!fdiv_divisor_ok(hs[i])) a.band = 0;
   }
+  a.rediv = const_div(prm->re);
+  if (!fdiv_divisor_ok(prm->re) || !(std::fabs(prm->mu_12) < 0x1p60) ||
+      !(std::fabs(prm->btn_sf) < 0x1p60) || (prm->btn_sf != 0 && !fdiv_divisor_ok(prm->we)))
+    a.band = 0;
   a.scheme = prm->adv_scheme;
   if (a.scheme != 0 && a.scheme != 1) {
     h->err = "adv_scheme must be 0 (second-order upwind) or 1 (QUICK)";

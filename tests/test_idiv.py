@@ -62,11 +62,17 @@ int main() {
       same(mul_k<7>(a), 7.0 * a, a, 7, "mul_k");
       same(mul_k<11>(a), 11.0 * a, a, 11, "mul_k");
       same(mul_k<13>(a), 13.0 * a, a, 13, "mul_k");
+      same(scale2<-1>(a), 0.5 * a, a, 0.5, "scale2");
+      same(scale2<-2>(a), 0.25 * a, a, 0.25, "scale2");
+      same(scale2<1>(a), 2.0 * a, a, 2, "scale2");
     }
     for (double a : edge) {
       for (double b : edge) same(mul_int(a, b), a * b, a, b, "mul_int edge");
       same(mul_k<3>(a), 3.0 * a, a, 3, "mul_k edge");
       same(mul_k<13>(a), 13.0 * a, a, 13, "mul_k edge");
+      same(scale2<-1>(a), 0.5 * a, a, 0.5, "scale2 edge");
+      same(scale2<-2>(a), 0.25 * a, a, 0.25, "scale2 edge");
+      same(scale2<1>(a), 2.0 * a, a, 2, "scale2 edge");
     }
     for (double a : edge)
       for (double b : edge) same(div_int(a, rcp_int(b)), a / b, a, b, "div_int edge");
@@ -100,7 +106,10 @@ int main() {
     }
     const ConstDiv c = const_div(h);
     modes[c.mode]++;
-    for (double a : edge) same(div_const(c, a), a / h, a, h, "div_const edge");
+    for (double a : edge) {
+      same(div_const(c, a), a / h, a, h, "div_const edge");
+      same(div_const_i(c, a), a / h, a, h, "div_const_i edge");
+    }
     for (int i = 0; i < 600; ++i) {
       double x = any(700, 1300);
       if (i % 3 == 0) {
@@ -109,6 +118,7 @@ int main() {
       }
       if (i % 7 == 0) x = any(0, 2047);
       same(div_const(c, x), x / h, x, h, "div_const");
+      same(div_const_i(c, x), x / h, x, h, "div_const_i");
     }
   }
   std::printf("%ld %ld %d %d %d %d\n", n, bad, modes[0], modes[1], modes[2], modes[3]);
