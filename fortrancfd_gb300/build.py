@@ -18,8 +18,10 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
          "-I", CSRC, "-I", INCLUDE]
 # Translation units whose FP64 results must equal the oracle's bit for bit are
-# compiled without multiply-add contraction.
-FILE_FLAGS = {"momentum.cu": ["-fmad=false"], "ccd.cu": ["-fmad=false"]}
+# compiled without multiply-add contraction (ns_host.cu: its host code, the CCD
+# factors).
+FILE_FLAGS = {"momentum.cu": ["-fmad=false"], "ccd.cu": ["-fmad=false"],
+              "ns_host.cu": ["-Xcompiler", "-ffp-contract=off"]}
 
 
 def nvcc():

@@ -6,171 +6,297 @@
 //
 // Every line of the ghost-padded box along an axis (L = n + 2g points, every
 // other index over its padded range) is one block tridiagonal system for
-// (f', f'').  Its matrix depends only on L and h, so k_ccd_decompose factors
-// it once per axis (one thread, the reference's operations in order) into a
-// table of 14 doubles per point that every line reads: the forward factors
-// (row 1), the back-substitution factors (row 3), the diagonal blocks (row 2)
-// and the block determinant with its IEEE reciprocal.  k_ccd_lines runs one
-// line per thread: the right-hand side (asgn_src_ccd) is formed on the fly in
-// the forward sweep from a sliding window of f, and the back substitution
-// reads the swept values back.  Lines along y and z are coalesced (adjacent
-// threads are adjacent in x); lines along x read with stride, served from L1.
+// (f', f'').  Its matrix depends only on L and h, so ccd_factor (host) factors
+// it once per axis (the reference's operations in order) into a table of 16
+// doubles per point that every line reads: the forward factors (row 1), the
+// back-substitution factors (row 3), the diagonal blocks (row 2), the block
+// determinant and its reciprocals.  k_ccd_lines runs one line per thread: the
+// right-hand side (asgn_src_ccd) is formed on the fly in the forward sweep from
+// a sliding window of f, and the back substitution reads the swept values
+// back; the loads of a batch of points are issued a batch ahead.  Lines along
+// y and z are coalesced (adjacent threads are adjacent in x); lines along x
+// read with stride, served from L1.
+//
+// A sweep is a chain of dependent operations, so what bounds it depends on the
+// number of lines.  Where they fill the GPU it is the FP64 pipe, and part of
+// the work runs on the integer pipes (k_ccd_lines: 21 FP64 operations per point
+// for 53); where they do not (2D) it is the chain of one warp, which
+// k_ccd_lines4 shortens by giving a line four lanes.
 // k_ccd_bc fills the ghost layers by zero-gradient copies (bc), k_curvature
 // forms the curvature on the interior.
 //
-// FP64 in the reference's operand order, compiled with -fmad=false;
-// quotients by h, h^2 and the block determinants come from correctly rounded
-// reciprocals (fdiv.cuh), so the derivatives equal the oracle's bit for bit.
+// FP64 in the reference's operand order, compiled with -fmad=false; quotients
+// and products off the FP64 pipe round the same (idiv.h), so the derivatives
+// equal the oracle's bit for bit.
 // The curvature's (|grad phi|^2 + 1e-12)^1.5 is formed as s * sqrt(s): sqrt is
 // correctly rounded, so the power is within two roundings of exact (the
 // reference's pow is within about one), at a fraction of pow's FP64 cost.
 #include <algorithm>
+#include <cmath>
 
-#include "fdiv.cuh"
 #include "gbmg_internal.h"
+#include "idiv.h"
 #include "reduce.cuh"
 
 namespace gbmg {
 
 namespace {
 
-constexpr int kRec = 14;  // doubles per point of the factor table
-
-// table layout per point i: A1 B1 AA1 BB1 | A3 B3 AA3 BB3 | A2 B2 AA2 BB2 | den rden
-__global__ void k_ccd_decompose(int L, double h, double* __restrict__ work,
-                                double* __restrict__ table) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  double* A = work;
-  double* B = work + 3 * (size_t)L;
-  double* AA = work + 6 * (size_t)L;
-  double* BB = work + 9 * (size_t)L;
-#define M_(X, r, i) X[((r) - 1) * (size_t)L + (i)]
-  const int is = 0, ie = L - 1;
-  // working_matrix_bc
-  M_(A, 2, is) = 1.0; M_(B, 2, is) = 0.0; M_(AA, 2, is) = 0.0; M_(BB, 2, is) = 1.0;
-  M_(A, 3, is) = 2.0; M_(B, 3, is) = -h; M_(AA, 3, is) = -(2.5 / h); M_(BB, 3, is) = 8.5;
-  M_(A, 2, ie) = 1.0; M_(B, 2, ie) = 0.0; M_(AA, 2, ie) = 0.0; M_(BB, 2, ie) = 1.0;
-  M_(A, 1, ie) = 2.0; M_(B, 1, ie) = h; M_(AA, 1, ie) = 2.5 / h; M_(BB, 1, ie) = 8.5;
-  // working_matrix_init_ccd
-  for (int i = is + 1; i <= ie - 1; ++i) {
-    M_(A, 1, i) = 7.0 / 16.0; M_(A, 2, i) = 1.0; M_(A, 3, i) = 7.0 / 16.0;
-    M_(B, 1, i) = h / 16.0; M_(B, 2, i) = 0.0; M_(B, 3, i) = -(h / 16.0);
-    M_(AA, 1, i) = -(9.0 / 8.0 / h); M_(AA, 2, i) = 0.0; M_(AA, 3, i) = 9.0 / 8.0 / h;
-    M_(BB, 1, i) = -(1.0 / 8.0); M_(BB, 2, i) = 1.0; M_(BB, 3, i) = -(1.0 / 8.0);
+// f(i) of the batch of kU points from i0, clamped to the line's end
+constexpr int kU = 4;
+__device__ __forceinline__ void ccd_load(const double* p, int64_t st, int i0, int step, int L,
+                                         double (&v)[kU]) {
+#pragma unroll
+  for (int u = 0; u < kU; ++u) {
+    int i = i0 + u * step;
+    i = i < 0 ? 0 : (i >= L ? L - 1 : i);
+    v[u] = p[(int64_t)i * st];
   }
-  // TWIN_DEC
-  M_(A, 1, is) = 0.0; M_(AA, 1, is) = 0.0; M_(A, 3, ie) = 0.0; M_(AA, 3, ie) = 0.0;
-  M_(B, 1, is) = 0.0; M_(BB, 1, is) = 0.0; M_(B, 3, ie) = 0.0; M_(BB, 3, ie) = 0.0;
-  for (int i = is + 1; i <= ie; ++i) {
-    const double den = M_(A, 2, i - 1) * M_(BB, 2, i - 1) - M_(AA, 2, i - 1) * M_(B, 2, i - 1);
-    double sc1 = -((M_(AA, 2, i - 1) * M_(B, 1, i) - M_(A, 1, i) * M_(BB, 2, i - 1)) / den);
-    double sc2 = (M_(B, 1, i) * M_(A, 2, i - 1) - M_(B, 2, i - 1) * M_(A, 1, i)) / den;
-    M_(A, 1, i) = sc1;
-    M_(A, 2, i) = M_(A, 2, i) - (sc1 * M_(A, 3, i - 1) + sc2 * M_(AA, 3, i - 1));
-    M_(B, 1, i) = sc2;
-    M_(B, 2, i) = M_(B, 2, i) - (sc1 * M_(B, 3, i - 1) + sc2 * M_(BB, 3, i - 1));
-    sc1 = -((M_(AA, 2, i - 1) * M_(BB, 1, i) - M_(AA, 1, i) * M_(BB, 2, i - 1)) / den);
-    sc2 = (M_(BB, 1, i) * M_(A, 2, i - 1) - M_(B, 2, i - 1) * M_(AA, 1, i)) / den;
-    M_(AA, 1, i) = sc1;
-    M_(AA, 2, i) = M_(AA, 2, i) - (sc1 * M_(A, 3, i - 1) + sc2 * M_(AA, 3, i - 1));
-    M_(BB, 1, i) = sc2;
-    M_(BB, 2, i) = M_(BB, 2, i) - (sc1 * M_(B, 3, i - 1) + sc2 * M_(BB, 3, i - 1));
-  }
-  for (int i = 0; i < L; ++i) {
-    double* t = table + (size_t)i * kRec;
-    t[0] = M_(A, 1, i); t[1] = M_(B, 1, i); t[2] = M_(AA, 1, i); t[3] = M_(BB, 1, i);
-    t[4] = M_(A, 3, i); t[5] = M_(B, 3, i); t[6] = M_(AA, 3, i); t[7] = M_(BB, 3, i);
-    t[8] = M_(A, 2, i); t[9] = M_(B, 2, i); t[10] = M_(AA, 2, i); t[11] = M_(BB, 2, i);
-    // the determinant of TWIN_BKS's diagonal block (the same products there)
-    t[12] = M_(A, 2, i) * M_(BB, 2, i) - M_(AA, 2, i) * M_(B, 2, i);
-    t[13] = 1.0 / t[12];
-  }
-#undef M_
 }
 
-__device__ __forceinline__ double qh(const CcdArgs& c, double x, double h, double rh) {
-  return c.fast ? div_known(x, h, rh) : x / h;
+__device__ __forceinline__ double ccd_over(const ConstDiv& c, double x) { return div_const_i(c, x); }
+// 15/16 x
+__device__ __forceinline__ double ccd_1516(double x) {
+  if (((unsigned)(__double2hiint(x) >> 20) & 0x7ffu) - 64u < 1900u) return scale2<-4>(mul_k<15>(x));
+  return __dmul_rn(0.9375, x);
 }
 
-// One line per thread.  Lines: line = i1 + n1 * i2, the line's first point
-// at i1 s1 + i2 s2 from the box origin, points st apart.
+// x over the block determinant of a table row
+__device__ __forceinline__ double ccd_det_int(const double* __restrict__ t, double x) {
+  const double den = __ldg(t + 12);
+  RcpInt r;
+  r.b = den;
+  r.y = (uint64_t)__double_as_longlong(__ldg(t + 15));
+  const uint64_t u = (uint64_t)__double_as_longlong(den);
+  r.m = (u & 0xfffffffffffffull) | (1ull << 52);
+  r.e = r.y != 0 ? (int)(u >> 52) : 0;
+  return div_int(x, r);
+}
+
+// the same in two dependent FP64 operations
+__device__ __forceinline__ double ccd_det(const double* __restrict__ t, double x) {
+  const double yl = __ldg(t + 14);
+  if (yl != 0.0 && ((unsigned)(__double2hiint(x) >> 20) & 0x7ffu) - 123u < 1800u)
+    return __fma_rn(x, __ldg(t + 13), __dmul_rn(x, yl));
+  return idiv_ieee(x, __ldg(t + 12));
+}
+
+// a pass and the pointers of one of its lines: line = i1 + n1 * i2, its first
+// point at i1 s1 + i2 s2 from the box origin
+struct CcdLine {
+  const double* f;
+  double *S, *SS;
+};
+__device__ __forceinline__ CcdLine ccd_line(const CcdBatch& batch, const CcdArgs& c, int pass,
+                                            int line) {
+  const int i1 = line % c.n1, i2 = line / c.n1;
+  const int64_t base = (int64_t)i1 * c.s1 + (int64_t)i2 * c.s2;
+  return CcdLine{batch.f[pass] + base, batch.S[pass] + base, batch.SS[pass] + base};
+}
+
+// right-hand sides at the ends (the high end's first one negated)
+__device__ __forceinline__ void ccd_end(const CcdArgs& c, double f0, double f1, double f2, double f3,
+                                        double* s, double* ss) {
+  *s = ccd_over(c.hd, (-3.5 * f0 + 4.0 * f1) - 0.5 * f2);
+  *ss = ccd_over(c.h2d, ((34.0 / 3.0 * f0 - 83.0 / 4.0 * f1) + 10.0 * f2) - 7.0 / 12.0 * f3);
+}
+
+// Many lines: one line per thread, bound by the arithmetic pipes.  The back
+// substitution keeps its products in FP64: with the forward sweep's and all
+// quotients on the integer pipes the two kinds of pipe take about as long
+// (curvature of 192x128x256 cells 5.43 ms before, now 2.74; 3.04 with every
+// product on the integer pipes, 3.30 with none; 256^3 6.50, 6.45, 7.21).
 __global__ void __launch_bounds__(128) k_ccd_lines(CcdBatch batch) {
   const int pass = blockIdx.y;
   const CcdArgs& c = batch.c[pass];
   const double* __restrict__ table = batch.table[pass];
-  const double* __restrict__ f = batch.f[pass];
-  double* __restrict__ S = batch.S[pass];
-  double* __restrict__ SS = batch.SS[pass];
   const int line = blockIdx.x * blockDim.x + threadIdx.x;
   if (line >= c.n1 * c.n2) return;
-  const int i1 = line % c.n1, i2 = line / c.n1;
-  const int64_t base = (int64_t)i1 * c.s1 + (int64_t)i2 * c.s2;
   const int64_t st = c.st;
   const int L = c.L;
-  const double* fl = f + base;
-  double* Sl = S + base;
-  double* SSl = SS + base;
-  const double h = c.h, h2 = c.h2;
+  const CcdLine P = ccd_line(batch, c, pass, line);
+  const double* __restrict__ fl = P.f;
+  double* __restrict__ Sl = P.S;
+  double* __restrict__ SSl = P.SS;
   // forward sweep with the right-hand side of asgn_src_ccd formed on the fly
-  double fm = fl[0], fc = fl[st], fp = fl[2 * st];
-  double s = qh(c, (-3.5 * fm + 4.0 * fc) - 0.5 * fp, h, c.rh);
-  double ss = qh(c, ((34.0 / 3.0 * fm - 83.0 / 4.0 * fc) + 10.0 * fp) - 7.0 / 12.0 * fl[3 * st],
-                 h2, c.rh2);
+  double fm = fl[0], fc = fl[st];
+  double s, ss;
+  ccd_end(c, fm, fc, fl[2 * st], fl[3 * st], &s, &ss);
   Sl[0] = s;
   SSl[0] = ss;
-  for (int i = 1; i < L - 1; ++i) {
-    const double* t = table + (size_t)i * kRec;
-    const double a1 = __ldg(t), b1 = __ldg(t + 1), aa1 = __ldg(t + 2), bb1 = __ldg(t + 3);
-    if (i > 1) {
+  double tm = mul_k<3>(fm), tc = mul_k<3>(fc);
+  double nf[kU];
+  ccd_load(fl, st, 2, 1, L, nf);
+  for (int i0 = 1; i0 < L - 1; i0 += kU) {
+    double cf[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) cf[u] = nf[u];
+    ccd_load(fl, st, i0 + 1 + kU, 1, L, nf);
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int i = i0 + u;
+      if (i >= L - 1) break;
+      const double* t = table + (size_t)i * kCcdRec;
+      const double fp = cf[u], tp = mul_k<3>(fp);
+      // 15/16 (f+ - f-)/h and ((3 f- - 6 f) + 3 f+)/h^2, 6 f = 2 (3 f) exactly
+      double sn = ccd_over(c.hd, ccd_1516(fp - fm));
+      double ssn = ccd_over(c.h2d, __fma_rn(-2.0, tc, tm) + tp);
+      sn = sn - (mul_int(__ldg(t), s) + mul_int(__ldg(t + 1), ss));
+      ssn = ssn - (mul_int(__ldg(t + 2), s) + mul_int(__ldg(t + 3), ss));
+      s = sn;
+      ss = ssn;
+      Sl[(int64_t)i * st] = s;
+      SSl[(int64_t)i * st] = ss;
       fm = fc;
       fc = fp;
-      fp = fl[(int64_t)(i + 1) * st];
+      tm = tc;
+      tc = tp;
     }
-    double sn = qh(c, 15.0 / 16.0 * (-fm + fp), h, c.rh);
-    double ssn = qh(c, (3.0 * fm - 6.0 * fc) + 3.0 * fp, h2, c.rh2);
-    sn = sn - (a1 * s + b1 * ss);
-    ssn = ssn - (aa1 * s + bb1 * ss);
-    s = sn;
-    ss = ssn;
-    Sl[(int64_t)i * st] = s;
-    SSl[(int64_t)i * st] = ss;
-  }
-  {
-    const int i = L - 1;
-    const double* t = table + (size_t)i * kRec;
-    const double f0 = fl[(int64_t)i * st], f1 = fl[(int64_t)(i - 1) * st];
-    const double f2 = fl[(int64_t)(i - 2) * st], f3 = fl[(int64_t)(i - 3) * st];
-    double sn = -qh(c, (-3.5 * f0 + 4.0 * f1) - 0.5 * f2, h, c.rh);
-    double ssn = qh(c, ((34.0 / 3.0 * f0 - 83.0 / 4.0 * f1) + 10.0 * f2) - 7.0 / 12.0 * f3, h2,
-                    c.rh2);
-    sn = sn - (__ldg(t) * s + __ldg(t + 1) * ss);
-    ssn = ssn - (__ldg(t + 2) * s + __ldg(t + 3) * ss);
-    s = sn;
-    ss = ssn;
   }
   // back substitution (TWIN_BKS)
   double sol, sol2;
   {
-    const double* t = table + (size_t)(L - 1) * kRec;
-    const double a2 = __ldg(t + 8), b2 = __ldg(t + 9), aa2 = __ldg(t + 10), bb2 = __ldg(t + 11);
-    const double den = __ldg(t + 12), rden = __ldg(t + 13);
-    sol = -div_known_checked(b2 * ss - bb2 * s, den, rden);
-    sol2 = div_known_checked(a2 * ss - aa2 * s, den, rden);
-    Sl[(int64_t)(L - 1) * st] = sol;
-    SSl[(int64_t)(L - 1) * st] = sol2;
+    const int i = L - 1;
+    const double* t = table + (size_t)i * kCcdRec;
+    double sn, ssn;
+    ccd_end(c, fl[(int64_t)i * st], fl[(int64_t)(i - 1) * st], fl[(int64_t)(i - 2) * st],
+            fl[(int64_t)(i - 3) * st], &sn, &ssn);
+    sn = -sn - (__ldg(t) * s + __ldg(t + 1) * ss);
+    ssn = ssn - (__ldg(t + 2) * s + __ldg(t + 3) * ss);
+    sol = -ccd_det_int(t, __ldg(t + 9) * ssn - __ldg(t + 11) * sn);
+    sol2 = ccd_det_int(t, __ldg(t + 8) * ssn - __ldg(t + 10) * sn);
+    Sl[(int64_t)i * st] = sol;
+    SSl[(int64_t)i * st] = sol2;
   }
-  for (int i = L - 2; i >= 0; --i) {
-    const double* t = table + (size_t)i * kRec;
-    const int64_t o = (int64_t)i * st;
-    double si = Sl[o], ssi = SSl[o];
-    si = si - (__ldg(t + 4) * sol + __ldg(t + 5) * sol2);
-    ssi = ssi - (__ldg(t + 6) * sol + __ldg(t + 7) * sol2);
-    const double a2 = __ldg(t + 8), b2 = __ldg(t + 9), aa2 = __ldg(t + 10), bb2 = __ldg(t + 11);
-    const double den = __ldg(t + 12), rden = __ldg(t + 13);
-    sol = -div_known_checked(b2 * ssi - bb2 * si, den, rden);
-    sol2 = div_known_checked(a2 * ssi - aa2 * si, den, rden);
-    Sl[o] = sol;
-    SSl[o] = sol2;
+  double ns[kU], nss[kU];
+  ccd_load(Sl, st, L - 2, -1, L, ns);
+  ccd_load(SSl, st, L - 2, -1, L, nss);
+  for (int i0 = L - 2; i0 >= 0; i0 -= kU) {
+    double cs[kU], css[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      cs[u] = ns[u];
+      css[u] = nss[u];
+    }
+    ccd_load(Sl, st, i0 - kU, -1, L, ns);
+    ccd_load(SSl, st, i0 - kU, -1, L, nss);
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int i = i0 - u;
+      if (i < 0) break;
+      const double* t = table + (size_t)i * kCcdRec;
+      const double si = cs[u] - (__dmul_rn(__ldg(t + 4), sol) + __dmul_rn(__ldg(t + 5), sol2));
+      const double ssi = css[u] - (__dmul_rn(__ldg(t + 6), sol) + __dmul_rn(__ldg(t + 7), sol2));
+      sol = -ccd_det_int(t, __dmul_rn(__ldg(t + 9), ssi) - __dmul_rn(__ldg(t + 11), si));
+      sol2 = ccd_det_int(t, __dmul_rn(__ldg(t + 8), ssi) - __dmul_rn(__ldg(t + 10), si));
+      Sl[(int64_t)i * st] = sol;
+      SSl[(int64_t)i * st] = sol2;
+    }
+  }
+}
+
+// Few lines: the chain of dependent operations along a line is what takes the
+// time (a warp's FP64 instruction takes as long for one line as for 32).  Four
+// lanes share a line: each forms one of the four products of a block row and
+// the right-hand side of one point of every four, so a point costs the warp
+// its chain of 3 + 7 FP64 instructions and 2 for the right-hand side, not 35
+// (curvature of 128x256 cells 1.23 ms before, now 0.57).
+__global__ void __launch_bounds__(32) k_ccd_lines4(CcdBatch batch) {
+  const int pass = blockIdx.y;
+  const CcdArgs& c = batch.c[pass];
+  const double* __restrict__ table = batch.table[pass];
+  const int lines = c.n1 * c.n2;
+  const int own = blockIdx.x * 8 + (threadIdx.x >> 2);
+  if (blockIdx.x * 8 >= lines) return;  // (whole warps only: lanes exchange values)
+  const bool live = own < lines;
+  const int r = threadIdx.x & 3;  // the lane's product, and its point of a batch
+  const bool odd = r & 1, low = r < 2;
+  const int64_t st = c.st;
+  const int L = c.L;
+  const CcdLine P = ccd_line(batch, c, pass, live ? own : lines - 1);
+  const double* __restrict__ fl = P.f;
+  double* __restrict__ Sl = P.S;
+  double* __restrict__ SSl = P.SS;
+  const unsigned all = 0xffffffffu;
+  const bool put_s = live && r == 0, put_ss = live && r == 2;
+  double s, ss;
+  ccd_end(c, fl[0], fl[st], fl[2 * st], fl[3 * st], &s, &ss);
+  if (put_s) Sl[0] = s;
+  if (put_ss) SSl[0] = ss;
+  // f(i-1), f(i), f(i+1) of the lane's point i0 + r, a batch ahead
+  double n0, n1, n2;
+  const auto load = [&](int i0) {
+    const int i = i0 + r < L - 2 ? i0 + r : L - 2;
+    n0 = fl[(int64_t)(i - 1) * st];
+    n1 = fl[(int64_t)i * st];
+    n2 = fl[(int64_t)(i + 1) * st];
+  };
+  load(1);
+  for (int i0 = 1; i0 < L - 1; i0 += 4) {
+    const double rs = div_const(c.hd, __dmul_rn(0.9375, n2 - n0));
+    const double rss =
+        div_const(c.h2d, __fma_rn(-2.0, __dmul_rn(3.0, n1), __dmul_rn(3.0, n0)) + __dmul_rn(3.0, n2));
+    load(i0 + 4);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u;
+      if (i >= L - 1) break;
+      const double a = __shfl_sync(all, rs, u, 4), b = __shfl_sync(all, rss, u, 4);
+      const double m = __dmul_rn(__ldg(table + (size_t)i * kCcdRec + r), odd ? ss : s);
+      const double v = (low ? a : b) - (m + __shfl_xor_sync(all, m, 1));
+      const double o = __shfl_xor_sync(all, v, 2);
+      s = low ? v : o;
+      ss = low ? o : v;
+      if (put_s) Sl[(int64_t)i * st] = s;
+      if (put_ss) SSl[(int64_t)i * st] = ss;
+    }
+  }
+  // back substitution (TWIN_BKS)
+  double sol, sol2;
+  {
+    const int i = L - 1;
+    const double* t = table + (size_t)i * kCcdRec;
+    double sn, ssn;
+    ccd_end(c, fl[(int64_t)i * st], fl[(int64_t)(i - 1) * st], fl[(int64_t)(i - 2) * st],
+            fl[(int64_t)(i - 3) * st], &sn, &ssn);
+    sn = -sn - (__ldg(t) * s + __ldg(t + 1) * ss);
+    ssn = ssn - (__ldg(t + 2) * s + __ldg(t + 3) * ss);
+    sol = -ccd_det(t, __ldg(t + 9) * ssn - __ldg(t + 11) * sn);
+    sol2 = ccd_det(t, __ldg(t + 8) * ssn - __ldg(t + 10) * sn);
+    if (put_s) Sl[(int64_t)i * st] = sol;
+    if (put_ss) SSl[(int64_t)i * st] = sol2;
+  }
+  __syncwarp();  // the lanes read back each other's swept values
+  const int k2 = low ? (odd ? 11 : 9) : (odd ? 10 : 8);
+  double ns, nss;
+  const auto back = [&](int i0) {
+    const int i = i0 - r > 0 ? i0 - r : 0;
+    ns = Sl[(int64_t)i * st];
+    nss = SSl[(int64_t)i * st];
+  };
+  back(L - 2);
+  for (int i0 = L - 2; i0 >= 0; i0 -= 4) {
+    const double cs = ns, css = nss;
+    back(i0 - 4);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 - u;
+      if (i < 0) break;
+      const double* t = table + (size_t)i * kCcdRec;
+      const double a = __shfl_sync(all, cs, u, 4), b = __shfl_sync(all, css, u, 4);
+      double m = __dmul_rn(__ldg(t + 4 + r), odd ? sol2 : sol);
+      double v = (low ? a : b) - (m + __shfl_xor_sync(all, m, 1));
+      double o = __shfl_xor_sync(all, v, 2);
+      // even lanes take ssi = the high pair's value, odd ones si = the low pair's
+      m = __dmul_rn(__ldg(t + k2), low == odd ? v : o);
+      o = __shfl_xor_sync(all, m, 1);
+      v = ccd_det(t, (odd ? o : m) - (odd ? m : o));
+      o = __shfl_xor_sync(all, v, 2);
+      sol = -(low ? v : o);
+      sol2 = low ? o : v;
+      if (put_s) Sl[(int64_t)i * st] = sol;
+      if (put_ss) SSl[(int64_t)i * st] = sol2;
+    }
   }
 }
 
@@ -224,18 +350,24 @@ __global__ void __launch_bounds__(256) k_curvature(NsArgs a, const double* __res
   const int k = blockIdx.z + 1;
   if (i > a.nx || j > a.ny) return;
   const int64_t q = (int64_t)(i - 1) + (int64_t)(j - 1) * a.sy + (int64_t)(k - 1) * a.sz;
+  // (products, the root and the quotient on the integer pipes: 14 FP64
+  // operations in 3D where the formula takes 33 and a root and a division)
   const double fx = fx_[q], fy = fy_[q];
+  const double xx = mul_int(fx, fx), yy = mul_int(fy, fy);
   if (!kThree) {
-    const double num = (fyy[q] * (fx * fx) + fxx[q] * (fy * fy)) - 2.0 * fxy[q] * fx * fy;
-    const double sq = (fx * fx + fy * fy) + 1.0e-12;
-    curv[q] = num / (sq * sqrt(sq));
+    const double num = (mul_int(fyy[q], xx) + mul_int(fxx[q], yy)) -
+                       mul_int(mul_int(scale2<1>(fxy[q]), fx), fy);
+    const double sq = (xx + yy) + 1.0e-12;
+    curv[q] = div_int(num, rcp_int(mul_int(sq, sqrt_int(sq))));
   } else {
-    const double fz = fz_[q];
-    const double num = (((fyy[q] + fzz[q]) * (fx * fx) + (fxx[q] + fzz[q]) * (fy * fy)) +
-                        (fxx[q] + fyy[q]) * (fz * fz)) -
-                       2.0 * ((fxy[q] * fx * fy + fxz[q] * fx * fz) + fyz[q] * fy * fz);
-    const double sq = ((fx * fx + fy * fy) + fz * fz) + 1.0e-12;
-    curv[q] = num / (sq * sqrt(sq));
+    const double fz = fz_[q], zz = mul_int(fz, fz);
+    const double a2 = fxx[q], b2 = fyy[q], c2 = fzz[q];
+    const double num =
+        ((mul_int(b2 + c2, xx) + mul_int(a2 + c2, yy)) + mul_int(a2 + b2, zz)) -
+        scale2<1>((mul_int(mul_int(fxy[q], fx), fy) + mul_int(mul_int(fxz[q], fx), fz)) +
+                  mul_int(mul_int(fyz[q], fy), fz));
+    const double sq = ((xx + yy) + zz) + 1.0e-12;
+    curv[q] = div_int(num, rcp_int(mul_int(sq, sqrt_int(sq))));
   }
 }
 
@@ -262,19 +394,34 @@ __device__ __forceinline__ void mp_funs(double phi, double ls_wid, double* heavy
 // mass_preserving_level_set's sums over the interior (ls_mv's mass and the
 // lambda denominator): acc[0] = sum rho H dv, acc[1] = sum delta^2 |grad phi|
 // (2 (1 - rho_12) H + rho_12) dv; |grad phi| from the compact gradient.
+// Beyond the band (|phi| > out, as bits; ls_outside_bits) H is 0 or 1 and delta
+// 0: a cell adds dv or nothing to the first sum and, its gradient being finite,
+// nothing to the second.
+__device__ __forceinline__ bool mp_outside(long long out, double phi) {
+  const long long m = __double_as_longlong(phi) & 0x7fffffffffffffffll;
+  return m > out && m <= 0x7ff0000000000000ll;
+}
+
 __global__ void __launch_bounds__(kRedThreads) k_mpls_sums(NsArgs a, const double* phi,
                                                            const double* gx, const double* gy,
                                                            const double* gz, double ls_wid,
-                                                           double rho_12, double dv,
-                                                           ReduceScratch R) {
+                                                           long long out, double rho_12,
+                                                           double dv, ReduceScratch R) {
   double acc[2] = {0.0, 0.0};
   const int rows = a.ny * a.nz;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const int j = row % a.ny + 1, k = row / a.ny + 1;
     for (int i = threadIdx.x + 1; i <= a.nx; i += blockDim.x) {
       const int64_t q = (int64_t)(i - 1) + (int64_t)(j - 1) * a.sy + (int64_t)(k - 1) * a.sz;
+      const double ph = phi[q];
+      if (mp_outside(out, ph) &&
+          (!gx || max(max(idiv_mag(gx[q]), idiv_mag(gy[q])), gz ? idiv_mag(gz[q]) : 0u) <
+                      (1023u + 400u) << 20)) {
+        if (__double_as_longlong(ph) >= 0) acc[0] += dv;
+        continue;
+      }
       double heavy, delta;
-      mp_funs(phi[q], ls_wid, &heavy, &delta);
+      mp_funs(ph, ls_wid, &heavy, &delta);
       const double rho = heavy + rho_12 * (1.0 - heavy);
       acc[0] += rho * heavy * dv;
       if (!gx) continue;  // the mass alone
@@ -293,17 +440,20 @@ __global__ void __launch_bounds__(kRedThreads) k_mpls_sums(NsArgs a, const doubl
 // phi += lam delta |grad phi| on the interior (delta of the phi before)
 __global__ void __launch_bounds__(256) k_mpls_update(NsArgs a, double* phi, const double* gx,
                                                      const double* gy, const double* gz,
-                                                     double ls_wid, double lam) {
+                                                     double ls_wid, long long out, double lam) {
   const int i = blockIdx.x * 32 + threadIdx.x + 1;
   const int j = blockIdx.y * 8 + threadIdx.y + 1;
   const int k = blockIdx.z + 1;
   if (i > a.nx || j > a.ny) return;
   const int64_t q = (int64_t)(i - 1) + (int64_t)(j - 1) * a.sy + (int64_t)(k - 1) * a.sz;
+  const double ph = phi[q];
+  const double x = gx[q], y = gy[q], z = gz ? gz[q] : 0.0;
+  if (mp_outside(out, ph) && max(max(idiv_mag(x), idiv_mag(y)), idiv_mag(z)) < (1023u + 400u) << 20)
+    return;  // delta = 0
   double heavy, delta;
-  mp_funs(phi[q], ls_wid, &heavy, &delta);
-  const double g2 = gz ? (gx[q] * gx[q] + gy[q] * gy[q]) + gz[q] * gz[q]
-                       : gx[q] * gx[q] + gy[q] * gy[q];
-  phi[q] = phi[q] + lam * delta * sqrt(g2);
+  mp_funs(ph, ls_wid, &heavy, &delta);
+  const double g2 = gz ? (x * x + y * y) + z * z : x * x + y * y;
+  phi[q] = ph + lam * delta * sqrt(g2);
 }
 
 // vof_wlic_solver's flux along axis ax at faces 0..n of that axis and rows
@@ -387,14 +537,16 @@ __global__ void __launch_bounds__(256) k_wlic_update(NsArgs a, int ax, int last,
 }
 }  // namespace
 
-void launch_ccd_decompose(cudaStream_t s, int L, double h, double* work, double* table) {
-  k_ccd_decompose<<<1, 1, 0, s>>>(L, h, work, table);
-}
-
 void launch_ccd_lines(cudaStream_t s, const CcdBatch& b) {
-  int lines = 0;
-  for (int i = 0; i < b.n; ++i) lines = std::max(lines, b.c[i].n1 * b.c[i].n2);
-  k_ccd_lines<<<dim3((unsigned)((lines + 127) / 128), (unsigned)b.n), 128, 0, s>>>(b);
+  int lines = 0, all = 0;
+  for (int i = 0; i < b.n; ++i) {
+    lines = std::max(lines, b.c[i].n1 * b.c[i].n2);
+    all += b.c[i].n1 * b.c[i].n2;
+  }
+  if (all >= kCcdManyLines)
+    k_ccd_lines<<<dim3((unsigned)((lines + 127) / 128), (unsigned)b.n), 128, 0, s>>>(b);
+  else  // one warp per block: the few warps spread over the SMs
+    k_ccd_lines4<<<dim3((unsigned)((lines + 7) / 8), (unsigned)b.n), 32, 0, s>>>(b);
 }
 
 void launch_ccd_bc(cudaStream_t s, const NsArgs& a, double* const f[4]) {
@@ -419,14 +571,16 @@ void launch_curvature(cudaStream_t s, const NsArgs& a, const double* const d1[3]
 void launch_mpls_sums(cudaStream_t s, const NsArgs& a, const double* phi, const double* const g[3],
                       double ls_wid, double rho_12, double dv, const ReduceScratch& R) {
   const int blocks = std::min(reduce_blocks_for((size_t)a.ny * a.nz), R.max_blocks);
-  k_mpls_sums<<<blocks, kRedThreads, 0, s>>>(a, phi, g[0], g[1], g[2], ls_wid, rho_12, dv, R);
+  const long long out = std::isfinite(rho_12) ? ls_outside_bits(ls_wid) : 0x7fffffffffffffffll;
+  k_mpls_sums<<<blocks, kRedThreads, 0, s>>>(a, phi, g[0], g[1], g[2], ls_wid, out, rho_12, dv, R);
 }
 
 void launch_mpls_update(cudaStream_t s, const NsArgs& a, double* phi, const double* const g[3],
                         double ls_wid, double lam) {
   const dim3 block(32, 8);
   const dim3 grid((unsigned)((a.nx + 31) / 32), (unsigned)((a.ny + 7) / 8), (unsigned)a.nz);
-  k_mpls_update<<<grid, block, 0, s>>>(a, phi, g[0], g[1], g[2], ls_wid, lam);
+  const long long out = std::isfinite(lam) ? ls_outside_bits(ls_wid) : 0x7fffffffffffffffll;
+  k_mpls_update<<<grid, block, 0, s>>>(a, phi, g[0], g[1], g[2], ls_wid, out, lam);
 }
 
 void launch_wlic(cudaStream_t s, const NsArgs& a, int ax, double* vof, const double* vof_old,

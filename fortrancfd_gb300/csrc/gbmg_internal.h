@@ -392,11 +392,17 @@ void launch_ns_change(cudaStream_t s, const NsArgs& a, const double* const now[3
 struct CcdArgs {
   int L, n1, n2;
   int64_t st, s1, s2;
-  double h, h2, rh, rh2;  // spacing, its square and their RN reciprocals
-  int fast;               // 1: quotients by h, h^2 from the reciprocals
+  ConstDiv hd, h2d;  // spacing and its square
 };
-// factor table of the CCD matrix for L points (14 doubles per point); work: 12 L doubles
-void launch_ccd_decompose(cudaStream_t s, int L, double h, double* work, double* table);
+// Factor table of the CCD matrix: per point A1 B1 AA1 BB1 | A3 B3 AA3 BB3 |
+// A2 B2 AA2 BB2 | det, 1/det, the rest of 1/det when a quotient by det is a
+// product and a multiply-add (idiv.h, kDivPair; else 0), and rcp_int's
+// significand as bits (0 when det is outside its range).
+constexpr int kCcdRec = 16;
+// Lines of one launch from which a thread takes a whole line: curvature of 64^3
+// cells (14,700 lines) 0.33 ms with four lanes per line against 0.37, of 96^3
+// (31,200) 0.95 against 0.68.
+constexpr int kCcdManyLines = 18000;
 // Up to three independent line passes in one launch (the grid's y index
 // picks the pass): f' into S and f'' into SS along every line of each pass
 // (box-origin pointers).

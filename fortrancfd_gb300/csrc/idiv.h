@@ -18,7 +18,8 @@
 //
 //   mul_int(a, b)  RN(a b) from the high half of the significands' product (the
 //                  low half is formed only when the high one ends in a tie);
-//   mul_k<K>(a)    RN(K a) for a small whole number K.
+//   mul_k<K>(a)    RN(K a) for a small whole number K;
+//   sqrt_int(a)    RN(sqrt(a)).
 //
 // One rcp_int serves all quotients with its divisor.  Subnormal, infinite or
 // NaN operands and results near the ends of the exponent range take the
@@ -257,6 +258,55 @@ GB_HD double scale2(double x) {
     return idiv_double(u + ((uint64_t)(int64_t)K << 52));
   return (u << 1) == 0 ? x : imul_ieee(x, K < 0 ? 1.0 / (double)(1ll << -K) : (double)(1ll << K));
 }
+
+#if defined(__CUDACC__)
+__host__ __device__ __noinline__ inline double isqrt_ieee(double a) { return sqrt(a); }
+#else
+inline double isqrt_ieee(double a) { return std::sqrt(a); }
+#endif
+
+// a float within 2^-22.9 (relative) of x^-1/2, x in [1, 4)
+GB_HD float isqrt_seed(float x) {
+#if defined(__CUDA_ARCH__)
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+#else
+  const float r = (float)(1.0 / std::sqrt((double)x));
+  return x == 1.0f ? r : idiv_float(idiv_fbits(r) + (uint32_t)idiv_seed_shift());
+#endif
+}
+
+// RN(sqrt(a)): a float square root, two steps s += (x - s^2)/(2 s) with exact
+// integer remainders (44 bits, then all), the last bit by the sign of
+// N - (K + 1/2)^2.
+GB_HD double sqrt_int(double a) {
+  const uint64_t u = idiv_bits(a);
+  const uint32_t ea = (uint32_t)(u >> 52);
+  if (ea - 1u >= 2046u) return isqrt_ieee(a);  // not positive, normal and finite
+  const int odd = (int)(~ea & 1u);  // odd exponent (the bias is odd)
+  const uint64_t m = ((u & 0xfffffffffffffull) | (1ull << 52)) << odd;  // x 2^52, x in [1, 4)
+  const float x = idiv_float((odd ? 0x40000000u : 0x3f800000u) | (uint32_t)((u >> 29) & 0x7fffffu));
+  const float r = isqrt_seed(x);
+  // r 2^31 and s0 2^31 (s0 = x r in [1, 2)) as integers
+  const uint32_t ri = (idiv_fbits(r) - 0x3f000000u + 0x800000u) << 7;
+  float s0 = x * r;
+  s0 = s0 < 1.0f ? 1.0f : (s0 > 1.9999999f ? 1.9999999f : s0);
+  const uint32_t si = ((idiv_fbits(s0) & 0x7fffffu) | 0x800000u) << 8;
+  const int64_t d0 = (int64_t)((m << 10) - (uint64_t)si * si);  // (x - s0^2) 2^62
+  const int64_t s1 = (int64_t)((uint64_t)si << 31) + (((int64_t)(int32_t)(d0 >> 13) * ri) >> 19);
+  const uint64_t h = (uint64_t)s1 >> 11;  // s 2^51
+  const int64_t d1 = (int64_t)((m << 50) - h * h);  // x 2^102 - h^2
+  uint64_t k = 2 * h + (uint64_t)(((int64_t)(int32_t)(d1 >> 31) * ri) >> 51);  // s 2^52, N = x 2^104
+  const int64_t d2 = (int64_t)((m << 52) - k * k);
+  k += (d2 > (int64_t)k ? 1u : 0u) - (uint64_t)(d2 <= -(int64_t)k ? 1u : 0u);
+  const uint32_t e = (ea + 1023u - (uint32_t)odd) >> 1;  // exponent of the root
+  return idiv_double(((uint64_t)(e - 1) << 52) + k);
+}
+
+// exponent field in place: larger for larger magnitudes, infinities and NaN on top
+GB_HD uint32_t idiv_mag(double x) { return (uint32_t)(idiv_bits(x) >> 32) & 0x7ff00000u; }
+constexpr uint32_t kMagOk = (1023u + 900u) << 20;  // below: |x| < 2^900
 
 // Bits of a magnitude slightly above ls_wid (1 - 1e-12): |phi| beyond it gives
 // |RN(phi/ls_wid)| > 1 - 1e-12, the clipping threshold of ls_funs, whatever the

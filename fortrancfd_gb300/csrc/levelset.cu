@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kLsThreads, 2)
                                      : larger(pos_part(v1), neg_part(v2));
   double sum = isq(v);
   if (kAxis > 0) sum = add(grad[q], sum);
-  if (kLast) sum = __dsqrt_rn(sum);
+  if (kLast) sum = sqrt_int(sum);
   grad[q] = sum;
   if (kLast && kLambda) {
     const double p = phi[q];

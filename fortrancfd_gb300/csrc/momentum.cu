@@ -58,11 +58,7 @@ __device__ __forceinline__ double overh(const ConstDiv& c, double x) { return di
 __device__ __forceinline__ bool is_zero(double x) {
   return ((unsigned long long)__double_as_longlong(x) << 1) == 0ull;
 }
-// exponent field in place: larger for larger magnitudes, infinities and NaN on top
-__device__ __forceinline__ unsigned mag(double x) {
-  return (unsigned)__double2hiint(x) & 0x7ff00000u;
-}
-constexpr unsigned kMagOk = (1023u + 900u) << 20;  // below: |x| < 2^900
+__device__ __forceinline__ unsigned mag(double x) { return idiv_mag(x); }
 // 2^-500 <= x < 2^500
 __device__ __forceinline__ bool mid_range(double x) {
   return (unsigned)(__double2hiint(x) >> 20) - 523u < 1000u;

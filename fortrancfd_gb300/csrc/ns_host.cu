@@ -12,6 +12,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <vector>
 
 #include "fdiv.cuh"
 #include "handle.h"
@@ -206,13 +207,68 @@ void ns_used(const gbmg_grid& g, const gbmg_ns_params* prm, bool (&used)[kNsFiel
 
 // Compact-difference normals and curvature (curv + surface_norms): scratch
 // slots after the momentum step's: the six second derivatives and a dummy
-// second derivative, then a factor table per axis and the factoring work.
+// second derivative, then a factor table per axis.
 constexpr int kCcdD2 = kNsDiff + 3, kCcdDummy = kCcdD2 + 6, kCcdTable = kCcdDummy + 1,
-              kCcdWork = kCcdTable + 3, kCcdSpare = kCcdWork + 1;  // two spare fields
+              kCcdSpare = kCcdTable + 3;  // two spare fields
 
-// One CCD line pass: its arguments, and the axis's factor table (made by
-// one sequential thread, so once, and kept while the line length and spacing
-// stay the same).
+// The CCD matrix of a line of L points (working_matrix_bc,
+// working_matrix_init_ccd) and its factors (TWIN_DEC), in the reference's
+// operation order, into the table k_ccd_lines reads.  On the host: one thread
+// of a GPU took 390 us for 262 points.  (This file's host code is compiled
+// without multiply-add contraction.)
+void ccd_factor(int L, double h, std::vector<double>* out) {
+  std::vector<double> w((size_t)12 * L);
+  double *A = w.data(), *B = A + 3 * (size_t)L, *AA = B + 3 * (size_t)L, *BB = AA + 3 * (size_t)L;
+#define M_(X, r, i) X[((r) - 1) * (size_t)L + (i)]
+  const int is = 0, ie = L - 1;
+  M_(A, 2, is) = 1.0; M_(B, 2, is) = 0.0; M_(AA, 2, is) = 0.0; M_(BB, 2, is) = 1.0;
+  M_(A, 3, is) = 2.0; M_(B, 3, is) = -h; M_(AA, 3, is) = -(2.5 / h); M_(BB, 3, is) = 8.5;
+  M_(A, 2, ie) = 1.0; M_(B, 2, ie) = 0.0; M_(AA, 2, ie) = 0.0; M_(BB, 2, ie) = 1.0;
+  M_(A, 1, ie) = 2.0; M_(B, 1, ie) = h; M_(AA, 1, ie) = 2.5 / h; M_(BB, 1, ie) = 8.5;
+  for (int i = is + 1; i <= ie - 1; ++i) {
+    M_(A, 1, i) = 7.0 / 16.0; M_(A, 2, i) = 1.0; M_(A, 3, i) = 7.0 / 16.0;
+    M_(B, 1, i) = h / 16.0; M_(B, 2, i) = 0.0; M_(B, 3, i) = -(h / 16.0);
+    M_(AA, 1, i) = -(9.0 / 8.0 / h); M_(AA, 2, i) = 0.0; M_(AA, 3, i) = 9.0 / 8.0 / h;
+    M_(BB, 1, i) = -(1.0 / 8.0); M_(BB, 2, i) = 1.0; M_(BB, 3, i) = -(1.0 / 8.0);
+  }
+  M_(A, 1, is) = 0.0; M_(AA, 1, is) = 0.0; M_(A, 3, ie) = 0.0; M_(AA, 3, ie) = 0.0;
+  M_(B, 1, is) = 0.0; M_(BB, 1, is) = 0.0; M_(B, 3, ie) = 0.0; M_(BB, 3, ie) = 0.0;
+  for (int i = is + 1; i <= ie; ++i) {
+    const double den = M_(A, 2, i - 1) * M_(BB, 2, i - 1) - M_(AA, 2, i - 1) * M_(B, 2, i - 1);
+    double sc1 = -((M_(AA, 2, i - 1) * M_(B, 1, i) - M_(A, 1, i) * M_(BB, 2, i - 1)) / den);
+    double sc2 = (M_(B, 1, i) * M_(A, 2, i - 1) - M_(B, 2, i - 1) * M_(A, 1, i)) / den;
+    M_(A, 1, i) = sc1;
+    M_(A, 2, i) = M_(A, 2, i) - (sc1 * M_(A, 3, i - 1) + sc2 * M_(AA, 3, i - 1));
+    M_(B, 1, i) = sc2;
+    M_(B, 2, i) = M_(B, 2, i) - (sc1 * M_(B, 3, i - 1) + sc2 * M_(BB, 3, i - 1));
+    sc1 = -((M_(AA, 2, i - 1) * M_(BB, 1, i) - M_(AA, 1, i) * M_(BB, 2, i - 1)) / den);
+    sc2 = (M_(BB, 1, i) * M_(A, 2, i - 1) - M_(B, 2, i - 1) * M_(AA, 1, i)) / den;
+    M_(AA, 1, i) = sc1;
+    M_(AA, 2, i) = M_(AA, 2, i) - (sc1 * M_(A, 3, i - 1) + sc2 * M_(AA, 3, i - 1));
+    M_(BB, 1, i) = sc2;
+    M_(BB, 2, i) = M_(BB, 2, i) - (sc1 * M_(B, 3, i - 1) + sc2 * M_(BB, 3, i - 1));
+  }
+  out->resize((size_t)L * kCcdRec);
+  ConstDiv c{};
+  for (int i = 0; i < L; ++i) {
+    double* t = out->data() + (size_t)i * kCcdRec;
+    t[0] = M_(A, 1, i); t[1] = M_(B, 1, i); t[2] = M_(AA, 1, i); t[3] = M_(BB, 1, i);
+    t[4] = M_(A, 3, i); t[5] = M_(B, 3, i); t[6] = M_(AA, 3, i); t[7] = M_(BB, 3, i);
+    t[8] = M_(A, 2, i); t[9] = M_(B, 2, i); t[10] = M_(AA, 2, i); t[11] = M_(BB, 2, i);
+    // the determinant of TWIN_BKS's diagonal block (the same products there);
+    // it settles within a few dozen points
+    t[12] = M_(A, 2, i) * M_(BB, 2, i) - M_(AA, 2, i) * M_(B, 2, i);
+    if (i == 0 || t[12] != c.h) c = const_div(t[12]);
+    t[13] = c.y;
+    t[14] = c.mode == kDivPair ? c.yl : 0.0;
+    const uint64_t y = c.r.e != 0 ? c.r.y : 0;
+    std::memcpy(&t[15], &y, sizeof y);
+  }
+#undef M_
+}
+
+// One CCD line pass: its arguments, and the axis's factor table (made once and
+// kept while the line length and spacing stay the same).
 int ccd_pass(gbmg_handle* h, const NsPlan& P, int axis, CcdArgs* out) {
   const NsArgs& a = P.a;
   const bool three = a.nz > 1;
@@ -226,21 +282,21 @@ int ccd_pass(gbmg_handle* h, const NsPlan& P, int axis, CcdArgs* out) {
   const int a1 = axis == 0 ? 1 : 0, a2 = axis == 2 ? 1 : 2;
   c.n1 = ext[a1]; c.s1 = str[a1];
   c.n2 = ext[a2]; c.s2 = str[a2];
-  c.h = hs[axis];
-  c.h2 = c.h * c.h;
-  c.rh = 1.0 / c.h;
-  c.rh2 = 1.0 / c.h2;
-  c.fast = fdiv_divisor_ok(c.h) && fdiv_divisor_ok(c.h2);
-  if (h->ccd_L[axis] != c.L || h->ccd_h[axis] != c.h) {
+  const double hx = hs[axis];
+  c.hd = const_div(hx);
+  c.h2d = const_div(hx * hx);
+  if (h->ccd_L[axis] != c.L || h->ccd_h[axis] != hx) {
     h->ccd_L[axis] = 0;
-    GB_TRY(ns_buffer(h, kCcdTable + axis, (size_t)14 * c.L));
-    GB_TRY(ns_buffer(h, kCcdWork, (size_t)12 * c.L));
-    LAUNCH(h, GBMG_PROF_MOMENTUM,
-           launch_ccd_decompose(h->stream, c.L, c.h, h->ns_buf[kCcdWork],
-                                h->ns_buf[kCcdTable + axis]));
-    GB_TRY(check_launch(h, "ccd factors"));
+    const size_t n = (size_t)kCcdRec * c.L;
+    GB_TRY(ns_buffer(h, kCcdTable + axis, n));
+    std::vector<double> table;
+    ccd_factor(c.L, hx, &table);
+    // (pageable memory: read before the call returns)
+    GB_CUDA(h, cudaMemcpyAsync(h->ns_buf[kCcdTable + axis], table.data(), n * sizeof(double),
+                               cudaMemcpyHostToDevice, h->stream));
+    GB_CUDA(h, cudaStreamSynchronize(h->stream));
     h->ccd_L[axis] = c.L;
-    h->ccd_h[axis] = c.h;
+    h->ccd_h[axis] = hx;
   }
   *out = c;
   return GBMG_OK;

@@ -1,6 +1,6 @@
 """The quotients formed without an FP64 division (fortrancfd_gb300/csrc/idiv.h:
 rcp_int / div_int, div_3, const_div / div_const) and the integer products
-(mul_int, mul_k), compiled as plain C++ and compared bit for bit with the
+and root (mul_int, mul_k, sqrt_int), compiled as plain C++ and compared bit for bit with the
 host's IEEE operations: random operands over the
 whole exponent range, quotients next to a rounding midpoint (random and solved
 for), zeros, subnormals, infinities and NaN, with the float seed of the
@@ -62,6 +62,14 @@ int main() {
       same(mul_k<7>(a), 7.0 * a, a, 7, "mul_k");
       same(mul_k<11>(a), 11.0 * a, a, 11, "mul_k");
       same(mul_k<13>(a), 13.0 * a, a, 13, "mul_k");
+      same(mul_k<15>(a), 15.0 * a, a, 15, "mul_k");
+      same(sqrt_int(std::fabs(a)), std::sqrt(std::fabs(a)), a, 0, "sqrt_int");
+      // squares of 53-bit values and their neighbours: roots next to a double
+      const double q = idiv_double((idiv_bits(a) & 0xfffffffffffffull) | (1023ull + i % 2) << 52);
+      for (int d = -2; d <= 2; ++d) {
+        const double sq = idiv_double(idiv_bits(q * q) + (uint64_t)(int64_t)d);
+        same(sqrt_int(sq), std::sqrt(sq), sq, 0, "sqrt_int square");
+      }
       same(scale2<-1>(a), 0.5 * a, a, 0.5, "scale2");
       same(scale2<-2>(a), 0.25 * a, a, 0.25, "scale2");
       same(scale2<1>(a), 2.0 * a, a, 2, "scale2");
@@ -69,6 +77,7 @@ int main() {
     for (double a : edge) {
       for (double b : edge) same(mul_int(a, b), a * b, a, b, "mul_int edge");
       same(mul_k<3>(a), 3.0 * a, a, 3, "mul_k edge");
+      same(sqrt_int(a), std::sqrt(a), a, 0, "sqrt_int edge");
       same(mul_k<13>(a), 13.0 * a, a, 13, "mul_k edge");
       same(scale2<-1>(a), 0.5 * a, a, 0.5, "scale2 edge");
       same(scale2<-2>(a), 0.25 * a, a, 0.25, "scale2 edge");
