@@ -362,15 +362,22 @@ GB_HD double div_const_i(const ConstDiv& c, double x) {
   return div_int(x, c.r);
 }
 
-inline ConstDiv const_div(double h) {
+// the constant for div_const_i alone (without const_div's search, about a
+// microsecond of the host)
+inline ConstDiv const_div_i(double h) {
   ConstDiv c{h, 1.0 / h, 0.0, kDivIeee, 0, rcp_int(h)};
-  if (!(std::fabs(h) >= 0x1p-60 && std::fabs(h) <= 0x1p60)) return c;
   int ex;
-  if (std::frexp(h, &ex) == 0.5) {
+  if (h >= 0x1p-60 && h <= 0x1p60 && std::frexp(h, &ex) == 0.5) {
     c.mode = kDivExact;
     c.ex = 1 - ex;
-    return c;
   }
+  return c;
+}
+
+inline ConstDiv const_div(double h) {
+  ConstDiv c = const_div_i(h);
+  if (c.mode == kDivExact || !(std::fabs(h) >= 0x1p-60 && std::fabs(h) <= 0x1p60)) return c;
+  int ex;
   c.mode = kDivKnown;
   if (!(h > 0)) return c;
   c.yl = std::fma(-h, c.y, 1.0) / h;

@@ -15,6 +15,7 @@
 
 #include "dword.cuh"
 #include "gbmg_internal.h"
+#include "idiv.h"
 #include "reduce.cuh"
 
 namespace gbmg {
@@ -39,6 +40,14 @@ inline unsigned stride_blocks(size_t n) {
 // rho_pos*1 + rho_neg*0 and rho_pos*0 + rho_neg*1 computed by the host: the
 // full formula's result for H = 1 and 0, without FP64 work.
 constexpr int kRhoPlanes = 4;
+
+// a divisor per axis (the spacings or their squares)
+struct Spacing {
+  ConstDiv d[3];
+};
+Spacing spacing(double x, double y, double z) {
+  return Spacing{{const_div_i(x), const_div_i(y), const_div_i(z)}};
+}
 
 __global__ void __launch_bounds__(256) k_rho_from_phi(int nx, int ny, int nz, Strided phi,
                                                       double eps, long long eps_out_bits,
@@ -95,9 +104,8 @@ __global__ void __launch_bounds__(256) k_copy_out(int nx, int ny, int nz, const 
 
 // coe = 2/(rho_i + rho_nb)/h^2 on the low face of every cell, 0 on the walls
 // (the reference's arithmetic, ns_ppe_solver.f90:12-24, so the operator is
-// bit-identical to the oracle's).  When h^2 is a power of two the division by
-// it is an exact scaling and is done as a multiplication by 1/h^2 (same
-// result, one FP64 division instead of two).  Optionally also writes the
+// bit-identical to the oracle's).  The quotients run on the integer pipes
+// (idiv.h; the FP64 pipe is what bounds these passes).  Optionally also writes the
 // FP32 copies of the cycle and the double-word copies of the defect kernel.
 struct BulkFaces {
   long long r[2];     // bit patterns of the two bulk densities (never equal to a double
@@ -128,8 +136,7 @@ __device__ __forceinline__ void face_store(const FaceOut& o, size_t q, double v)
 // ra, rb: the two cells' densities.  The bulk test compares bit patterns
 // (integer operations; FP64 compares and adds run at GB300's FP64 rate).
 __device__ __forceinline__ void face_value(const BulkFaces& B, int a, double ra, double rb,
-                                           double h2, double ih2, bool pow2, const FaceOut& o,
-                                           size_t q) {
+                                           const ConstDiv& h2, const FaceOut& o, size_t q) {
   const long long ba = __double_as_longlong(ra), bb = __double_as_longlong(rb);
   for (int v = 0; v < 2; ++v)
     if (ba == B.r[v] && bb == B.r[v]) {
@@ -138,12 +145,10 @@ __device__ __forceinline__ void face_value(const BulkFaces& B, int a, double ra,
       if (o.cw) o.cw[q] = B.cw[a][v];
       return;
     }
-  const double t = 2.0 / (ra + rb);
-  face_store(o, q, pow2 ? t * ih2 : t / h2);
+  face_store(o, q, div_const_i(h2, div_int(2.0, rcp_int(ra + rb))));
 }
 
-__global__ void __launch_bounds__(256) k_face_coef(int nx, int ny, int nz, double3 h2, double3 ih2,
-                                                   int pow2, BulkFaces B,
+__global__ void __launch_bounds__(256) k_face_coef(int nx, int ny, int nz, Spacing h2, BulkFaces B,
                                                    const double* __restrict__ rho, FaceOut ox,
                                                    FaceOut oy, FaceOut oz, float* rho32,
                                                    size_t hstride) {
@@ -157,47 +162,46 @@ __global__ void __launch_bounds__(256) k_face_coef(int nx, int ny, int nz, doubl
   // when hstride != 0)
   if (rho32) rho32[hstride ? (size_t)((i + j + k) & 1) * hstride + (q >> 1) : q] =
       dw_from_double_int(r).hi;
-  if (i > 0) face_value(B, 0, r, rho[q - 1], h2.x, ih2.x, pow2 & 1, ox, q);
+  if (i > 0) face_value(B, 0, r, rho[q - 1], h2.d[0], ox, q);
   else face_store(ox, q, 0.0);
-  if (j > 0) face_value(B, 1, r, rho[q - nx], h2.y, ih2.y, pow2 & 2, oy, q);
+  if (j > 0) face_value(B, 1, r, rho[q - nx], h2.d[1], oy, q);
   else face_store(oy, q, 0.0);
-  if (k > 0) face_value(B, 2, r, rho[q - (size_t)nx * ny], h2.z, ih2.z, pow2 & 4, oz, q);
+  if (k > 0) face_value(B, 2, r, rho[q - (size_t)nx * ny], h2.d[2], oz, q);
   else face_store(oz, q, 0.0);
 }
 
 // b = div(u)/dt with MAC faces: u(f,j,k) on the x-face at f*dx, f = 0..nx.
-// x / h, as a product with the exact reciprocal when h is a power of two
-// (bit-identical to the division and without its FP64 cost); pow2 is the
-// host's is_pow2(h), ih = 1/h.
-__device__ __forceinline__ double over(double x, double h, double ih, bool pow2) {
-  return pow2 ? x * ih : x / h;
-}
-
 __global__ void __launch_bounds__(256) k_divergence(int nx, int ny, int nz, Strided u, Strided v,
-                                                    Strided w, double3 h, double3 ih, int pow2,
-                                                    double dt, double* b) {
+                                                    Strided w, Spacing h, ConstDiv dt,
+                                                    double* b) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
   if (i >= nx || j >= ny) return;
   const int64_t qu = i + j * u.sy + k * u.sz;
   const int64_t qv = i + j * v.sy + k * v.sz;
-  double d = over(u.data[qu + 1] - u.data[qu], h.x, ih.x, pow2 & 1) +
-             over(v.data[qv + v.sy] - v.data[qv], h.y, ih.y, pow2 & 2);
+  double d = div_const_i(h.d[0], u.data[qu + 1] - u.data[qu]) +
+             div_const_i(h.d[1], v.data[qv + v.sy] - v.data[qv]);
   if (w.data) {
     const int64_t qw = i + j * w.sy + k * w.sz;
-    d += over(w.data[qw + w.sz] - w.data[qw], h.z, ih.z, pow2 & 4);
+    d += div_const_i(h.d[2], w.data[qw + w.sz] - w.data[qw]);
   }
-  b[((size_t)k * ny + j) * nx + i] = d / dt;
+  b[((size_t)k * ny + j) * nx + i] = div_const_i(dt, d);
 }
 
 // u_f -= dt (p_i - p_{i-1})/dx / ((rho_i + rho_{i-1})/2) on every interior
 // face; each cell corrects its low faces.
-// (halving is exact, so /2 is taken as *0.5)
+// (halving is exact, so /2 is taken as *0.5; three FP64 operations per face,
+// the rest on the integer pipes: 256^3 1.30 ms before)
+__device__ __forceinline__ double correction(double ra, double rb, double pa, double pb,
+                                             const ConstDiv& h, double dt) {
+  return div_int(mul_int(dt, div_const_i(h, pa - pb)), rcp_int(scale2<-1>(ra + rb)));
+}
+
 __global__ void __launch_bounds__(256) k_correct(int nx, int ny, int nz,
                                                  const double* __restrict__ rho,
-                                                 const double* __restrict__ p, double3 h,
-                                                 double3 ih, int pow2, double dt, double* u,
+                                                 const double* __restrict__ p, Spacing h,
+                                                 double dt, double* u,
                                                  int64_t usy, int64_t usz, double* v, int64_t vsy,
                                                  int64_t vsz, double* w, int64_t wsy, int64_t wsz) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -205,21 +209,12 @@ __global__ void __launch_bounds__(256) k_correct(int nx, int ny, int nz,
   const int k = blockIdx.z;
   if (i >= nx || j >= ny) return;
   const size_t q = ((size_t)k * ny + j) * nx + i;
-  if (i > 0) {
-    const double rf = (rho[q] + rho[q - 1]) * 0.5;
-    const double px = over(p[q] - p[q - 1], h.x, ih.x, pow2 & 1);
-    u[i + j * usy + k * usz] -= dt * px / rf;
-  }
-  if (j > 0) {
-    const double rf = (rho[q] + rho[q - nx]) * 0.5;
-    const double py = over(p[q] - p[q - nx], h.y, ih.y, pow2 & 2);
-    v[i + j * vsy + k * vsz] -= dt * py / rf;
-  }
+  const double r = rho[q], pq = p[q];
+  if (i > 0) u[i + j * usy + k * usz] -= correction(r, rho[q - 1], pq, p[q - 1], h.d[0], dt);
+  if (j > 0) v[i + j * vsy + k * vsz] -= correction(r, rho[q - nx], pq, p[q - nx], h.d[1], dt);
   if (k > 0 && w) {
     const size_t sz = (size_t)nx * ny;
-    const double rf = (rho[q] + rho[q - sz]) * 0.5;
-    const double pz = over(p[q] - p[q - sz], h.z, ih.z, pow2 & 4);
-    w[i + j * wsy + k * wsz] -= dt * pz / rf;
+    w[i + j * wsy + k * wsz] -= correction(r, rho[q - sz], pq, p[q - sz], h.d[2], dt);
   }
 }
 
@@ -264,24 +259,25 @@ __global__ void __launch_bounds__(256) k_adjoint(int nx, int ny, int nz, double3
 // max |div u| by atomicMax on the bit pattern (non-negative doubles order as
 // unsigned integers) and sum |div u| through the deterministic reducer.
 __global__ void __launch_bounds__(kRedThreads) k_div_stats(int nx, int ny, int nz, Strided u,
-                                                           Strided v, Strided w, double dx,
-                                                           double dy, double dz,
+                                                           Strided v, Strided w, Spacing h,
                                                            ReduceScratch R) {
   double acc[1] = {0.0};
-  double mx = 0.0;
+  double mx = 0.0;  // (compared as bits: non-negative, NaN never taken)
   const int rows = ny * nz;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const int j = row % ny, k = row / ny;
     for (int i = threadIdx.x; i < nx; i += blockDim.x) {
       const int64_t qu = i + j * u.sy + k * u.sz;
       const int64_t qv = i + j * v.sy + k * v.sz;
-      double d = (u.data[qu + 1] - u.data[qu]) / dx + (v.data[qv + v.sy] - v.data[qv]) / dy;
+      double d = div_const_i(h.d[0], u.data[qu + 1] - u.data[qu]) +
+                 div_const_i(h.d[1], v.data[qv + v.sy] - v.data[qv]);
       if (w.data) {
         const int64_t qw = i + j * w.sy + k * w.sz;
-        d += (w.data[qw + w.sz] - w.data[qw]) / dz;
+        d += div_const_i(h.d[2], w.data[qw + w.sz] - w.data[qw]);
       }
       d = fabs(d);
-      mx = fmax(mx, d);
+      const long long db = __double_as_longlong(d);
+      if (db > __double_as_longlong(mx) && db <= 0x7ff0000000000000ll) mx = d;
       acc[0] += d;
     }
   }
@@ -458,27 +454,22 @@ void launch_face_coef(cudaStream_t s, int nx, int ny, int nz, double dx2, double
   const FaceOut ox{cx, c32 ? c32[0] : nullptr, cw ? cw[0] : nullptr};
   const FaceOut oy{cy, c32 ? c32[1] : nullptr, cw ? cw[1] : nullptr};
   const FaceOut oz{cz, c32 ? c32[2] : nullptr, cw ? cw[2] : nullptr};
-  k_face_coef<<<grid3(nx, ny, nz), dim3(32, 8), 0, s>>>(
-      nx, ny, nz, make_double3(dx2, dy2, dz2), make_double3(1.0 / dx2, 1.0 / dy2, 1.0 / dz2), pow2,
-      B, rho, ox, oy, oz, rho32, hstride);
+  k_face_coef<<<grid3(nx, ny, nz), dim3(32, 8), 0, s>>>(nx, ny, nz, spacing(dx2, dy2, dz2), B, rho,
+                                                        ox, oy, oz, rho32, hstride);
 }
 
 void launch_divergence(cudaStream_t s, int nx, int ny, int nz, Strided u, Strided v, Strided w,
                        double dx, double dy, double dz, double dt, double* b) {
-  const int pow2 = (is_pow2(dx) ? 1 : 0) | (is_pow2(dy) ? 2 : 0) | (is_pow2(dz) ? 4 : 0);
-  k_divergence<<<grid3(nx, ny, nz), dim3(32, 8), 0, s>>>(
-      nx, ny, nz, u, v, w, make_double3(dx, dy, dz), make_double3(1.0 / dx, 1.0 / dy, 1.0 / dz),
-      pow2, dt, b);
+  k_divergence<<<grid3(nx, ny, nz), dim3(32, 8), 0, s>>>(nx, ny, nz, u, v, w,
+                                                         spacing(dx, dy, dz), const_div_i(dt), b);
 }
 
 void launch_correct(cudaStream_t s, int nx, int ny, int nz, const double* rho, const double* p,
                     double dx, double dy, double dz, double dt, double* u, int64_t usy,
                     int64_t usz, double* v, int64_t vsy, int64_t vsz, double* w, int64_t wsy,
                     int64_t wsz) {
-  const int pow2 = (is_pow2(dx) ? 1 : 0) | (is_pow2(dy) ? 2 : 0) | (is_pow2(dz) ? 4 : 0);
-  k_correct<<<grid3(nx, ny, nz), dim3(32, 8), 0, s>>>(
-      nx, ny, nz, rho, p, make_double3(dx, dy, dz), make_double3(1.0 / dx, 1.0 / dy, 1.0 / dz),
-      pow2, dt, u, usy, usz, v, vsy, vsz, w, wsy, wsz);
+  k_correct<<<grid3(nx, ny, nz), dim3(32, 8), 0, s>>>(nx, ny, nz, rho, p, spacing(dx, dy, dz), dt,
+                                                      u, usy, usz, v, vsy, vsz, w, wsy, wsz);
 }
 
 void launch_adjoint(cudaStream_t s, int nx, int ny, int nz, double dx2, double dy2, double dz2,
@@ -493,7 +484,7 @@ void launch_div_stats(cudaStream_t s, int nx, int ny, int nz, Strided u, Strided
                       double dx, double dy, double dz, const ReduceScratch& R) {
   cudaMemsetAsync(R.result + kSlotMax, 0, sizeof(double), s);
   const int blocks = std::min(reduce_blocks_for((size_t)ny * nz), R.max_blocks);
-  k_div_stats<<<blocks, kRedThreads, 0, s>>>(nx, ny, nz, u, v, w, dx, dy, dz, R);
+  k_div_stats<<<blocks, kRedThreads, 0, s>>>(nx, ny, nz, u, v, w, spacing(dx, dy, dz), R);
 }
 
 // *flag |= 1 when any x[q] is nonzero (-0 counts as zero): bit tests only,

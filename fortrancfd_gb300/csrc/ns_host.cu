@@ -107,11 +107,11 @@ int ns_prepare(gbmg_handle* h, const gbmg_ns_params* prm, const gbmg_ns_fields* 
   const double hs[3] = {g.dx, g.dy, g.dz};
   a.band = 1;
   for (int i = 0; i < 3; ++i) {
-    a.h[i] = const_div(hs[i]);
-    a.h2[i] = const_div(hs[i] * hs[i]);
+    a.h[i] = const_div_i(hs[i]);
+    a.h2[i] = const_div_i(hs[i] * hs[i]);
     if (!fdiv_divisor_ok(hs[i])) a.band = 0;
   }
-  a.rediv = const_div(prm->re);
+  a.rediv = const_div_i(prm->re);
   if (!fdiv_divisor_ok(prm->re) || !(std::fabs(prm->mu_12) < 0x1p60) ||
       !(std::fabs(prm->btn_sf) < 0x1p60) || (prm->btn_sf != 0 && !fdiv_divisor_ok(prm->we)))
     a.band = 0;

@@ -117,7 +117,7 @@ int main() {
     modes[c.mode]++;
     for (double a : edge) {
       same(div_const(c, a), a / h, a, h, "div_const edge");
-      same(div_const_i(c, a), a / h, a, h, "div_const_i edge");
+      same(div_const_i(const_div_i(h), a), a / h, a, h, "div_const_i edge");
     }
     for (int i = 0; i < 600; ++i) {
       double x = any(700, 1300);
