@@ -97,7 +97,10 @@ enum : int {
 };
 
 // ---- the bottom of the cycle in one block (subcycle.cu) ----------------------
-constexpr int kSubMaxCells = 4096;  // levels this small run inside one block
+// Levels this small run inside one block.  FP64 less: one SM takes 2 FP64 lanes
+// per clock, so a 4096-cell level costs the block 55 us of arithmetic per cycle
+// and ten separate launches about 30 (the whole 256^3 FP64 bottom 164 us before).
+constexpr int kSubMaxCells = 4096, kSubMaxCells64 = 1024;
 constexpr int kSubMaxLevels = 8;
 template <typename T>
 struct SubLevel {
@@ -106,6 +109,7 @@ struct SubLevel {
   const T* cx;
   const T* cy;
   const T* cz;
+  const T* id;  // 1/diagonal, or null (the update divides)
   int lx, ly;  // log2 of nx and ny when both are powers of two (index by shifts), else -1
 };
 template <typename T>
@@ -131,11 +135,13 @@ void launch_subcycle(cudaStream_t s, const SubCycle<T>& S);
 template <typename T>
 void launch_smooth(cudaStream_t s, const LevelView<T>& L, int color, bool zero_guess = false);
 // zero_sol: also set the coarse unknown to zero (not needed when its first
-// sweep starts from a zero guess)
+// sweep starts from a zero guess); half (FP64): the fine level's last colour
+// launch relaxed colour 1, whose residual is taken as zero
 template <typename T>
-void launch_restrict(cudaStream_t s, const LevelView<T>& F, const LevelView<T>& C, bool zero_sol);
-// live >= 0 (split finest level only): correct only the cells of colour live,
-// when the next sweep's first colour launch overwrites the other colour unread
+void launch_restrict(cudaStream_t s, const LevelView<T>& F, const LevelView<T>& C, bool zero_sol,
+                     bool half);
+// live >= 0: correct only the cells of colour live, when the next sweep's
+// first colour launch overwrites the other colour unread
 template <typename T>
 void launch_prolong(cudaStream_t s, const LevelView<T>& F, const LevelView<T>& C, int live = -1);
 // r = src - A sol on a level; writes r (type TO, may be null) and sum r^2 into slot.

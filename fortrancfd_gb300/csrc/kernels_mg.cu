@@ -26,12 +26,20 @@ inline unsigned cdiv(size_t a, unsigned b) { return (unsigned)((a + b - 1) / b);
 
 using namespace cells;
 
+// The block's z plane: FP64 levels alternate the direction launch by launch
+// (LevelView::zrev); the FP32 levels of this layout fit in L2.
+template <typename T>
+__device__ __forceinline__ int plane_of(const LevelView<T>& L, int nz) {
+  if constexpr (sizeof(T) == 8) return L.zrev ? nz - 1 - (int)blockIdx.z : (int)blockIdx.z;
+  else return (int)blockIdx.z;
+}
+
 // One colour of a red-black sweep, one thread per cell of the colour.
 template <typename T, bool kIdiag, bool kZero, bool kRho>
 __global__ void __launch_bounds__(256) k_smooth(LevelView<T> L, int color) {
   pdl_enter();
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z;
+  const int k = plane_of(L, L.nz);
   if (j >= L.ny) return;
   const int i = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + ((j + k + color) & 1);
   if (i >= L.nx) return;
@@ -39,25 +47,25 @@ __global__ void __launch_bounds__(256) k_smooth(LevelView<T> L, int color) {
 }
 
 // Fused residual + restriction, one thread per coarse cell.
-template <typename T, bool kRho>
+template <typename T, bool kRho, bool kHalf>
 __global__ void __launch_bounds__(256) k_restrict(LevelView<T> F, LevelView<T> C, int zero_sol) {
   pdl_enter();
   const int I = blockIdx.x * blockDim.x + threadIdx.x;
   const int J = blockIdx.y * blockDim.y + threadIdx.y;
-  const int K = blockIdx.z;
+  const int K = plane_of(F, C.nz);
   if (I >= C.nx || J >= C.ny) return;
-  restrict_cell<T, kRho>(F, C, I, J, K, zero_sol);
+  restrict_cell<T, kRho, kHalf>(F, C, I, J, K, zero_sol);
 }
 
 // Prolongation + correction, one thread per coarse cell.
 template <typename T>
-__global__ void __launch_bounds__(256) k_prolong(LevelView<T> F, LevelView<T> C) {
+__global__ void __launch_bounds__(256) k_prolong(LevelView<T> F, LevelView<T> C, int live) {
   pdl_enter();
   const int I = blockIdx.x * blockDim.x + threadIdx.x;
   const int J = blockIdx.y * blockDim.y + threadIdx.y;
-  const int K = blockIdx.z;
+  const int K = plane_of(F, C.nz);
   if (I >= C.nx || J >= C.ny) return;
-  prolong_cell<T>(F, C, I, J, K);
+  prolong_cell<T>(F, C, I, J, K, sizeof(T) == 8 ? live : -1);
 }
 
 // FP64 residual r = src - A sol (flux form) with sum r^2.  Blocks stride over (y, z) rows,
@@ -417,7 +425,8 @@ void launch_smooth(cudaStream_t s, const LevelView<T>& L, int color, bool zero_g
 }
 
 template <typename T>
-void launch_restrict(cudaStream_t s, const LevelView<T>& F, const LevelView<T>& C, bool zero_sol) {
+void launch_restrict(cudaStream_t s, const LevelView<T>& F, const LevelView<T>& C, bool zero_sol,
+                     bool half) {
   const dim3 blk(32, 8, 1);
   const dim3 grd(cdiv((size_t)C.nx, 32), cdiv((size_t)C.ny, 8), (unsigned)C.nz);
   if constexpr (std::is_same<T, float>::value) {
@@ -426,11 +435,14 @@ void launch_restrict(cudaStream_t s, const LevelView<T>& F, const LevelView<T>& 
       return;
     }
     if (F.rho) {
-      launch_pdl(k_restrict<T, true>, grd, blk, 0, s, F, C, zero_sol ? 1 : 0);
+      launch_pdl(k_restrict<T, true, false>, grd, blk, 0, s, F, C, zero_sol ? 1 : 0);
       return;
     }
+    launch_pdl(k_restrict<T, false, false>, grd, blk, 0, s, F, C, zero_sol ? 1 : 0);
+  } else {
+    launch_pdl(half ? k_restrict<T, false, true> : k_restrict<T, false, false>, grd, blk, 0, s, F,
+               C, zero_sol ? 1 : 0);
   }
-  launch_pdl(k_restrict<T, false>, grd, blk, 0, s, F, C, zero_sol ? 1 : 0);
 }
 
 template <typename T>
@@ -443,7 +455,7 @@ void launch_prolong(cudaStream_t s, const LevelView<T>& F, const LevelView<T>& C
       return;
     }
   }
-  launch_pdl(k_prolong<T>, grd, blk, 0, s, F, C);
+  launch_pdl(k_prolong<T>, grd, blk, 0, s, F, C, live);
 }
 
 // Blocks for a grid-stride reduction: 8 per SM, at most one per row.  The SM
@@ -516,9 +528,9 @@ void launch_to_float(cudaStream_t s, const double* a, float* b, size_t n) {
 template void launch_smooth<double>(cudaStream_t, const LevelView<double>&, int, bool);
 template void launch_smooth<float>(cudaStream_t, const LevelView<float>&, int, bool);
 template void launch_restrict<double>(cudaStream_t, const LevelView<double>&,
-                                      const LevelView<double>&, bool);
+                                      const LevelView<double>&, bool, bool);
 template void launch_restrict<float>(cudaStream_t, const LevelView<float>&,
-                                     const LevelView<float>&, bool);
+                                     const LevelView<float>&, bool, bool);
 template void launch_prolong<double>(cudaStream_t, const LevelView<double>&,
                                      const LevelView<double>&, int);
 template void launch_prolong<float>(cudaStream_t, const LevelView<float>&,

@@ -171,11 +171,28 @@ __device__ __forceinline__ void smooth_cell(const LevelView<T>& L, int i, int j,
 // Fused residual + restriction: coarse src = mean over the children of
 // (src - A sol) on the fine level; coarse sol = 0.  One thread per coarse
 // cell; the children are summed in the order z, y, x (the oracle's).
-template <typename T, bool kRho, bool kCg = false>
+// kHalf: the level's last colour launch relaxed the cells of colour 1, whose
+// residual is therefore zero up to the rounding of the update: only the
+// children of colour 0 are visited (half the arithmetic; 256^3 FP64, bound by
+// the FP64 pipe, 484 -> 261 us).  FP64 only: in FP32 that rounding reaches 1e-4
+// of the residual within a correction's four cycles, enough to move the mixed
+// loop's schedule and with it the error left at the tolerance.
+template <typename T, bool kRho, bool kHalf, bool kCg = false>
 __device__ __forceinline__ void restrict_cell(const LevelView<T>& F, const LevelView<T>& C, int I,
                                               int J, int K, int zero_sol) {
   T acc = T(0);
-  if (F.fx == 2) {
+  if constexpr (kHalf) {
+    for (int dz = 0; dz < F.fz; ++dz)
+      for (int dy = 0; dy < F.fy; ++dy) {
+        const int j = F.fy * J + dy, k = F.fz * K + dz;
+        const int i = F.fx * I + (F.fx == 2 ? (j + k) & 1 : 0);
+        if (F.fx == 1 && ((i + j + k) & 1)) continue;
+        const size_t q = ((size_t)k * F.ny + j) * F.nx + i;
+        T s, d;
+        stencil<T, kCg>(F, F.sol, i, j, k, q, s, d);
+        acc += ldc<kCg>(F.src + q) - (s - d * ldc<kCg>(F.sol + q));
+      }
+  } else if (F.fx == 2) {
     // the two x-children of each child row as vector loads
     using V2 = typename Vec2<T>::type;
     const size_t sy = (size_t)F.nx, sz = (size_t)F.nx * F.ny;
@@ -263,9 +280,11 @@ __device__ __forceinline__ void restrict_cell(const LevelView<T>& F, const Level
 // One thread per coarse cell updates its children; with fx = 2 the two
 // x-children are one vector load and store.  Per child the terms are added in
 // the order x, y, z, as the oracle does.
+// live >= 0: only the children of that colour (the other colour is overwritten,
+// unread, by the next sweep's first colour launch).
 template <typename T, bool kCg = false>
 __device__ __forceinline__ void prolong_cell(const LevelView<T>& F, const LevelView<T>& C, int I,
-                                             int J, int K) {
+                                             int J, int K, int live) {
   using V2 = typename Vec2<T>::type;
   const size_t csy = (size_t)C.nx, csz = (size_t)C.nx * C.ny;
   const size_t cq = (size_t)K * csz + (size_t)J * csy + I;
@@ -286,7 +305,14 @@ __device__ __forceinline__ void prolong_cell(const LevelView<T>& F, const LevelV
       T* row = F.sol + ((size_t)k * F.ny + j) * F.nx;
       const T ty = dy ? T(0.25) * my : -(T(0.25) * my);
       const T tz = dz ? T(0.25) * mz : -(T(0.25) * mz);
-      if (F.fx == 2) {
+      if (F.fx == 2 && live >= 0) {
+        const int o = (j + k + live) & 1;  // the live child: x = 2I + o
+        T v = ec + (o ? T(0.25) * mx : -(T(0.25) * mx));
+        if (F.fy == 2) v += ty;
+        if (F.fz == 2) v += tz;
+        T* pr = row + 2 * I + o;
+        *pr = ldc<kCg>(pr) + v;
+      } else if (F.fx == 2) {
         T v0 = ec + -(T(0.25) * mx), v1 = ec + T(0.25) * mx;
         if (F.fy == 2) { v0 += ty; v1 += ty; }
         if (F.fz == 2) { v0 += tz; v1 += tz; }
@@ -295,7 +321,7 @@ __device__ __forceinline__ void prolong_cell(const LevelView<T>& F, const LevelV
         cur.x += v0;
         cur.y += v1;
         *pr = cur;
-      } else {
+      } else if (live < 0 || ((I + j + k) & 1) == live) {
         T v = ec;
         if (F.fy == 2) v += ty;
         if (F.fz == 2) v += tz;

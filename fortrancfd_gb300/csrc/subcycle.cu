@@ -18,6 +18,9 @@ namespace gbmg {
 namespace {
 
 constexpr int kSubThreads = 1024;
+// the FP64 levels carry 1/diagonal, the FP32 levels divide
+template <typename T>
+constexpr bool kSubIdiag = sizeof(T) == 8;
 
 template <typename T>
 __device__ __forceinline__ void sub_stencil(const SubLevel<T>& L, const T* __restrict__ p, int i,
@@ -71,16 +74,21 @@ __device__ void sub_colour(const SubLevel<T>& L, T* sol, const T* src, int color
     const int i = 2 * m + ((j + k + color) & 1);
     if (i >= L.nx) continue;
     const int q = (k * L.ny + j) * L.nx + i;
-    T s, d;
-    if (zero) {
-      T dd;
-      sub_stencil(L, sol, i, j, k, q, s, dd);  // for d only; p is ignored
-      s = T(0);
-      d = dd;
+    T s = T(0), d;
+    if constexpr (kSubIdiag<T>) {
+      if (!zero) sub_stencil(L, sol, i, j, k, q, s, d);
+      sol[q] = (s - src[q]) * L.id[q];
     } else {
-      sub_stencil(L, sol, i, j, k, q, s, d);
+      if (zero) {
+        T dd;
+        sub_stencil(L, sol, i, j, k, q, s, dd);  // for d only; p is ignored
+        s = T(0);
+        d = dd;
+      } else {
+        sub_stencil(L, sol, i, j, k, q, s, d);
+      }
+      sol[q] = (s - src[q]) / d;
     }
-    sol[q] = (s - src[q]) / d;
   }
   __syncthreads();
 }
@@ -91,10 +99,12 @@ __device__ void sub_sweep(const SubLevel<T>& L, T* sol, const T* src, int first,
   sub_colour(L, sol, src, 1 - first, false);
 }
 
-// coarse src = mean of the children's residuals (fine -> coarse, shared memory)
+// coarse src = mean of the children's residuals (fine -> coarse, shared
+// memory); half (FP64, as restrict_cell): the children of colour 1, relaxed
+// last, have none
 template <typename T>
 __device__ void sub_restrict(const SubLevel<T>& F, const T* fsol, const T* fsrc,
-                             const SubLevel<T>& C, T* csrc) {
+                             const SubLevel<T>& C, T* csrc, bool half) {
   const int n = C.nx * C.ny * C.nz;
   for (int cq = threadIdx.x; cq < n; cq += blockDim.x) {
     int I, J, K;
@@ -104,6 +114,7 @@ __device__ void sub_restrict(const SubLevel<T>& F, const T* fsol, const T* fsrc,
       for (int dy = 0; dy < F.fy; ++dy)
         for (int dx = 0; dx < F.fx; ++dx) {
           const int i = F.fx * I + dx, j = F.fy * J + dy, k = F.fz * K + dz;
+          if (sizeof(T) == 8 && half && ((i + j + k) & 1)) continue;
           const int q = (k * F.ny + j) * F.nx + i;
           T s, d;
           sub_stencil(F, fsol, i, j, k, q, s, d);
@@ -115,13 +126,16 @@ __device__ void sub_restrict(const SubLevel<T>& F, const T* fsol, const T* fsrc,
 }
 
 // fine sol += central-slope interpolation of the coarse sol
+// (FP64: live >= 0, the cells of that colour only)
 template <typename T>
-__device__ void sub_prolong(const SubLevel<T>& F, T* fsol, const SubLevel<T>& C, const T* e) {
+__device__ void sub_prolong(const SubLevel<T>& F, T* fsol, const SubLevel<T>& C, const T* e,
+                            int live) {
   const int n = F.nx * F.ny * F.nz;
   const int csy = C.nx, csz = C.nx * C.ny;
   for (int q = threadIdx.x; q < n; q += blockDim.x) {
     int i, j, k;
     sub_ijk(F, q, i, j, k);
+    if (sizeof(T) == 8 && live >= 0 && ((i + j + k) & 1) != live) continue;
     const int I = i >> (F.fx - 1), J = j >> (F.fy - 1), K = k >> (F.fz - 1);
     const int cq = K * csz + J * csy + I;
     const T ec = e[cq];
@@ -182,8 +196,9 @@ __device__ void sub_coarse(int n, const T* __restrict__ minv, const T* __restric
   __syncthreads();
 }
 
-// Shared memory per level: sol, src, then the three face-coefficient arrays
-// (staged once at the start, so no phase waits on L2), n cells each.
+// Shared memory per level: sol, src, then the three face-coefficient arrays and
+// 1/diagonal where there is one (staged once at the start, so no phase waits on
+// L2), n cells each.
 template <typename T>
 __device__ void subcycle_body(const SubCycle<T>& S, T* base) {
   const int nl = S.nlev;
@@ -197,6 +212,7 @@ __device__ void subcycle_body(const SubCycle<T>& S, T* base) {
       c[q] = S.lv[l].cx[q];
       c[n + q] = S.lv[l].cy[q];
       c[2 * n + q] = S.lv[l].cz[q];
+      if (kSubIdiag<T>) c[3 * n + q] = S.lv[l].id[q];
     }
   }
   // level l with its coefficients in shared memory
@@ -207,6 +223,7 @@ __device__ void subcycle_body(const SubCycle<T>& S, T* base) {
     L.cx = c;
     L.cy = c + n;
     L.cz = c + 2 * n;
+    if (kSubIdiag<T>) L.id = c + 3 * n;
     return L;
   };
   T* scratch = base + S.off[nl];
@@ -222,11 +239,11 @@ __device__ void subcycle_body(const SubCycle<T>& S, T* base) {
       for (int q = threadIdx.x; q < n; q += blockDim.x) sol(l)[q] = T(0);
       __syncthreads();
     }
-    sub_restrict(lv(l), sol(l), src(l), lv(l + 1), src(l + 1));
+    sub_restrict(lv(l), sol(l), src(l), lv(l + 1), src(l + 1), S.nu1 > 0);
   }
   sub_coarse(S.n_coarse, S.minv, S.adense, src(nl - 1), sol(nl - 1), scratch);
   for (int l = nl - 2; l >= 0; --l) {
-    sub_prolong(lv(l), sol(l), lv(l + 1), sol(l + 1));
+    sub_prolong(lv(l), sol(l), lv(l + 1), sol(l + 1), S.nu2 > 0 ? (S.reverse ? 0 : 1) : -1);
     for (int it = 0; it < S.nu2; ++it) sub_sweep(lv(l), sol(l), src(l), S.reverse ? 1 : 0, false);
   }
   const int n0 = S.lv[0].nx * S.lv[0].ny * S.lv[0].nz;
