@@ -141,17 +141,15 @@ SubCycle<T> make_subcycle(gbmg_handle* h, bool reverse) {
   int off = 0;
   for (int i = 0; i < S.nlev; ++i) {
     const LevelView<T> V = view<T>(h->lv[lc + i]);
-    const auto log2_of = [](int v) {
-      int l = 0;
-      while ((1 << l) < v) ++l;
-      return (1 << l) == v ? l : -1;
+    const auto rcp = [](int d) {
+      return d == 1 ? 0u : (unsigned)(((1ull << 32) + (unsigned)d - 1) / (unsigned)d);
     };
-    const int lx = log2_of(V.nx), ly = log2_of(V.ny);
     S.lv[i] = SubLevel<T>{V.nx, V.ny, V.nz, V.fx, V.fy, V.fz, V.cx, V.cy, V.cz, V.idiag,
-                          (lx >= 0 && ly >= 0) ? lx : -1, (lx >= 0 && ly >= 0) ? ly : -1};
+                          rcp(V.nx), rcp(V.ny), rcp((V.nx + 1) / 2),
+                          V.nz > 1 ? V.nx * V.ny : V.nx, T(1) / T(V.fx * V.fy * V.fz)};
     S.off[i] = off;
-    // sol, src, the three coefficient arrays and 1/diagonal
-    off += (V.idiag ? 6 : 5) * V.nx * V.ny * V.nz;
+    // sol, src, the three coefficient arrays and 1/diagonal, with their padding
+    off += (V.idiag ? 6 : 5) * V.nx * V.ny * V.nz + 5 * S.lv[i].pad;
   }
   S.off[S.nlev] = off;
   const LevelView<T> V0 = view<T>(h->lv[lc]);

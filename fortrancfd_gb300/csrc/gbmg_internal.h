@@ -110,13 +110,16 @@ struct SubLevel {
   const T* cy;
   const T* cz;
   const T* id;  // 1/diagonal, or null (the update divides)
-  int lx, ly;  // log2 of nx and ny when both are powers of two (index by shifts), else -1
+  // ceil(2^32 / d) for d = nx, ny and the x pairs (nx + 1)/2 (0 for d = 1)
+  unsigned rx, ry, rh;
+  int pad;  // zeros around an array in shared memory: a plane (2D: a row)
+  T mean;   // 1/(fx fy fz)
 };
 template <typename T>
 struct SubCycle {
   int nlev, nu1, nu2, reverse, n_coarse;
   SubLevel<T> lv[kSubMaxLevels];   // the levels from the first small one down
-  int off[kSubMaxLevels + 1];      // shared-memory offsets (elements): sol, src per level
+  int off[kSubMaxLevels + 1];      // shared-memory offsets of the levels (elements)
   const T* src_in;                 // right-hand side of the first small level (global)
   T* sol_out;                      // its result (global)
   const T* minv;

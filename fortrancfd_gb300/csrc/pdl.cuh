@@ -15,9 +15,13 @@
 
 namespace gbmg {
 
-__device__ __forceinline__ void pdl_enter() {
+__device__ __forceinline__ void pdl_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_enter() {
+  pdl_launch();
+  pdl_wait();
 }
 
 // kernel<<<g, b, smem, s>>>(args...) with programmatic stream serialization
