@@ -274,6 +274,7 @@ int free_all(gbmg_handle* h) {
   dfree(h->kdiag); dfree(h->kr); dfree(h->kz); dfree(h->kzold); dfree(h->kd); dfree(h->kq);
   dfree(h->gmV); dfree(h->gmZ); dfree(h->gmPart); dfree(h->gmDev);
   if (h->gmHost) cudaFreeHost(h->gmHost);
+  if (h->gmEv) cudaEventDestroy(h->gmEv);
   dfree(h->minv); dfree(h->adense); dfree(h->cwork); dfree(h->minv32); dfree(h->adense32); dfree(h->derr);
   for (int i = 0; i < 48; ++i) dfree(h->ns_buf[i]);
   delete[] h->dmaps;
@@ -400,16 +401,18 @@ int allocate(gbmg_handle* h) {
   if (h->prm.krylov) {
     GB_TRY(dmalloc(h, &h->kdiag, h->n0));
     GB_TRY(dmalloc(h, &h->kr, h->n0));
-    if (!h->mixed || h->prm.krylov == 2) GB_TRY(dmalloc(h, &h->kz, h->n0));
+    if (!h->mixed) GB_TRY(dmalloc(h, &h->kz, h->n0));
     GB_TRY(dmalloc(h, &h->kzold, h->n0));
     GB_TRY(dmalloc(h, &h->kd, h->n0));
     GB_TRY(dmalloc(h, &h->kq, h->n0));
     if (h->prm.krylov == 2) {
-      GB_TRY(dmalloc(h, &h->gmV, (size_t)(kGmresRestart + 1) * h->n0));
-      GB_TRY(dmalloc(h, &h->gmZ, (size_t)kGmresRestart * h->n0));
+      h->gmLd = h->n0 + (h->n0 & 1);
+      GB_TRY(dmalloc(h, &h->gmV, (size_t)(kGmresRestart + 1) * h->gmLd));
+      GB_TRY(dmalloc(h, &h->gmZ, (size_t)kGmresRestart * h->gmLd));
       GB_TRY(dmalloc(h, &h->gmPart, (size_t)(kGmresRestart + 1) * kGmresBlocks));
-      GB_TRY(dmalloc(h, &h->gmDev, (size_t)3 * (kGmresRestart + 1)));
-      GB_CUDA(h, cudaMallocHost((void**)&h->gmHost, 3 * (kGmresRestart + 1) * sizeof(double)));
+      GB_TRY(dmalloc(h, &h->gmDev, (size_t)3 * (kGmresRestart + 2)));
+      GB_CUDA(h, cudaMallocHost((void**)&h->gmHost, 3 * (kGmresRestart + 2) * sizeof(double)));
+      GB_CUDA(h, cudaEventCreateWithFlags(&h->gmEv, cudaEventDisableTiming));
     }
   }
   GB_TRY(dmalloc(h, &h->minv, (size_t)nc * nc));
@@ -828,42 +831,34 @@ int run_loop(gbmg_handle* h, int kind, CycleCtl* c, bool* used) {
   return GBMG_OK;
 }
 
-// The solve loop on the internal (b, p).  Leaves p mean-free.
-// z = M v: one V-cycle from zero on v (the flexible-CG preconditioner),
-// mean-free.  Leaves the finest level's sol/src pointing at p and b.
-int precondition(gbmg_handle* h, const double* v, double* z) {
-  const cudaStream_t s = h->stream;
-  Level& f = h->lv[0];
-  const size_t n = h->n0;
-  const int V = GBMG_PROF_VECTOR;
-  const bool zg = h->prm.nu1 > 0;
-  if (!h->mixed) {
-    if (!zg) GB_CUDA(h, cudaMemsetAsync(z, 0, n * sizeof(double), s));
-    f.sol = z; f.src = const_cast<double*>(v);
-    GB_TRY(enqueue_vcycle<double>(h, true, zg));
-  } else {
-    if (f.split) LAUNCH(h, V, launch_to_split(s, v, f.src32, f.nx, f.ny, f.nz, f.hstride));
-    else LAUNCH(h, V, launch_double_to_float(s, v, f.src32, n));
-    if (!zg) GB_CUDA(h, cudaMemsetAsync(f.sol32, 0, n * sizeof(float), s));
-    GB_TRY(enqueue_vcycle<float>(h, true, zg));
-    if (f.split) LAUNCH(h, V, launch_from_split(s, f.sol32, z, f.nx, f.ny, f.nz, f.hstride));
-    else LAUNCH(h, V, launch_float_to_double(s, f.sol32, z, n));
-  }
-  LAUNCH(h, V, launch_sum(s, z, n, h->red, kSlotSum));
-  LAUNCH(h, V, launch_shift_by_mean(s, z, z, n, h->red, kSlotSum, -1));
-  f.sol = h->p; f.src = h->b;
-  return check_launch(h, "preconditioner");
+// The finest level's right-hand side and unknown as flexible GMRES uses them:
+// FP64 kr and kz, or the FP32 level's own
+PcgVec gm_vec(gbmg_handle* h) {
+  const Level& f = h->lv[0];
+  return PcgVec{h->mixed ? nullptr : h->kz, h->mixed ? f.sol32 : nullptr, h->n0,
+                f.split ? f.hstride : 0, f.nx, f.ny};
 }
 
-// kz = M kr, kq = A kz: enqueued, or replayed from a graph captured on first use
-int gm_apply(gbmg_handle* h) {
+// One V-cycle from zero on that right-hand side and the sum of its result, enqueued, or
+// replayed from a graph captured on first use
+int gm_vcycle(gbmg_handle* h) {
   const cudaStream_t s = h->stream;
   Level& f = h->lv[0];
   const auto enqueue = [&]() -> int {
-    GB_TRY(precondition(h, h->kr, h->kz));
-    LAUNCH(h, GBMG_PROF_RESIDUAL,
-           launch_apply_diag(s, v64(f), h->kdiag, h->kz, h->kq, h->red, kSlotDot2, false));
-    return check_launch(h, "preconditioned product");
+    const bool zg = h->prm.nu1 > 0;
+    if (!h->mixed) {
+      if (!zg) GB_CUDA(h, cudaMemsetAsync(h->kz, 0, h->n0 * sizeof(double), s));
+      f.sol = h->kz; f.src = h->kr;
+      const int rc = enqueue_vcycle<double>(h, true, zg);
+      f.sol = h->p; f.src = h->b;
+      GB_TRY(rc);
+    } else {
+      if (!zg)
+        GB_CUDA(h, cudaMemsetAsync(f.sol32, 0, (f.split ? h->n0 / 2 + f.hstride : h->n0) * sizeof(float), s));
+      GB_TRY(enqueue_vcycle<float>(h, true, zg));
+    }
+    LAUNCH(h, GBMG_PROF_VECTOR, launch_gm_sum(s, gm_vec(h), h->red, kSlotSum));
+    return check_launch(h, "preconditioner");
   };
   if (!h->prm.use_graph || h->prof) return enqueue();
   if (!h->gm_graph) {
@@ -896,11 +891,11 @@ int gm_apply(gbmg_handle* h) {
 // Flexible GMRES(kGmresRestart) around the V-cycle (right preconditioning,
 // Saad's FGMRES): the residual norm falls monotonically, where conjugate
 // gradients can first raise it many-fold on a smooth right-hand side (the
-// adjoint of a smooth objective).  Per Arnoldi step: z_j = M v_j and
-// w = A z_j (one captured graph on fixed buffers: v_j is copied in, z_j out),
-// classical Gram-Schmidt on the device with a second pass only when the
+// adjoint of a smooth objective).  Per Arnoldi step: z_j = M v_j (the V-cycle one captured
+// graph) and w = A z_j, classical Gram-Schmidt on the device with a second pass only when the
 // first removed most of w, one copy of the coefficients to the host for the
-// Givens rotations, and w scaled into v_{j+1}.  At each restart and at the end the true FP64 residual b - A p
+// Givens rotations, and w scaled into v_{j+1} while the host does these.  At each restart and at
+// the end the true FP64 residual b - A p
 // is recomputed.  On entry kr holds r0 = b - A p and host_res[kSlotNorm] its
 // squared norm.
 int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles, int* status) {
@@ -909,10 +904,23 @@ int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles
   const size_t n = h->n0;
   const int m = kGmresRestart;
   const int VC = GBMG_PROF_VECTOR;
-  const size_t bytes = n * sizeof(double);
-  double* h1 = h->gmDev;               // first Gram-Schmidt pass
-  double* h2 = h->gmDev + (m + 1);     // second pass
-  double* nrm = h->gmDev + 2 * (m + 1);  // |w|^2 after, then before, the first pass
+  const size_t ld = h->gmLd;
+  const PcgVec z = gm_vec(h);
+  double* h1 = h->gmDev;               // first Gram-Schmidt pass, then |w|^2 before it
+  double* h2 = h->gmDev + (m + 2);     // second pass
+  double* nrm = h->gmDev + 2 * (m + 2);  // |w|^2 after, 1/|w|
+  double* src64 = h->mixed ? nullptr : h->kr;
+  float* src32 = h->mixed ? f.src32 : nullptr;
+  // coefficients to the host, v_{j+1} written meanwhile
+  const auto fetch = [&](int j) -> int {
+    GB_CUDA(h, cudaMemcpyAsync(h->gmHost, h->gmDev, 3 * (m + 2) * sizeof(double),
+                               cudaMemcpyDeviceToHost, s));
+    GB_CUDA(h, cudaEventRecord(h->gmEv, s));
+    LAUNCH(h, VC, launch_gm_next(s, h->gmV + (size_t)(j + 1) * ld, h->kq, nrm + 1, 0.0, src64,
+                                 src32, z));
+    GB_CUDA(h, cudaEventSynchronize(h->gmEv));
+    return check_launch(h, "arnoldi");
+  };
   std::vector<double> H((size_t)(m + 1) * m, 0.0), cs(m), sn(m), g(m + 1), y(m), col(m + 1);
   double r2 = h->host_res[kSlotNorm];
   double rel = *rel_io;
@@ -921,45 +929,36 @@ int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles
   while (total < h->prm.max_cycles) {
     const double beta = std::sqrt(r2);
     if (!(beta > 0.0)) { *status = GBMG_OK; break; }
-    LAUNCH(h, VC, launch_scale_copy(s, h->gmV, h->kr, 1.0 / beta, n));
+    LAUNCH(h, VC, launch_gm_next(s, h->gmV, h->kr, nullptr, 1.0 / beta, src64, src32, z));
     std::fill(g.begin(), g.end(), 0.0);
     g[0] = beta;
     int j = 0;
     for (; j < m && total < h->prm.max_cycles;) {
-      double* vj = h->gmV + (size_t)j * n;
       double* w = h->kq;  // A z_j, orthogonalised in place, then scaled into V_{j+1}
-      GB_CUDA(h, cudaMemcpyAsync(h->kr, vj, bytes, cudaMemcpyDeviceToDevice, s));
-      GB_TRY(gm_apply(h));
-      GB_CUDA(h, cudaMemcpyAsync(h->gmZ + (size_t)j * n, h->kz, bytes, cudaMemcpyDeviceToDevice, s));
+      double* zj = h->gmZ + (size_t)j * ld;
+      GB_TRY(gm_vcycle(h));
+      LAUNCH(h, VC, launch_gm_z(s, z, zj, h->red.result + kSlotSum));
+      LAUNCH(h, GBMG_PROF_RESIDUAL, launch_apply_diag(s, v64(f), h->kdiag, zj, w, h->red, -1, false));
       // classical Gram-Schmidt; a second pass only when the first removed most
       // of w (|w| fell below 0.7 of its length: "twice is enough")
-      LAUNCH(h, VC, launch_mdot(s, w, n, 1, w, n, h->gmPart, kGmresBlocks, nrm + 1));
-      LAUNCH(h, VC, launch_mdot(s, h->gmV, n, j + 1, w, n, h->gmPart, kGmresBlocks, h1));
-      LAUNCH(h, VC, launch_maxpy(s, w, h->gmV, n, h1, j + 1, -1.0, n));
-      LAUNCH(h, VC, launch_mdot(s, w, n, 1, w, n, h->gmPart, kGmresBlocks, nrm));
-      h->launches += 3;  // the finishing kernels of the dot launches
-      GB_CUDA(h, cudaMemcpyAsync(h->gmHost, h->gmDev, 3 * (m + 1) * sizeof(double),
-                                 cudaMemcpyDeviceToHost, s));
-      GB_CUDA(h, cudaStreamSynchronize(s));
-      GB_TRY(check_launch(h, "arnoldi"));
+      LAUNCH(h, VC, launch_gm_dots(s, h->gmV, ld, j + 1, w, n, h->gmPart, h1));
+      LAUNCH(h, VC, launch_gm_update(s, w, h->gmV, ld, h1, j + 1, -1.0, n, h->gmPart,
+                                     h->red.counter, nrm));
+      ++h->launches;  // the products' finishing kernel
+      GB_TRY(fetch(j));
       for (int i = 0; i <= j; ++i) col[i] = h->gmHost[i];
-      double hn = std::sqrt(h->gmHost[2 * (m + 1)]);
-      const double before = std::sqrt(h->gmHost[2 * (m + 1) + 1]);
+      double hn = std::sqrt(h->gmHost[2 * (m + 2)]);
+      const double before = std::sqrt(h->gmHost[j + 1]);
       if (hn < 0.7 * before) {
-        LAUNCH(h, VC, launch_mdot(s, h->gmV, n, j + 1, w, n, h->gmPart, kGmresBlocks, h2));
-        LAUNCH(h, VC, launch_maxpy(s, w, h->gmV, n, h2, j + 1, -1.0, n));
-        LAUNCH(h, VC, launch_mdot(s, w, n, 1, w, n, h->gmPart, kGmresBlocks, nrm));
-        h->launches += 2;
-        GB_CUDA(h, cudaMemcpyAsync(h->gmHost, h->gmDev, 3 * (m + 1) * sizeof(double),
-                                   cudaMemcpyDeviceToHost, s));
-        GB_CUDA(h, cudaStreamSynchronize(s));
-        GB_TRY(check_launch(h, "arnoldi"));
-        for (int i = 0; i <= j; ++i) col[i] += h->gmHost[(m + 1) + i];
-        hn = std::sqrt(h->gmHost[2 * (m + 1)]);
+        LAUNCH(h, VC, launch_gm_dots(s, h->gmV, ld, j + 1, w, n, h->gmPart, h2));
+        LAUNCH(h, VC, launch_gm_update(s, w, h->gmV, ld, h2, j + 1, -1.0, n, h->gmPart,
+                                       h->red.counter, nrm));
+        ++h->launches;
+        GB_TRY(fetch(j));
+        for (int i = 0; i <= j; ++i) col[i] += h->gmHost[(m + 2) + i];
+        hn = std::sqrt(h->gmHost[2 * (m + 2)]);
       }
       col[j + 1] = hn;
-      LAUNCH(h, VC, launch_scale_copy(s, h->gmV + (size_t)(j + 1) * n, w, hn > 0.0 ? 1.0 / hn : 0.0,
-                                      n));
       for (int i = 0; i < j; ++i) {
         const double t = cs[i] * col[i] + sn[i] * col[i + 1];
         col[i + 1] = -sn[i] * col[i] + cs[i] * col[i + 1];
@@ -986,7 +985,7 @@ int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles
     }
     std::copy(y.begin(), y.begin() + j, h->gmHost);
     GB_CUDA(h, cudaMemcpyAsync(h->gmDev, h->gmHost, j * sizeof(double), cudaMemcpyHostToDevice, s));
-    LAUNCH(h, VC, launch_maxpy(s, h->p, h->gmZ, n, h->gmDev, j, 1.0, n));
+    LAUNCH(h, VC, launch_gm_update(s, h->p, h->gmZ, ld, h->gmDev, j, 1.0, n, nullptr, nullptr, nullptr));
     f.sol = h->p; f.src = h->b;
     LAUNCH(h, GBMG_PROF_RESIDUAL,
            launch_residual_norm<double>(s, v64(f), h->kr, h->red, kSlotNorm));

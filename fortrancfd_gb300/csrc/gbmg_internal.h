@@ -230,8 +230,6 @@ void launch_prolong_split(cudaStream_t s, const LevelView<float>& F, const Level
                           int live);
 void launch_to_split(cudaStream_t s, const double* a, float* out, int nx, int ny, int nz,
                      size_t hstride);
-void launch_from_split(cudaStream_t s, const float* a, double* out, int nx, int ny, int nz,
-                       size_t hstride);
 // elements reserved past n in each split FP32 finest-level array for the pad
 constexpr size_t kSplitPadMax = 65536;
 
@@ -273,6 +271,7 @@ void launch_zero_wall_faces(cudaStream_t s, int nx, int ny, int nz, double* u, i
                             int64_t wsy, int64_t wsz);
 // slot <- sum x
 void launch_sum(cudaStream_t s, const double* x, size_t n, const ReduceScratch& R, int slot);
+int sum_blocks(size_t n, const ReduceScratch& R);  // its blocks
 // y = x - result[slot]/n ; result[slot2] <- sum y^2 (slot2 < 0: no norm)
 void launch_shift_by_mean(cudaStream_t s, const double* x, double* y, size_t n,
                           const ReduceScratch& R, int slot, int slot2);
@@ -299,20 +298,29 @@ void launch_pcg_x(cudaStream_t s, double* x, const double* d, size_t n,
 void launch_pcg_step(cudaStream_t s, double* x, const double* d, double* r, const double* q,
                      float* r32, const PcgVec& z, const ReduceScratch& R);
 // sum of the face coefficients of each cell, and q = A d with it, d.q into
-// slot; keep_rz: kSlotDot2+1 <- kSlotDot (kernels_mg.cu)
+// slot (none when slot < 0); keep_rz: kSlotDot2+1 <- kSlotDot (kernels_mg.cu)
 void launch_diag(cudaStream_t s, const LevelView<double>& L, double* diag);
 void launch_apply_diag(cudaStream_t s, const LevelView<double>& L, const double* diag,
                        const double* d, double* q, const ReduceScratch& R, int slot, bool keep_rz);
-void launch_float_to_double(cudaStream_t s, const float* a, double* b, size_t n);
-// flexible GMRES vector kernels (krylov.cu): out[i] = V_i . w for i < cnt
-// (basis V_i at V + i*ld; partials: cnt * max_blocks doubles), w += sign *
-// sum_i coef[i] V_i, out = alpha * in
-void launch_mdot(cudaStream_t s, const double* V, size_t ld, int cnt, const double* w, size_t n,
-                 double* partials, int max_blocks, double* out);
-void launch_maxpy(cudaStream_t s, double* w, const double* V, size_t ld, const double* coef,
-                  int cnt, double sign, size_t n);
-void launch_scale_copy(cudaStream_t s, double* out, const double* in, double alpha, size_t n);
-void launch_scale_rsqrt(cudaStream_t s, double* w, const double* nrm2, size_t n);  // w /= |w|
+// Flexible GMRES passes (krylov.cu), basis V_i at V + i*ld; partials:
+// kGmresBlocks doubles per sum; counter as ReduceScratch::counter.
+constexpr int kGmresRestart = 30;   // restart length
+constexpr int kGmresBlocks = 1024;  // blocks of the products and the update
+// the sum of z
+void launch_gm_sum(cudaStream_t s, const PcgVec& z, const ReduceScratch& R, int slot);
+// out[i] = V_i.w for i < cnt, out[cnt] = w.w
+void launch_gm_dots(cudaStream_t s, const double* V, size_t ld, int cnt, const double* w, size_t n,
+                    double* partials, double* out);
+// w += sign * sum_i coef[i] V_i; nrm (may be null): |w|^2, 1/|w|
+void launch_gm_update(cudaStream_t s, double* w, const double* V, size_t ld, const double* coef,
+                      int cnt, double sign, size_t n, double* partials, unsigned int* counter,
+                      double* nrm);
+// v = (*inv or scale) * w, and the same as the V-cycle's right-hand side: src64,
+// or src32 in z's layout
+void launch_gm_next(cudaStream_t s, double* v, const double* w, const double* inv, double scale,
+                    double* src64, float* src32, const PcgVec& z);
+// out = z - *sum / n
+void launch_gm_z(cudaStream_t s, const PcgVec& z, double* out, const double* sum);
 void launch_double_to_float(cudaStream_t s, const double* a, float* b, size_t n);
 
 int reduce_blocks_for(size_t n);

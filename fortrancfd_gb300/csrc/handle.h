@@ -32,8 +32,6 @@ struct Level {
 };
 
 enum GraphKind { kGraphNone = -1, kGraphFp64 = 0, kGraphMixed = 1, kGraphPcg64 = 2, kGraphPcgMixed = 3 };
-constexpr int kGmresRestart = 30;   // flexible GMRES restart length
-constexpr int kGmresBlocks = 1024;  // blocks of its dot-product kernel
 
 
 }  // namespace gbmg
@@ -65,6 +63,9 @@ struct gbmg_handle {
   double* kdiag = nullptr;  // sum of the finest level's face coefficients per cell
   // flexible GMRES (krylov = 2): basis V (restart + 1 vectors), preconditioned
   // vectors Z (restart), dot partials, device and pinned host coefficients
+  // gmLd: stride of V and Z (n0 rounded up to even); gmEv: the step's coefficients copied
+  size_t gmLd = 0;
+  cudaEvent_t gmEv = nullptr;
   double *gmV = nullptr, *gmZ = nullptr, *gmPart = nullptr, *gmDev = nullptr, *gmHost = nullptr;
   // coarsest level
   int nc = 0;
@@ -105,7 +106,8 @@ struct gbmg_handle {
   bool loop_off = false;          // the device loop could not be built: host loop
   gbmg::CycleCtl* ctl = nullptr;  // its state on the device, and a pinned mirror
   gbmg::CycleCtl* ctl_host = nullptr;
-  // flexible GMRES: kz = M kr and kq = A kz as one captured graph
+  // flexible GMRES: a V-cycle on the right-hand side in place and the sum of its
+  // result as one captured graph
   cudaGraphExec_t gm_graph = nullptr;
   int64_t gm_graph_kernels = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;

@@ -388,10 +388,6 @@ __global__ void k_add_float(double* p, const float* __restrict__ e, size_t n) {
           [&](size_t q, double2 v) { p[q] = v.x + v.y; });
 }
 
-__global__ void k_f2d(const float* __restrict__ a, double* b, size_t n) {
-  stride4(n, [&](size_t q) { return a[q]; }, [&](size_t q, float v) { b[q] = (double)v; });
-}
-
 __global__ void k_d2f(const double* __restrict__ a, float* b, size_t n) {
   stride4(n, [&](size_t q) { return a[q]; }, [&](size_t q, double v) { b[q] = (float)v; });
 }
@@ -578,8 +574,12 @@ void launch_nonzero(cudaStream_t s, const double* x, size_t n, double* flag) {
       x, n, reinterpret_cast<unsigned long long*>(flag));
 }
 
+int sum_blocks(size_t n, const ReduceScratch& R) {
+  return (int)std::min<unsigned>(stride_blocks(n), (unsigned)R.max_blocks);
+}
+
 void launch_sum(cudaStream_t s, const double* x, size_t n, const ReduceScratch& R, int slot) {
-  const unsigned b = std::min<unsigned>(stride_blocks(n), (unsigned)R.max_blocks);
+  const unsigned b = (unsigned)sum_blocks(n, R);
   k_sum<<<b, kRedThreads, 0, s>>>(x, n, R, slot);
 }
 
@@ -591,10 +591,6 @@ void launch_shift_by_mean(cudaStream_t s, const double* x, double* y, size_t n,
 
 void launch_add_float(cudaStream_t s, double* p, const float* e, size_t n) {
   k_add_float<<<stride_blocks(n) * 2, kRedThreads, 0, s>>>(p, e, n);
-}
-
-void launch_float_to_double(cudaStream_t s, const float* a, double* b, size_t n) {
-  k_f2d<<<stride_blocks(n) * 2, kRedThreads, 0, s>>>(a, b, n);
 }
 
 void launch_double_to_float(cudaStream_t s, const double* a, float* b, size_t n) {

@@ -100,20 +100,26 @@ __global__ void __launch_bounds__(256) k_diag(LevelView<double> L, double* diag)
   diag[q] = d;
 }
 
-// q = A d and sum d.q (the Krylov matrix product): a warp per row, the
-// diagonal read back instead of summed, 8 FP64 operations per cell for 13
-// (bound by the FP64 pipe: 512^3, 3.5 ms before)
+// q = A d and (kDot) sum d.q (the Krylov matrix product): a warp per 128 cells
+// of a row, the diagonal read back instead of summed, 8 FP64 operations per
+// cell for 13 (bound by the FP64 pipe: 512^3, 3.5 ms before; a warp per whole
+// row left 1024^2 with 7 warps per SM)
+constexpr int kApplySeg = 128;
+
+template <bool kDot>
 __global__ void __launch_bounds__(kRedThreads)
     k_apply_diag(LevelView<double> L, const double* __restrict__ diag,
                  const double* __restrict__ dvec, double* __restrict__ qvec, ReduceScratch R,
                  int slot, int keep_rz) {
   double acc[1] = {0.0};
-  const int rows = L.ny * L.nz;
+  const int segs = (L.nx + kApplySeg - 1) / kApplySeg;
+  const int items = L.ny * L.nz * segs;
   const int lane = threadIdx.x & 31, warps = kRedThreads / 32;
   const size_t sy = (size_t)L.nx, sz = (size_t)L.nx * L.ny;
-  for (int row = blockIdx.x * warps + (threadIdx.x >> 5); row < rows; row += gridDim.x * warps) {
+  for (int it = blockIdx.x * warps + (threadIdx.x >> 5); it < items; it += gridDim.x * warps) {
+    const int row = it / segs, i0 = (it - row * segs) * kApplySeg;
     const int j = row % L.ny, k = row / L.ny;
-    for (int i = lane; i < L.nx; i += 32) {
+    for (int i = i0 + lane; i < min(L.nx, i0 + kApplySeg); i += 32) {
       const size_t q = ((size_t)k * L.ny + j) * L.nx + i;
       double s = 0.0;
       if (i > 0) s += L.cx[q] * dvec[q - 1];
@@ -124,9 +130,10 @@ __global__ void __launch_bounds__(kRedThreads)
       if (k < L.nz - 1) s += L.cz[q + sz] * dvec[q + sz];
       const double a = s - diag[q] * dvec[q];
       qvec[q] = a;
-      acc[0] += dvec[q] * a;
+      if (kDot) acc[0] += dvec[q] * a;
     }
   }
+  if (!kDot) return;
   if (keep_rz && blockIdx.x == 0 && threadIdx.x == 0)
     R.result[kSlotDot2 + 1] = R.result[kSlotDot];
   grid_sum_finish<1>(acc, R, slot);
@@ -488,8 +495,10 @@ void launch_diag(cudaStream_t s, const LevelView<double>& L, double* diag) {
 void launch_apply_diag(cudaStream_t s, const LevelView<double>& L, const double* diag,
                        const double* d, double* q, const ReduceScratch& R, int slot,
                        bool keep_rz) {
-  const int blocks = std::min(reduce_blocks_for(((size_t)L.ny * L.nz + 7) / 8), R.max_blocks);
-  k_apply_diag<<<blocks, kRedThreads, 0, s>>>(L, diag, d, q, R, slot, keep_rz ? 1 : 0);
+  const size_t items = (size_t)L.ny * L.nz * cdiv((size_t)L.nx, kApplySeg);
+  const int blocks = std::min(reduce_blocks_for(items * 32), R.max_blocks);
+  if (slot < 0) k_apply_diag<false><<<blocks, kRedThreads, 0, s>>>(L, diag, d, q, R, slot, 0);
+  else k_apply_diag<true><<<blocks, kRedThreads, 0, s>>>(L, diag, d, q, R, slot, keep_rz ? 1 : 0);
 }
 
 template <typename T>

@@ -445,16 +445,6 @@ __global__ void k_to_split(const double* __restrict__ a, float* __restrict__ out
   out[(size_t)((i + j + k) & 1) * half + (q >> 1)] = (float)a[q];
 }
 
-__global__ void k_from_split(const float* __restrict__ a, double* __restrict__ out, int nx, int ny,
-                             int nz, size_t half) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z;
-  if (i >= nx || j >= ny) return;
-  const size_t q = ((size_t)k * ny + j) * nx + i;
-  out[q] = (double)a[(size_t)((i + j + k) & 1) * half + (q >> 1)];
-}
-
 }  // namespace
 
 // the four-cell kernels need rows of whole float4 groups in each half
@@ -505,13 +495,6 @@ void launch_to_split(cudaStream_t s, const double* a, float* out, int nx, int ny
   const dim3 blk(32, 8, 1);
   const dim3 grd(cdiv((size_t)nx, 32), cdiv((size_t)ny, 8), (unsigned)nz);
   k_to_split<<<grd, blk, 0, s>>>(a, out, nx, ny, nz, hstride);
-}
-
-void launch_from_split(cudaStream_t s, const float* a, double* out, int nx, int ny, int nz,
-                       size_t hstride) {
-  const dim3 blk(32, 8, 1);
-  const dim3 grd(cdiv((size_t)nx, 32), cdiv((size_t)ny, 8), (unsigned)nz);
-  k_from_split<<<grd, blk, 0, s>>>(a, out, nx, ny, nz, hstride);
 }
 
 }  // namespace gbmg

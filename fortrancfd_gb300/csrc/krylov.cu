@@ -1,117 +1,362 @@
 // Vector kernels of the flexible GMRES outer iteration (sm_103a).
 //
-// Block Gram-Schmidt needs, per Arnoldi step j, the j+1 dot products of the
-// new vector w with the basis V_0..V_j and the update w -= sum_i h_i V_i.
-// k_mdot reads w once per basis vector from L2 and writes per-block partial
-// sums; k_mdot_finish adds each dot's partials in block order (one block per
-// dot, the same order every run, so results are bit-reproducible);
-// k_maxpy applies the j+1 coefficients in index order.  The basis is one
-// array of cnt vectors of n doubles at a stride of ld.
+// Per Arnoldi step j, around the V-cycle on v_j:
+//   k_gm_z       z_j = the V-cycle's result less its mean, into Z_j
+//   k_apply_diag w = A z_j
+//   k_gm_dots    the j+1 products V_i.w and w.w
+//   k_gm_update  w -= sum_i h_i V_i, |w|^2 and 1/|w|
+//   k_gm_next    v_{j+1} = w/|w| into V_{j+1} and into the V-cycle's right-hand side
+// The products and the update are an FP64 operation per basis element each,
+// for 8 bytes read: the FP64 pipe (2 lanes per clock and SM) takes 1.8 us per
+// 1024^2 vector, memory 1.25 us, so both passes are bound by that pipe and
+// everything beside the one operation is kept off it: w is read once for all
+// vectors, and the sums of a warp are folded together (9 additions for eight
+// sums, 40 one by one, which with four elements per thread were more than the
+// products).  1024^2, 12 vectors on average: products 36 + 4 us, update 37, mean
+// 18, v 8; before, 65 + 2 x 31 (a pass per vector, separate norms), 28, 31 with two
+// conversions, and two copies of 6.
+// The sums keep a fixed order (thread: stride of the grid; warp: halves;
+// block: warps in order; then blocks the same way), whatever is summed together:
+// the vectors go to float for the next V-cycle, and a last bit that differs here
+// is a float's last bit there.  The basis is one array of vectors of n doubles
+// at a stride of ld.
 #include "gbmg_internal.h"
+#include "idiv.h"
+#include "pairs.cuh"
+#include "pdl.cuh"
 
 namespace gbmg {
 
 namespace {
 
-constexpr int kMThreads = 256;
+constexpr int kGmThreads = 256, kGmWarps = kGmThreads / 32;
+constexpr int kGmVals = 32;  // sums of one launch
 
-template <int NV>
-__device__ __forceinline__ double block_sum1(double v, double* ws) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+// sums of the lanes' a[0..NV-1]: sum v in a[0] of the lanes v * 32/NV and up
+template <int NV, int kOff = 16>
+__device__ __forceinline__ void warp_fold(double* a) {
+  if constexpr (NV > 1) {
+    const bool up = threadIdx.x & kOff;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if (lane == 0) ws[wid] = v;
+    for (int u = 0; u < NV / 2; ++u) {
+      const double lo = a[u], hi = a[u + NV / 2];
+      a[u] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, kOff);
+    }
+  } else {
+    a[0] += __shfl_xor_sync(0xffffffffu, a[0], kOff);
+  }
+  if constexpr (kOff > 1) warp_fold<(NV > 1 ? NV / 2 : 1), kOff / 2>(a);
+}
+
+// sum of one value per thread of the block (valid in thread 0)
+__device__ __forceinline__ double block_fold(double v, double* ws) {
+  double a[1] = {v};
+  warp_fold<1>(a);
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = a[0];
   __syncthreads();
   double t = 0.0;
   if (threadIdx.x == 0)
-    for (int w = 0; w < NV; ++w) t += ws[w];
+    for (int w = 0; w < kGmWarps; ++w) t += ws[w];
   __syncthreads();
   return t;
 }
 
-__global__ void __launch_bounds__(kMThreads) k_mdot(const double* __restrict__ V, size_t ld, int cnt,
-                                                    const double* __restrict__ w, size_t n,
-                                                    double* __restrict__ partials) {
-  __shared__ double ws[kMThreads / 32];
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (int i = 0; i < cnt; ++i) {
-    const double* vi = V + (size_t)i * ld;
-    double acc = 0.0;
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += stride)
-      acc += vi[q] * w[q];
-    const double t = block_sum1<kMThreads / 32>(acc, ws);
-    if (threadIdx.x == 0) partials[(size_t)i * gridDim.x + blockIdx.x] = t;
+// sum of the partials of a launch's blocks (valid in thread 0)
+__device__ __forceinline__ double blocks_fold(const double* partials, int blocks, double* ws) {
+  double a = 0.0;
+  for (int b = threadIdx.x; b < blocks; b += kGmThreads) a += __ldcg(partials + b);
+  return block_fold(a, ws);
+}
+
+// partials of V_i.w, i < cnt, and of w.w as the one after; 4 (G - 1) <= cnt < 4 G
+template <int G>
+__global__ void __launch_bounds__(kGmThreads, G <= 4 ? 3 : 2)
+    k_gm_dots(const double* __restrict__ V, size_t ld, int cnt, const double* __restrict__ w,
+              size_t n, double* __restrict__ partials) {
+  pdl_enter();
+  __shared__ double ws[kGmWarps][kGmVals];
+  const size_t step = (size_t)gridDim.x * kGmThreads;
+  double a[4 * G];
+#pragma unroll
+  for (int v = 0; v < 4 * G; ++v) a[v] = 0.0;
+  // (the last group alone may be short, and holds w.w)
+  const auto in = [&](int g, int u) { return g < G - 1 || u == 0 || 4 * g + u <= cnt; };
+  const auto self = [&](int g, int u) { return g == G - 1 && 4 * g + u == cnt; };
+  size_t q = (size_t)blockIdx.x * kGmThreads + threadIdx.x;
+  for (; q + step < n; q += 2 * step) {
+    const double w0 = w[q], w1 = w[q + step];
+    const double* v = V + q;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      double v0[4], v1[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u, v += ld)
+        if (in(g, u)) {
+          const double* p = self(g, u) ? w + q : v;
+          v0[u] = p[0];
+          v1[u] = p[step];
+        }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (in(g, u)) {
+          a[4 * g + u] += v0[u] * w0;
+          a[4 * g + u] += v1[u] * w1;
+        }
+    }
+  }
+  if (q < n) {
+    const double w0 = w[q];
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (in(g, u)) a[4 * g + u] += (self(g, u) ? w : V + (size_t)(4 * g + u) * ld)[q] * w0;
+  }
+  const int lane = threadIdx.x & 31;
+  double* mine = ws[threadIdx.x >> 5];
+#pragma unroll
+  for (int g = 0; g + 1 < G; g += 2) {
+    warp_fold<8>(a + 4 * g);
+    if (lane % 4 == 0) mine[4 * g + lane / 4] = a[4 * g];
+  }
+  if constexpr (G & 1) {
+    warp_fold<4>(a + 4 * (G - 1));
+    if (lane % 8 == 0) mine[4 * (G - 1) + lane / 8] = a[4 * (G - 1)];
+  }
+  __syncthreads();
+  if ((int)threadIdx.x <= cnt) {
+    double t = 0.0;
+#pragma unroll
+    for (int u = 0; u < kGmWarps; ++u) t += ws[u][threadIdx.x];
+    partials[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = t;
   }
 }
 
-__global__ void __launch_bounds__(kMThreads) k_mdot_finish(const double* __restrict__ partials,
-                                                           int blocks, double* __restrict__ out) {
-  __shared__ double ws[kMThreads / 32];
-  const int i = blockIdx.x;
-  double acc = 0.0;
-  for (int b = threadIdx.x; b < blocks; b += blockDim.x) acc += partials[(size_t)i * blocks + b];
-  const double t = block_sum1<kMThreads / 32>(acc, ws);
-  if (threadIdx.x == 0) out[i] = t;
+// out[i] = the sum of the blocks' partials, a block per sum
+__global__ void __launch_bounds__(kGmThreads) k_gm_finish(const double* __restrict__ partials,
+                                                          int blocks, double* __restrict__ out) {
+  pdl_enter();
+  __shared__ double ws[kGmWarps];
+  const double t = blocks_fold(partials + (size_t)blockIdx.x * blocks, blocks, ws);
+  if (threadIdx.x == 0) out[blockIdx.x] = t;
 }
 
-// w += sign * sum_i coef[i] V_i
-__global__ void __launch_bounds__(kMThreads) k_maxpy(double* __restrict__ w,
-                                                     const double* __restrict__ V, size_t ld,
-                                                     const double* __restrict__ coef, int cnt,
-                                                     double sign, size_t n) {
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n;
-       q += (size_t)gridDim.x * blockDim.x) {
-    double acc = 0.0;
-    for (int i = 0; i < cnt; ++i) acc += coef[i] * V[(size_t)i * ld + q];
-    w[q] += sign * acc;
+// w += sign * sum_i coef[i] V_i (added in index order); kNorm: nrm[0] = |w|^2,
+// nrm[1] = 1/|w| (0 for w = 0)
+template <bool kNorm>
+__global__ void __launch_bounds__(kGmThreads, 4)
+    k_gm_update(double* __restrict__ w, const double* __restrict__ V, size_t ld,
+                const double* __restrict__ coef, int cnt, double sign, size_t n, double* partials,
+                unsigned int* counter, double* nrm) {
+  pdl_enter();
+  __shared__ double ws[kGmWarps], c[kGmVals];
+  __shared__ bool last;
+  if (threadIdx.x < (unsigned)cnt) c[threadIdx.x] = coef[threadIdx.x];
+  __syncthreads();
+  const size_t step = (size_t)gridDim.x * kGmThreads;
+  double s = 0.0;
+  size_t q = (size_t)blockIdx.x * kGmThreads + threadIdx.x;
+  for (; q + step < n; q += 2 * step) {
+    const double w0 = w[q], w1 = w[q + step];
+    double a0 = 0.0, a1 = 0.0;
+    const double* v = V + q;
+#pragma unroll 4
+    for (int i = 0; i < cnt; ++i, v += ld) {
+      a0 += c[i] * v[0];
+      a1 += c[i] * v[step];
+    }
+    const double x0 = w0 + sign * a0, x1 = w1 + sign * a1;
+    w[q] = x0;
+    w[q + step] = x1;
+    if (kNorm) {
+      s += x0 * x0;
+      s += x1 * x1;
+    }
+  }
+  if (q < n) {
+    double a = 0.0;
+    for (int i = 0; i < cnt; ++i) a += c[i] * V[(size_t)i * ld + q];
+    const double x = w[q] + sign * a;
+    w[q] = x;
+    if (kNorm) s += x * x;
+  }
+  if (kNorm) {
+    const double t = block_fold(s, ws);
+    if (threadIdx.x == 0) {
+      partials[blockIdx.x] = t;
+      __threadfence();
+      last = atomicAdd(counter, 1u) == gridDim.x - 1u;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const double r = blocks_fold(partials, (int)gridDim.x, ws);
+    if (threadIdx.x == 0) {
+      nrm[0] = r;
+      nrm[1] = r > 0.0 ? 1.0 / sqrt(r) : 0.0;
+      *counter = 0u;
+    }
   }
 }
 
-// out may be in (scaling in place)
-__global__ void __launch_bounds__(kMThreads) k_scale_copy(double* out, const double* in,
-                                                          double alpha, size_t n) {
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n;
-       q += (size_t)gridDim.x * blockDim.x)
-    out[q] = alpha * in[q];
+// v = scale * w (scale read from inv when there is one), and v as the V-cycle's
+// right-hand side: src64 (K = kZ64), or rounded to float in the level's layout.
+// w may be src64.
+template <int K>
+__global__ void __launch_bounds__(kGmThreads)
+    k_gm_next(double* __restrict__ v, const double* w, const double* __restrict__ inv, double scale,
+              double* src64, float* __restrict__ src32, size_t n, PairRows P, size_t hstride) {
+  const double a = inv ? *inv : scale;
+  const size_t step = (size_t)gridDim.x * kGmThreads;
+  for (size_t m = (size_t)blockIdx.x * kGmThreads + threadIdx.x; m < n / 2; m += step) {
+    const double2 x = reinterpret_cast<const double2*>(w)[m];
+    const double2 y = make_double2(a * x.x, a * x.y);
+    reinterpret_cast<double2*>(v)[m] = y;
+    if constexpr (K == kZ64) reinterpret_cast<double2*>(src64)[m] = y;
+    else store_pair32<K>(src32, m, y.x, y.y, P, hstride);
+  }
+  if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
+    const double y = a * w[n - 1];
+    v[n - 1] = y;
+    if constexpr (K == kZ64) src64[n - 1] = y;
+    else src32[n - 1] = (float)y;
+  }
 }
 
-// w *= 1/sqrt(*nrm2) (w unchanged when the norm is 0)
-__global__ void __launch_bounds__(kMThreads) k_scale_rsqrt(double* w, const double* nrm2,
-                                                           size_t n) {
-  const double v = *nrm2;
-  if (!(v > 0.0)) return;
-  const double a = 1.0 / sqrt(v);
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n;
-       q += (size_t)gridDim.x * blockDim.x)
-    w[q] = a * w[q];
+// The sum of the V-cycle's FP32 result into R.result[slot], the additions of k_sum on
+// its FP64 copy: kSumTogether of its blocks in one, their warps folded together
+// (1024^2: 18.7 us before, beside the copy)
+constexpr int kSumTogether = 4;
+
+template <int K>
+__global__ void __launch_bounds__(kGmThreads)
+    k_gm_sum(const float* __restrict__ z, size_t n, PairRows P, size_t hstride, int blocks,
+             ReduceScratch R, int slot) {
+  static_assert(kGmThreads == kRedThreads, "k_sum's blocks");
+  __shared__ double ws[kGmWarps][kSumTogether], fin[kGmWarps];
+  __shared__ bool last;
+  const size_t step = (size_t)blocks * kGmThreads;
+  const int b0 = blockIdx.x * kSumTogether;
+  double a[kSumTogether] = {0.0, 0.0, 0.0, 0.0};
+  const auto load = [&](size_t q) {
+    if constexpr (K == kZSplit)
+      return z[(size_t)(pair_colour(P, q >> 1) ^ (int)(q & 1)) * hstride + (q >> 1)];
+    else return z[q];
+  };
+  size_t q = (size_t)b0 * kGmThreads + threadIdx.x;
+  for (; q < n; q += step) {
+    float v[kSumTogether];
+#pragma unroll
+    for (int u = 0; u < kSumTogether; ++u) {
+      const size_t e = q + (size_t)u * kGmThreads;
+      v[u] = b0 + u < blocks && e < n ? load(e) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < kSumTogether; ++u)
+      if (b0 + u < blocks && q + (size_t)u * kGmThreads < n) a[u] += float_to_double_int(v[u]);
+  }
+  const int lane = threadIdx.x & 31;
+  warp_fold<kSumTogether>(a);
+  if (lane % (32 / kSumTogether) == 0) ws[threadIdx.x >> 5][lane / (32 / kSumTogether)] = a[0];
+  __syncthreads();
+  if (threadIdx.x < kSumTogether) {
+    const int u = threadIdx.x;
+    const double t = ((ws[0][u] + ws[4][u]) + (ws[2][u] + ws[6][u])) +
+                     ((ws[1][u] + ws[5][u]) + (ws[3][u] + ws[7][u]));
+    if (b0 + u < blocks) R.partials[b0 + u] = t;
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(R.counter, 1u) == gridDim.x - 1u;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double acc[1] = {0.0};
+  for (int b = threadIdx.x; b < blocks; b += kGmThreads) acc[0] += __ldcg(&R.partials[b]);
+  warp_fold<1>(acc);
+  if (lane == 0) fin[threadIdx.x >> 5] = acc[0];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    R.result[slot] = ((fin[0] + fin[4]) + (fin[2] + fin[6])) + ((fin[1] + fin[5]) + (fin[3] + fin[7]));
+    *R.counter = 0u;
+  }
 }
 
-unsigned grid_for(size_t n, int max_blocks) {
-  size_t b = (n + kMThreads - 1) / kMThreads;
-  if (b > (size_t)max_blocks) b = (size_t)max_blocks;
-  return (unsigned)(b > 0 ? b : 1);
+// out = z - (sum of z)/n
+template <int K>
+__global__ void __launch_bounds__(kGmThreads)
+    k_gm_z(const void* __restrict__ z, double* __restrict__ out, size_t n, PairRows P,
+           size_t hstride, const double* __restrict__ sum) {
+  const double mean = div_int(*sum, rcp_int((double)n));
+  const size_t step = (size_t)gridDim.x * kGmThreads;
+  for (size_t m = (size_t)blockIdx.x * kGmThreads + threadIdx.x; m < n / 2; m += step) {
+    const double2 x = widen(load_pair<K>(z, m, P, hstride));
+    reinterpret_cast<double2*>(out)[m] = make_double2(x.x - mean, x.y - mean);
+  }
+  if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) out[n - 1] = load_one<K>(z, n - 1) - mean;
+}
+
+unsigned gm_blocks(size_t items, unsigned most) {
+  const size_t b = (items + kGmThreads - 1) / kGmThreads;
+  return (unsigned)std::max<size_t>(1, std::min<size_t>(b, most));
 }
 
 }  // namespace
 
-void launch_mdot(cudaStream_t s, const double* V, size_t ld, int cnt, const double* w, size_t n,
-                 double* partials, int max_blocks, double* out) {
-  const unsigned g = grid_for(n, max_blocks);
-  k_mdot<<<g, kMThreads, 0, s>>>(V, ld, cnt, w, n, partials);
-  k_mdot_finish<<<(unsigned)cnt, kMThreads, 0, s>>>(partials, (int)g, out);
+namespace {
+template <int G>
+void dots_groups(cudaStream_t s, unsigned b, const double* V, size_t ld, int cnt, const double* w,
+                 size_t n, double* partials) {
+  if constexpr (G > 1)
+    if (cnt < 4 * (G - 1)) return dots_groups<G - 1>(s, b, V, ld, cnt, w, n, partials);
+  launch_pdl(k_gm_dots<G>, dim3(b), dim3(kGmThreads), 0, s, V, ld, cnt, w, n, partials);
+}
+}  // namespace
+
+void launch_gm_dots(cudaStream_t s, const double* V, size_t ld, int cnt, const double* w, size_t n,
+                    double* partials, double* out) {
+  static_assert(kGmresRestart < kGmVals, "sums of one launch");
+  const unsigned b = gm_blocks(n, kGmresBlocks);
+  dots_groups<kGmVals / 4>(s, b, V, ld, cnt, w, n, partials);
+  launch_pdl(k_gm_finish, dim3((unsigned)cnt + 1u), dim3(kGmThreads), 0, s,
+             (const double*)partials, (int)b, out);
 }
 
-void launch_maxpy(cudaStream_t s, double* w, const double* V, size_t ld, const double* coef,
-                  int cnt, double sign, size_t n) {
-  k_maxpy<<<grid_for(n, 4096), kMThreads, 0, s>>>(w, V, ld, coef, cnt, sign, n);
+void launch_gm_update(cudaStream_t s, double* w, const double* V, size_t ld, const double* coef,
+                      int cnt, double sign, size_t n, double* partials, unsigned int* counter,
+                      double* nrm) {
+  const dim3 b(gm_blocks(n, kGmresBlocks)), t(kGmThreads);
+  if (nrm)
+    launch_pdl(k_gm_update<true>, b, t, 0, s, w, V, ld, coef, cnt, sign, n, partials, counter, nrm);
+  else
+    launch_pdl(k_gm_update<false>, b, t, 0, s, w, V, ld, coef, cnt, sign, n, partials, counter, nrm);
 }
 
-void launch_scale_copy(cudaStream_t s, double* out, const double* in, double alpha, size_t n) {
-  k_scale_copy<<<grid_for(n, 4096), kMThreads, 0, s>>>(out, in, alpha, n);
+void launch_gm_sum(cudaStream_t s, const PcgVec& z, const ReduceScratch& R, int slot) {
+  if (z.z64) return launch_sum(s, z.z64, z.n, R, slot);
+  const PairRows P = pair_rows(z.nx, z.ny);
+  const int blocks = sum_blocks(z.n, R);
+  const unsigned b = (unsigned)(blocks + kSumTogether - 1) / kSumTogether;
+  if (z.hstride) k_gm_sum<kZSplit><<<b, kGmThreads, 0, s>>>(z.z32, z.n, P, z.hstride, blocks, R, slot);
+  else k_gm_sum<kZ32><<<b, kGmThreads, 0, s>>>(z.z32, z.n, P, 0, blocks, R, slot);
 }
 
-void launch_scale_rsqrt(cudaStream_t s, double* w, const double* nrm2, size_t n) {
-  k_scale_rsqrt<<<grid_for(n, 4096), kMThreads, 0, s>>>(w, nrm2, n);
+void launch_gm_next(cudaStream_t s, double* v, const double* w, const double* inv, double scale,
+                    double* src64, float* src32, const PcgVec& z) {
+  const PairRows P = pair_rows(z.nx, z.ny);
+  const unsigned b = gm_blocks(z.n / 2, 152 * 8);
+  if (src64) k_gm_next<kZ64><<<b, kGmThreads, 0, s>>>(v, w, inv, scale, src64, src32, z.n, P, 0);
+  else if (z.hstride)
+    k_gm_next<kZSplit><<<b, kGmThreads, 0, s>>>(v, w, inv, scale, src64, src32, z.n, P, z.hstride);
+  else k_gm_next<kZ32><<<b, kGmThreads, 0, s>>>(v, w, inv, scale, src64, src32, z.n, P, 0);
+}
+
+void launch_gm_z(cudaStream_t s, const PcgVec& z, double* out, const double* sum) {
+  const PairRows P = pair_rows(z.nx, z.ny);
+  const unsigned b = gm_blocks(z.n / 2, 152 * 8);
+  if (z.z64) k_gm_z<kZ64><<<b, kGmThreads, 0, s>>>(z.z64, out, z.n, P, 0, sum);
+  else if (z.hstride) k_gm_z<kZSplit><<<b, kGmThreads, 0, s>>>(z.z32, out, z.n, P, z.hstride, sum);
+  else k_gm_z<kZ32><<<b, kGmThreads, 0, s>>>(z.z32, out, z.n, P, 0, sum);
 }
 
 }  // namespace gbmg

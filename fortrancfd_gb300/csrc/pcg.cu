@@ -18,65 +18,14 @@
 // z is read straight from the V-cycle's result: FP64, FP32, or FP32 in the
 // colour-split layout (cell q in half (i+j+k)&1 at q/2).  All passes work on
 // pairs of cells (2m, 2m+1), which share a row when nx is even.
-#include <algorithm>
-
 #include "dword.cuh"
 #include "gbmg_internal.h"
+#include "pairs.cuh"
 #include "reduce.cuh"
 
 namespace gbmg {
 
 namespace {
-
-enum : int { kZ64 = 0, kZ32 = 1, kZSplit = 2 };
-
-// row and plane of a pair by products with 2^64/divisor (an integer division
-// by a variable goes through the FP64 pipe): exact for m * divisor < 2^64
-struct PairRows {
-  unsigned hx, ny;
-  unsigned long long rx, ry;  // floor(2^64 / hx) + 1, floor(2^64 / ny) + 1; 0 for a divisor of 1
-};
-
-__device__ __forceinline__ unsigned long long div_by(unsigned long long m, unsigned long long r) {
-  return r ? __umul64hi(m, r) : m;
-}
-
-__device__ __forceinline__ int pair_colour(const PairRows& P, unsigned long long m) {
-  const unsigned long long row = div_by(m, P.rx);
-  const unsigned long long k = div_by(row, P.ry);
-  return (int)((row - k * P.ny + k) & 1ull);  // (j + k) & 1: the colour of cell 2m
-}
-
-// cells 2m and 2m+1 of z as floats
-template <int K>
-__device__ __forceinline__ float2 load_pair32(const float* __restrict__ z, size_t m,
-                                              const PairRows& P, size_t hstride) {
-  if constexpr (K == kZSplit) {
-    const int c = pair_colour(P, m);
-    return make_float2(z[(size_t)c * hstride + m], z[(size_t)(1 - c) * hstride + m]);
-  } else {
-    return reinterpret_cast<const float2*>(z)[m];
-  }
-}
-
-template <int K>
-__device__ __forceinline__ auto load_pair(const void* __restrict__ z, size_t m, const PairRows& P,
-                                          size_t hstride) {
-  if constexpr (K == kZ64) return reinterpret_cast<const double2*>(z)[m];
-  else return load_pair32<K>(static_cast<const float*>(z), m, P, hstride);
-}
-
-__device__ __forceinline__ double2 widen(double2 v) { return v; }
-__device__ __forceinline__ double2 widen(float2 v) {
-  return make_double2(float_to_double_int(v.x), float_to_double_int(v.y));
-}
-
-// a last cell without a partner (n odd; never split)
-template <int K>
-__device__ __forceinline__ double load_one(const void* __restrict__ z, size_t q) {
-  if constexpr (K == kZ64) return static_cast<const double*>(z)[q];
-  else return (double)static_cast<const float*>(z)[q];
-}
 
 // sum of floats in three cascaded parts (TwoSum at each step; Ogita, Rump and
 // Oishi, "Accurate sum and dot product", SIAM J. Sci. Comput. 26(6), 2005):
@@ -188,16 +137,7 @@ __global__ void __launch_bounds__(kRedThreads)
     r2[m] = make_double2(a, b);
     acc[0] += a * a;
     acc[0] += b * b;
-    if constexpr (K != kZ64) {
-      const float fa = dw_from_double_int(a).hi, fb = dw_from_double_int(b).hi;
-      if constexpr (K == kZSplit) {
-        const int c = pair_colour(P, m);
-        r32[(size_t)c * hstride + m] = fa;
-        r32[(size_t)(1 - c) * hstride + m] = fb;
-      } else {
-        reinterpret_cast<float2*>(r32)[m] = make_float2(fa, fb);
-      }
-    }
+    if constexpr (K != kZ64) store_pair32<K>(r32, m, a, b, P, hstride);
   };
   size_t m = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t pairs = n / 2;
@@ -219,26 +159,13 @@ __global__ void __launch_bounds__(kRedThreads)
   grid_sum_finish<1>(acc, R, kSlotNorm);
 }
 
-PairRows pair_rows(int nx, int ny) {
-  PairRows P{};
-  P.hx = (unsigned)std::max(nx / 2, 1);
-  P.ny = (unsigned)ny;
-  P.rx = P.hx == 1 ? 0ull : ~0ull / P.hx + 1;
-  P.ry = P.ny == 1 ? 0ull : ~0ull / P.ny + 1;
-  return P;
-}
-
-unsigned blocks_of(size_t items, const ReduceScratch& R) {
-  const size_t b = (items + kRedThreads - 1) / kRedThreads;
-  return (unsigned)std::max<size_t>(
-      1, std::min<size_t>(b, std::min<size_t>(152 * 8, (size_t)R.max_blocks)));
-}
-
 }  // namespace
 
 void launch_pcg_sum(cudaStream_t s, const PcgVec& v, const ReduceScratch& R, int slot) {
   const PairRows P = pair_rows(v.nx, v.ny);
-  const unsigned b = blocks_of(v.n, R);
+  // 16 cells a thread: the FP64 additions that join the threads' sums cost as
+  // much as reading 50 cells each (1024^2: 14.8 us at 4 cells a thread)
+  const unsigned b = std::max(blocks_of(v.n / 16, R), std::min(blocks_of(v.n, R), 152u));
   if (v.z64) k_pcg_sum<kZ64><<<b, kRedThreads, 0, s>>>(v.z64, v.n, P, 0, R, slot);
   else if (v.hstride) k_pcg_sum<kZSplit><<<b, kRedThreads, 0, s>>>(v.z32, v.n, P, v.hstride, R, slot);
   else k_pcg_sum<kZ32><<<b, kRedThreads, 0, s>>>(v.z32, v.n, P, 0, R, slot);

@@ -1,0 +1,40 @@
+"""Flexible GMRES's vector passes (products in groups of one to eight basis vectors,
+the update with the norm, the scaled vector written in the V-cycle's layout) over
+odd and even cell counts, FP64 and FP32 levels in both layouts, a preconditioner
+from a zero guess with no sweeps before the coarse correction, and enough steps for
+every group size: the true FP64 residual and the oracle's solution, as the
+parity test of the same solver asks."""
+import numpy as np
+import pytest
+
+from fortrancfd_gb300 import PressurePoisson, inputs
+from oracle import oracle as orc
+from tests import cases
+from tests.cases import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shape", [(1, 7, 7), (1, 24, 40), (16, 24, 40), (1, 128, 64)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("nu", [(2, 2), (1, 0), (0, 1)])
+def test_residual_and_solution(cuda, shape, precision, nu):
+    nz, ny, nx = shape
+    n = max(shape)
+    ext = tuple(m / n if m > 1 else 1.0 for m in (nx, ny, nz))
+    c = cases.Built(inputs.custom(shape, extent=ext, radii=(0.2,), seed=3,
+                                  centers=(tuple(0.45 * e for e in ext),)))
+    want, st_or = orc.mg_solve(c.coef, c.b, tol=1e-10, krylov=1)
+    assert st_or["status"] == 0
+    out = []
+    for graph in (True, False):
+        with PressurePoisson(c.shape, c.spacing, precision=precision, krylov="fgmres",
+                             max_cycles=400, nu1=nu[0], nu2=nu[1], use_graph=graph) as s:
+            s.ppe_init(c.rho)
+            p, st = s.solve(c.b, tol=1e-10)
+        assert st["status"] == 0
+        out.append(p)
+    _, r2 = orc.residual(c.coef, p, c.b)
+    assert np.sqrt(r2) / np.linalg.norm(c.b) < 1e-10
+    assert rel_l2(p, want) <= 1e-9
+    assert np.array_equal(out[0], out[1])
