@@ -315,7 +315,7 @@ void setup_subcycle(gbmg_handle* h) {
   if (h->sub_lc >= h->L) return;
   const SubCycle<T> S = make_subcycle<T>(h, false);
   const size_t smem = subcycle_smem<T>(S);
-  if (smem > 200 * 1024 || subcycle_init<T>(smem) != 0) h->sub_lc = h->L;
+  if (subcycle_init<T>(smem) != 0) h->sub_lc = h->L;
 }
 
 // TMA maps of the double-word defect kernel (finest level with nx % 4 == 0;

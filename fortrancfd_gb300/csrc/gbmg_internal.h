@@ -102,6 +102,7 @@ enum : int {
 // and ten separate launches about 30 (the whole 256^3 FP64 bottom 164 us before).
 constexpr int kSubMaxCells = 4096, kSubMaxCells64 = 1024;
 constexpr int kSubMaxLevels = 8;
+constexpr size_t kSubMaxSmem = 200 * 1024;  // its shared memory at most
 template <typename T>
 struct SubLevel {
   int nx, ny, nz;

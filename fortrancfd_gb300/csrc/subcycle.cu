@@ -412,10 +412,14 @@ size_t subcycle_smem(const SubCycle<T>& S) {
   return (size_t)(S.off[S.nlev] + n0 + 2 * S.n_coarse * S.n_coarse + kMaxCoarse) * sizeof(T);
 }
 
+// The attribute belongs to the kernel, not to a handle: every handle sets the same
+// limit (with its own need, a later and smaller handle took the launch from an
+// earlier one: invalid argument).
 template <typename T>
 int subcycle_init(size_t smem) {
-  return cudaFuncSetAttribute(k_subcycle<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)smem) == cudaSuccess
+  return smem <= kSubMaxSmem &&
+                 cudaFuncSetAttribute(k_subcycle<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kSubMaxSmem) == cudaSuccess
              ? 0
              : -1;
 }

@@ -32,3 +32,17 @@ def test_same_bits_as_separate_launches(cuda, monkeypatch, shape, nu):
         got.append(p)
     assert np.isfinite(got[0]).all()
     assert np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_a_smaller_handle_leaves_an_earlier_one_alone(cuda, precision):
+    """The block's shared-memory limit is the kernel's, shared by all handles."""
+    big, small = cases.config(1, 8), cases.Built(inputs.custom(
+        (1, 16, 16), extent=(1.0, 1.0, 1.0), radii=(0.2,), seed=3, centers=((0.5, 0.5, 0.5),)))
+    with PressurePoisson(big.shape, big.spacing, precision=precision) as s:
+        with PressurePoisson(small.shape, small.spacing, precision=precision) as t:
+            t.ppe_init(small.rho)
+            t.solve(small.b, tol=1e-8)
+            s.ppe_init(big.rho)
+            _, st = s.solve(big.b, tol=1e-8)
+    assert st["status"] == 0
