@@ -160,6 +160,46 @@ SubCycle<T> make_subcycle(gbmg_handle* h, bool reverse) {
   return S;
 }
 
+template <typename T> T* alt_of(const Level& l);
+template <> double* alt_of<double>(const Level& l) { return l.alt; }
+template <> float* alt_of<float>(const Level& l) { return l.alt32; }
+
+// Launches that `nu` sweeps of a level take in tiles
+int tile_launches(int nu) { return (nu + kTileSweeps - 1) / kTileSweeps; }
+
+// Whether level l runs in tiles: the unknown changes its array with every launch
+// and has to end in its own, which a zero guess can always arrange.  The finest
+// level of a mixed solve does in its colour-split layout.
+bool by_tiles(const gbmg_handle* h, int l, bool zero) {
+  const Level& v = h->lv[l];
+  if (!v.tile || (l == 0 && h->mixed && !v.split)) return false;
+  return zero || (tile_launches(h->prm.nu1) + tile_launches(h->prm.nu2)) % 2 == 0;
+}
+
+// Sweeps of level l down (with the restriction) or up (with the prolongation).
+template <typename T>
+void tile_leg(gbmg_handle* h, int l, bool up, int first, bool zero) {
+  const Level& v = h->lv[l];
+  const LevelView<T> F = view<T>(v), C = view<T>(h->lv[l + 1]);
+  T* buf[2] = {F.sol, alt_of<T>(v)};
+  // launches still to come, this one included: an odd number writes the
+  // unknown's own array
+  int left = tile_launches(h->prm.nu2) + (up ? 0 : tile_launches(h->prm.nu1));
+  int n = up ? h->prm.nu2 : h->prm.nu1;
+  const int cs = l == 0 ? GBMG_PROF_SMOOTH_FINE : GBMG_PROF_SMOOTH_COARSE;
+  for (bool start = true; n > 0; start = false, --left) {
+    const int m = std::min(n, kTileSweeps);
+    n -= m;
+    const bool last = n == 0;
+    TileEnds e = kTilePlain;
+    if (up && start) e = kTileProlong;
+    else if (!up && start && zero) e = last ? kTileZeroRestrict : kTileZero;
+    else if (!up && last) e = kTileRestrict;
+    const int to = left & 1 ? 0 : 1;
+    LAUNCH(h, cs, launch_tile<T>(h->stream, F, C, buf[1 - to], buf[to], m, first, e));
+  }
+}
+
 // One V-cycle on the current level-0 (sol, src) of type T.  reverse_post runs
 // the post-smoothing colours black-first (symmetric preconditioner for CG).
 // zero_fine: the level-0 unknown starts at zero (correction and Krylov
@@ -171,8 +211,12 @@ int enqueue_vcycle(gbmg_handle* h, bool reverse_post, bool zero_fine) {
   const bool pre = h->prm.nu1 > 0;
   const int top = std::min(h->sub_lc, L - 1);  // levels above the bottom block
   for (int l = 0; l < top; ++l) {
-    for (int it = 0; it < h->prm.nu1; ++it)
-      sweep<T>(h, l, 0, it == 0 && (l > 0 || zero_fine));
+    const bool zero = l > 0 || zero_fine;
+    if (by_tiles(h, l, zero)) {
+      tile_leg<T>(h, l, false, 0, zero);
+      continue;
+    }
+    for (int it = 0; it < h->prm.nu1; ++it) sweep<T>(h, l, 0, it == 0 && zero);
     LAUNCH(h, l == 0 ? GBMG_PROF_RESTRICT_FINE : GBMG_PROF_RESTRICT_COARSE,
            launch_restrict<T>(s, view_next<T>(h->lv[l]), view<T>(h->lv[l + 1]), !pre, pre));
   }
@@ -184,6 +228,10 @@ int enqueue_vcycle(gbmg_handle* h, bool reverse_post, bool zero_fine) {
            launch_coarse_solve<T>(s, h->nc, minv_of<T>(h), adense_of<T>(h), C.src, C.sol));
   }
   for (int l = top - 1; l >= 0; --l) {
+    if (by_tiles(h, l, l > 0 || zero_fine)) {
+      tile_leg<T>(h, l, true, reverse_post ? 1 : 0, false);
+      continue;
+    }
     // A colour launch does not read its own colour's values (Gauss-Seidel
     // overwrites them), so the colour that the first post-smoothing launch
     // updates needs no correction: only the other one is corrected.  Results
@@ -266,6 +314,7 @@ int free_all(gbmg_handle* h) {
     dfree(v.cx); dfree(v.cy); dfree(v.cz); dfree(v.idiag);
     if (l > 0) { dfree(v.sol); dfree(v.src); }
     dfree(v.cx32); dfree(v.cy32); dfree(v.cz32); dfree(v.sol32); dfree(v.src32);
+    dfree(v.alt); dfree(v.alt32);
   }
   dfree(h->b); dfree(h->p); dfree(h->rho); dfree(h->rho32);
   dfree(h->pw[0]); dfree(h->pw[1]); dfree(h->bw); dfree(h->cxw); dfree(h->cyw); dfree(h->czw);
@@ -306,9 +355,12 @@ void setup_subcycle(gbmg_handle* h) {
   h->sub_lc = h->L;
   if (const char* e = std::getenv("GBMG_SUBCYCLE"))
     if (std::atoi(e) == 0) return;
+  // (levels that tiles can take leave the block earlier)
+  const bool tiles = h->tiles && h->grid.nz == 1 && h->grid.nx > 1 && h->grid.ny > 1;
+  const size_t most = h->mixed ? (tiles ? kSubMaxCellsTiles : kSubMaxCells)
+                               : (tiles ? kSubMaxCells64Tiles : kSubMaxCells64);
   for (int l = 1; l + 1 < h->L; ++l)
-    if (h->lv[l].n <= (size_t)(h->mixed ? kSubMaxCells : kSubMaxCells64) &&
-        h->L - l <= kSubMaxLevels) {
+    if (h->lv[l].n <= most && h->L - l <= kSubMaxLevels) {
       h->sub_lc = l;
       break;
     }
@@ -316,6 +368,21 @@ void setup_subcycle(gbmg_handle* h) {
   const SubCycle<T> S = make_subcycle<T>(h, false);
   const size_t smem = subcycle_smem<T>(S);
   if (subcycle_init<T>(smem) != 0) h->sub_lc = h->L;
+}
+
+// The levels that run in tiles, with their second arrays.
+int setup_tiles(gbmg_handle* h) {
+  if (!h->tiles) return GBMG_OK;
+  const int top = std::min(h->sub_lc, h->L - 1);
+  for (int l = 0; l < top; ++l) {
+    Level& v = h->lv[l];
+    const bool finest = l == 0 && h->mixed;
+    v.tile = tile_level(v.nx, v.ny, v.nz, v.fx, v.fy);
+    if (!v.tile) continue;
+    if (h->mixed) GB_TRY(dmalloc(h, &v.alt32, finest ? v.n + kSplitPadMax : v.n));
+    else GB_TRY(dmalloc(h, &v.alt, v.n));
+  }
+  return GBMG_OK;
 }
 
 // TMA maps of the double-word defect kernel (finest level with nx % 4 == 0;
@@ -436,8 +503,12 @@ int allocate(gbmg_handle* h) {
   GB_TRY(dmalloc(h, &h->derr, 4));
   GB_CUDA(h, cudaMemsetAsync(h->derr, 0, 4 * sizeof(int), h->stream));
   if (h->mixed) GB_TRY(setup_tma(h));
+  // (GBMG_TILES=0: every level above the bottom takes separate launches)
+  const char* et = std::getenv("GBMG_TILES");
+  h->tiles = h->prm.nu1 > 0 && h->prm.nu2 > 0 && !(et && std::atoi(et) == 0);
   if (h->mixed) setup_subcycle<float>(h);
   else setup_subcycle<double>(h);
+  GB_TRY(setup_tiles(h));
   GB_CUDA(h, cudaEventCreate(&h->ev0));
   GB_CUDA(h, cudaStreamCreateWithFlags(&h->cstream, cudaStreamNonBlocking));
   for (int i = 0; i < 5; ++i) GB_CUDA(h, cudaEventCreateWithFlags(&h->cev[i], cudaEventDisableTiming));

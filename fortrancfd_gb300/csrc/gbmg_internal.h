@@ -101,6 +101,10 @@ enum : int {
 // per clock, so a 4096-cell level costs the block 55 us of arithmetic per cycle
 // and ten separate launches about 30 (the whole 256^3 FP64 bottom 164 us before).
 constexpr int kSubMaxCells = 4096, kSubMaxCells64 = 1024;
+// 2D levels in tiles (tiles.cu) cost two launches of about 2.5 us each, less than
+// this block: a 128^2 FP64 cycle takes 49.5 us with its 32^2 level in tiles, 56.5
+// in the block; a 1024^2 FP32 cycle 83.9 us with 64^2 in tiles, 87.9 in the block.
+constexpr int kSubMaxCellsTiles = 1024, kSubMaxCells64Tiles = 256;
 constexpr int kSubMaxLevels = 8;
 constexpr size_t kSubMaxSmem = 200 * 1024;  // its shared memory at most
 template <typename T>
@@ -132,6 +136,20 @@ template <typename T>
 int subcycle_init(size_t smem);
 template <typename T>
 void launch_subcycle(cudaStream_t s, const SubCycle<T>& S);
+
+// ---- 2D levels by tiles (tiles.cu) -------------------------------------------
+// What a launch does besides its sweeps: kTileZero starts from a zero guess,
+// kTileRestrict restricts the residual behind them, kTileProlong adds the coarse
+// correction before them.
+enum TileEnds { kTilePlain, kTileZero, kTileRestrict, kTileZeroRestrict, kTileProlong };
+// sweeps of one launch at most
+constexpr int kTileSweeps = 2;
+// whether a level may run in tiles
+bool tile_level(int nx, int ny, int nz, int fx, int fy);
+// `sweeps` red-black sweeps of level F, in -> out (distinct arrays); C: the next level
+template <typename T>
+void launch_tile(cudaStream_t s, const LevelView<T>& F, const LevelView<T>& C, const T* in, T* out,
+                 int sweeps, int first, TileEnds e);
 
 // ---- launchers (kernels_mg.cu) ---------------------------------------------
 // zero_guess: the level's current values are taken as zero (first colour of

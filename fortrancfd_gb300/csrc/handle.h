@@ -28,6 +28,9 @@ struct Level {
   float k32[3] = {0.f, 0.f, 0.f};  // 2/h^2 per axis
   int split = 0;  // sol32, src32 and rho32 in the colour-split layout
   size_t hstride = 0;  // distance between the colour halves (elements)
+  bool tile = false;   // the level runs in tiles
+  double* alt = nullptr;   // tiles: the unknown's second array
+  float* alt32 = nullptr;
   int zrev = 0;   // direction of the next split-kernel launch (toggles per launch)
 };
 
@@ -91,6 +94,7 @@ struct gbmg_handle {
   // the residual is under 1000 tol
   int stag_mode = 0;
   bool stagnated = false;
+  bool tiles = false;     // 2D levels above the bottom block in tiles
   int sub_lc = 0;         // first level run by the one-block bottom of the cycle (L = none)
   int* derr = nullptr;   // device error flags (bulk-copy wait timeouts)
   gbmg::DefectMaps* dmaps = nullptr;  // TMA maps of the defect kernel: [p buffer][e: none,
