@@ -148,8 +148,14 @@ SubCycle<T> make_subcycle(gbmg_handle* h, bool reverse) {
                           rcp(V.nx), rcp(V.ny), rcp((V.nx + 1) / 2),
                           V.nz > 1 ? V.nx * V.ny : V.nx, T(1) / T(V.fx * V.fy * V.fz)};
     S.off[i] = off;
+    const int n = V.nx * V.ny * V.nz, pad = S.lv[i].pad;
+    S.lv[i].at_sol = off + pad;
+    S.lv[i].at_src = off + n + 2 * pad;
+    S.lv[i].at_c = off + 2 * (n + pad);
+    S.lv[i].at_na = n + pad;
     // sol, src, the three coefficient arrays and 1/diagonal, with their padding
-    off += (V.idiag ? 6 : 5) * V.nx * V.ny * V.nz + 5 * S.lv[i].pad;
+    off += (V.idiag ? 6 : 5) * n + 5 * pad;
+    off += off & 1;  // (pairs of values are read together)
   }
   S.off[S.nlev] = off;
   const LevelView<T> V0 = view<T>(h->lv[lc]);

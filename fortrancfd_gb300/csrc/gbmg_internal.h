@@ -119,6 +119,9 @@ struct SubLevel {
   unsigned rx, ry, rh;
   int pad;  // zeros around an array in shared memory: a plane (2D: a row)
   T mean;   // 1/(fx fy fz)
+  // offsets in shared memory: unknown, right-hand side, coefficients (each of
+  // the arrays at_na long)
+  int at_sol, at_src, at_c, at_na;
 };
 template <typename T>
 struct SubCycle {
