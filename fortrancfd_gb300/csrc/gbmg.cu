@@ -968,12 +968,15 @@ int gm_vcycle(gbmg_handle* h) {
 // Flexible GMRES(kGmresRestart) around the V-cycle (right preconditioning,
 // Saad's FGMRES): the residual norm falls monotonically, where conjugate
 // gradients can first raise it many-fold on a smooth right-hand side (the
-// adjoint of a smooth objective).  Per Arnoldi step: z_j = M v_j (the V-cycle one captured
-// graph) and w = A z_j, classical Gram-Schmidt on the device with a second pass only when the
-// first removed most of w, one copy of the coefficients to the host for the
-// Givens rotations, and w scaled into v_{j+1} while the host does these.  At each restart and at
-// the end the true FP64 residual b - A p
-// is recomputed.  On entry kr holds r0 = b - A p and host_res[kSlotNorm] its
+// adjoint of a smooth objective).  Per Arnoldi step: z_j = M v_j (the V-cycle one
+// captured graph) and w = A z_j, classical Gram-Schmidt with a second pass only
+// when the first removed most of w, decided on the device, one copy of the
+// coefficients to the host for the Givens rotations, and w scaled into v_{j+1}
+// meanwhile.  Where the last reduction of the residual does not promise that this
+// step is the last, the next step's V-cycle is launched before the host waits: it
+// reads the device's data alone, and the GPU has work while the host rotates (a
+// step of 1024^2 left it idle for 50 of 345 us with two waits per step).  At each
+// restart and at the end the true FP64 residual b - A p is recomputed.  On entry kr holds r0 = b - A p and host_res[kSlotNorm] its
 // squared norm.
 int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles, int* status) {
   const cudaStream_t s = h->stream;
@@ -985,22 +988,13 @@ int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles
   const PcgVec z = gm_vec(h);
   double* h1 = h->gmDev;               // first Gram-Schmidt pass, then |w|^2 before it
   double* h2 = h->gmDev + (m + 2);     // second pass
-  double* nrm = h->gmDev + 2 * (m + 2);  // |w|^2 after, 1/|w|
+  double* nrm = h->gmDev + 2 * (m + 2);  // |w|^2 at the end, 1/|w|
+  double* nrm1 = nrm + 2;  // after the first pass, and whether there is a second
   double* src64 = h->mixed ? nullptr : h->kr;
   float* src32 = h->mixed ? f.src32 : nullptr;
-  // coefficients to the host, v_{j+1} written meanwhile
-  const auto fetch = [&](int j) -> int {
-    GB_CUDA(h, cudaMemcpyAsync(h->gmHost, h->gmDev, 3 * (m + 2) * sizeof(double),
-                               cudaMemcpyDeviceToHost, s));
-    GB_CUDA(h, cudaEventRecord(h->gmEv, s));
-    LAUNCH(h, VC, launch_gm_next(s, h->gmV + (size_t)(j + 1) * ld, h->kq, nrm + 1, 0.0, src64,
-                                 src32, z));
-    GB_CUDA(h, cudaEventSynchronize(h->gmEv));
-    return check_launch(h, "arnoldi");
-  };
   std::vector<double> H((size_t)(m + 1) * m, 0.0), cs(m), sn(m), g(m + 1), y(m), col(m + 1);
   double r2 = h->host_res[kSlotNorm];
-  double rel = *rel_io;
+  double rel = *rel_io, factor = 0.2;  // factor: last reduction of the residual
   int total = 0;
   *status = GBMG_NOT_CONVERGED;
   while (total < h->prm.max_cycles) {
@@ -1010,31 +1004,36 @@ int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles
     std::fill(g.begin(), g.end(), 0.0);
     g[0] = beta;
     int j = 0;
+    bool ahead = false;  // the step's V-cycle is already launched
     for (; j < m && total < h->prm.max_cycles;) {
       double* w = h->kq;  // A z_j, orthogonalised in place, then scaled into V_{j+1}
       double* zj = h->gmZ + (size_t)j * ld;
-      GB_TRY(gm_vcycle(h));
+      if (!ahead) GB_TRY(gm_vcycle(h));
       LAUNCH(h, VC, launch_gm_z(s, z, zj, h->red.result + kSlotSum));
       LAUNCH(h, GBMG_PROF_RESIDUAL, launch_apply_diag(s, v64(f), h->kdiag, zj, w, h->red, -1, false));
       // classical Gram-Schmidt; a second pass only when the first removed most
       // of w (|w| fell below 0.7 of its length: "twice is enough")
-      LAUNCH(h, VC, launch_gm_dots(s, h->gmV, ld, j + 1, w, n, h->gmPart, h1));
+      LAUNCH(h, VC, launch_gm_dots(s, h->gmV, ld, j + 1, w, n, h->gmPart, h1, nullptr));
       LAUNCH(h, VC, launch_gm_update(s, w, h->gmV, ld, h1, j + 1, -1.0, n, h->gmPart,
-                                     h->red.counter, nrm));
-      ++h->launches;  // the products' finishing kernel
-      GB_TRY(fetch(j));
+                                     h->red.counter, nrm1, h1 + j + 1, nullptr));
+      LAUNCH(h, VC, launch_gm_dots(s, h->gmV, ld, j + 1, w, n, h->gmPart, h2, nrm1));
+      LAUNCH(h, VC, launch_gm_update(s, w, h->gmV, ld, h2, j + 1, -1.0, n, h->gmPart,
+                                     h->red.counter, nrm, nullptr, nrm1));
+      h->launches += 2;  // the products' finishing kernels
+      GB_CUDA(h, cudaMemcpyAsync(h->gmHost, h->gmDev, 3 * (m + 2) * sizeof(double),
+                                 cudaMemcpyDeviceToHost, s));
+      GB_CUDA(h, cudaEventRecord(h->gmEv, s));
+      LAUNCH(h, VC, launch_gm_next(s, h->gmV + (size_t)(j + 1) * ld, w, nrm + 1, 0.0, src64,
+                                   src32, z));
+      ahead = j + 1 < m && total + 1 < h->prm.max_cycles && rel * factor > 1.5 * tol;
+      if (ahead) GB_TRY(gm_vcycle(h));
+      GB_CUDA(h, cudaEventSynchronize(h->gmEv));
+      GB_TRY(check_launch(h, "arnoldi"));
       for (int i = 0; i <= j; ++i) col[i] = h->gmHost[i];
-      double hn = std::sqrt(h->gmHost[2 * (m + 2)]);
-      const double before = std::sqrt(h->gmHost[j + 1]);
-      if (hn < 0.7 * before) {
-        LAUNCH(h, VC, launch_gm_dots(s, h->gmV, ld, j + 1, w, n, h->gmPart, h2));
-        LAUNCH(h, VC, launch_gm_update(s, w, h->gmV, ld, h2, j + 1, -1.0, n, h->gmPart,
-                                       h->red.counter, nrm));
-        ++h->launches;
-        GB_TRY(fetch(j));
+      const double* norms = h->gmHost + 2 * (m + 2);
+      const double hn = std::sqrt(norms[0]);
+      if (norms[4] != 0.0)
         for (int i = 0; i <= j; ++i) col[i] += h->gmHost[(m + 2) + i];
-        hn = std::sqrt(h->gmHost[2 * (m + 2)]);
-      }
       col[j + 1] = hn;
       for (int i = 0; i < j; ++i) {
         const double t = cs[i] * col[i] + sn[i] * col[i + 1];
@@ -1051,7 +1050,9 @@ int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles
       for (int i = 0; i <= j; ++i) H[(size_t)i * m + j] = col[i];
       ++j;
       ++total;
+      const double last = rel;
       rel = std::fabs(g[j]) / scale;
+      factor = rel < last ? rel / last : 1.0;
       if (!std::isfinite(rel) || rel < tol || !(hn > 0.0)) break;
     }
     // x += Z y with R y = g (R: the rotated Hessenberg, upper triangular)
@@ -1062,7 +1063,8 @@ int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles
     }
     std::copy(y.begin(), y.begin() + j, h->gmHost);
     GB_CUDA(h, cudaMemcpyAsync(h->gmDev, h->gmHost, j * sizeof(double), cudaMemcpyHostToDevice, s));
-    LAUNCH(h, VC, launch_gm_update(s, h->p, h->gmZ, ld, h->gmDev, j, 1.0, n, nullptr, nullptr, nullptr));
+    LAUNCH(h, VC, launch_gm_update(s, h->p, h->gmZ, ld, h->gmDev, j, 1.0, n, nullptr, nullptr, nullptr,
+                                   nullptr, nullptr));
     f.sol = h->p; f.src = h->b;
     LAUNCH(h, GBMG_PROF_RESIDUAL,
            launch_residual_norm<double>(s, v64(f), h->kr, h->red, kSlotNorm));

@@ -330,13 +330,16 @@ constexpr int kGmresRestart = 30;   // restart length
 constexpr int kGmresBlocks = 1024;  // blocks of the products and the update
 // the sum of z
 void launch_gm_sum(cudaStream_t s, const PcgVec& z, const ReduceScratch& R, int slot);
-// out[i] = V_i.w for i < cnt, out[cnt] = w.w
+// out[i] = V_i.w for i < cnt, out[cnt] = w.w.  first: null in a first Gram-Schmidt
+// pass, in a second one the first one's nrm; its kernels return at once where the
+// verdict there is 0.
 void launch_gm_dots(cudaStream_t s, const double* V, size_t ld, int cnt, const double* w, size_t n,
-                    double* partials, double* out);
-// w += sign * sum_i coef[i] V_i; nrm (may be null): |w|^2, 1/|w|
+                    double* partials, double* out, const double* first);
+// w += sign * sum_i coef[i] V_i; nrm (may be null): |w|^2, 1/|w| and, with |w|^2 as it
+// was before, whether a second pass is needed
 void launch_gm_update(cudaStream_t s, double* w, const double* V, size_t ld, const double* coef,
                       int cnt, double sign, size_t n, double* partials, unsigned int* counter,
-                      double* nrm);
+                      double* nrm, const double* before, const double* first);
 // v = (*inv or scale) * w, and the same as the V-cycle's right-hand side: src64,
 // or src32 in z's layout
 void launch_gm_next(cudaStream_t s, double* v, const double* w, const double* inv, double scale,

@@ -68,12 +68,20 @@ __device__ __forceinline__ double blocks_fold(const double* partials, int blocks
   return block_fold(a, ws);
 }
 
+// Whether a pass runs: the first one does, the second one where the first one's
+// norms say so (the verdict is a double's bits: a comparison of its own in every
+// thread, two roots, cost the FP64 pipe 20 us at 1024^2).
+__device__ __forceinline__ bool gm_runs(const double* first) {
+  return !first || __double_as_longlong(__ldcg(first + 2)) != 0;
+}
+
 // partials of V_i.w, i < cnt, and of w.w as the one after; 4 (G - 1) <= cnt < 4 G
 template <int G>
 __global__ void __launch_bounds__(kGmThreads, G <= 4 ? 3 : 2)
     k_gm_dots(const double* __restrict__ V, size_t ld, int cnt, const double* __restrict__ w,
-              size_t n, double* __restrict__ partials) {
+              size_t n, double* __restrict__ partials, const double* first) {
   pdl_enter();
+  if (!gm_runs(first)) return;
   __shared__ double ws[kGmWarps][kGmVals];
   const size_t step = (size_t)gridDim.x * kGmThreads;
   double a[4 * G];
@@ -134,21 +142,29 @@ __global__ void __launch_bounds__(kGmThreads, G <= 4 ? 3 : 2)
 
 // out[i] = the sum of the blocks' partials, a block per sum
 __global__ void __launch_bounds__(kGmThreads) k_gm_finish(const double* __restrict__ partials,
-                                                          int blocks, double* __restrict__ out) {
+                                                          int blocks, double* __restrict__ out,
+                                                          const double* first) {
   pdl_enter();
+  if (!gm_runs(first)) return;
   __shared__ double ws[kGmWarps];
   const double t = blocks_fold(partials + (size_t)blockIdx.x * blocks, blocks, ws);
   if (threadIdx.x == 0) out[blockIdx.x] = t;
 }
 
 // w += sign * sum_i coef[i] V_i (added in index order); kNorm: nrm[0] = |w|^2,
-// nrm[1] = 1/|w| (0 for w = 0)
+// nrm[1] = 1/|w| (0 for w = 0), and from the first pass nrm[2] = 1 when it left less
+// than 0.7 of the length sqrt(*before) ("twice is enough"): a second pass that is
+// not needed takes the first one's norms
 template <bool kNorm>
 __global__ void __launch_bounds__(kGmThreads, 4)
     k_gm_update(double* __restrict__ w, const double* __restrict__ V, size_t ld,
                 const double* __restrict__ coef, int cnt, double sign, size_t n, double* partials,
-                unsigned int* counter, double* nrm) {
+                unsigned int* counter, double* nrm, const double* before, const double* first) {
   pdl_enter();
+  if (!gm_runs(first)) {
+    if (kNorm && blockIdx.x == 0 && threadIdx.x < 2) nrm[threadIdx.x] = first[threadIdx.x];
+    return;
+  }
   __shared__ double ws[kGmWarps], c[kGmVals];
   __shared__ bool last;
   if (threadIdx.x < (unsigned)cnt) c[threadIdx.x] = coef[threadIdx.x];
@@ -194,6 +210,7 @@ __global__ void __launch_bounds__(kGmThreads, 4)
     if (threadIdx.x == 0) {
       nrm[0] = r;
       nrm[1] = r > 0.0 ? 1.0 / sqrt(r) : 0.0;
+      if (before) nrm[2] = sqrt(r) < 0.7 * sqrt(*before) ? 1.0 : 0.0;
       *counter = 0u;
     }
   }
@@ -306,30 +323,30 @@ unsigned gm_blocks(size_t items, unsigned most) {
 namespace {
 template <int G>
 void dots_groups(cudaStream_t s, unsigned b, const double* V, size_t ld, int cnt, const double* w,
-                 size_t n, double* partials) {
+                 size_t n, double* partials, const double* first) {
   if constexpr (G > 1)
-    if (cnt < 4 * (G - 1)) return dots_groups<G - 1>(s, b, V, ld, cnt, w, n, partials);
-  launch_pdl(k_gm_dots<G>, dim3(b), dim3(kGmThreads), 0, s, V, ld, cnt, w, n, partials);
+    if (cnt < 4 * (G - 1)) return dots_groups<G - 1>(s, b, V, ld, cnt, w, n, partials, first);
+  launch_pdl(k_gm_dots<G>, dim3(b), dim3(kGmThreads), 0, s, V, ld, cnt, w, n, partials, first);
 }
 }  // namespace
 
 void launch_gm_dots(cudaStream_t s, const double* V, size_t ld, int cnt, const double* w, size_t n,
-                    double* partials, double* out) {
+                    double* partials, double* out, const double* first) {
   static_assert(kGmresRestart < kGmVals, "sums of one launch");
   const unsigned b = gm_blocks(n, kGmresBlocks);
-  dots_groups<kGmVals / 4>(s, b, V, ld, cnt, w, n, partials);
+  dots_groups<kGmVals / 4>(s, b, V, ld, cnt, w, n, partials, first);
   launch_pdl(k_gm_finish, dim3((unsigned)cnt + 1u), dim3(kGmThreads), 0, s,
-             (const double*)partials, (int)b, out);
+             (const double*)partials, (int)b, out, first);
 }
 
 void launch_gm_update(cudaStream_t s, double* w, const double* V, size_t ld, const double* coef,
                       int cnt, double sign, size_t n, double* partials, unsigned int* counter,
-                      double* nrm) {
+                      double* nrm, const double* before, const double* first) {
   const dim3 b(gm_blocks(n, kGmresBlocks)), t(kGmThreads);
   if (nrm)
-    launch_pdl(k_gm_update<true>, b, t, 0, s, w, V, ld, coef, cnt, sign, n, partials, counter, nrm);
+    launch_pdl(k_gm_update<true>, b, t, 0, s, w, V, ld, coef, cnt, sign, n, partials, counter, nrm, before, first);
   else
-    launch_pdl(k_gm_update<false>, b, t, 0, s, w, V, ld, coef, cnt, sign, n, partials, counter, nrm);
+    launch_pdl(k_gm_update<false>, b, t, 0, s, w, V, ld, coef, cnt, sign, n, partials, counter, nrm, before, first);
 }
 
 void launch_gm_sum(cudaStream_t s, const PcgVec& z, const ReduceScratch& R, int slot) {

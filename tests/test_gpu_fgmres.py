@@ -38,3 +38,29 @@ def test_residual_and_solution(cuda, shape, precision, nu):
     assert np.sqrt(r2) / np.linalg.norm(c.b) < 1e-10
     assert rel_l2(p, want) <= 1e-9
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_cycle_limit_and_restart(cuda, precision):
+    """The V-cycle launched ahead of the host's tests ends with the cycle limit and
+    with the basis (30 vectors): the asked number of steps, the reported residual
+    that of the returned p in FP64 (its norms differ by rounding, 1e-10 of it here:
+    it stays above 1e-5 of b), never larger after more steps."""
+    shape = (1, 128, 64)
+    c = cases.Built(inputs.custom(shape, extent=(0.5, 1.0, 1.0), radii=(0.2,), seed=3,
+                                  centers=((0.25, 0.5, 0.5),)))
+    rels = []
+    for k in (1, 2, 5, 29, 30, 31, 61):
+        # (one sweep before the coarse correction alone: many steps)
+        with PressurePoisson(c.shape, c.spacing, precision=precision, krylov="fgmres",
+                             max_cycles=k, nu1=1, nu2=0) as s:
+            s.ppe_init(c.rho)
+            p, st = s.solve(c.b, tol=1e-300, check=False)
+        _, r2 = orc.residual(c.coef, p, c.b)
+        rel = np.sqrt(r2) / np.linalg.norm(c.b)
+        assert st["cycles"] == k
+        if rel > 1e-5:
+            assert abs(st["rel_residual"] - rel) <= 1e-10 * rel
+            rels.append(rel)
+    assert len(rels) >= 2
+    assert all(b <= a * (1 + 1e-6) for a, b in zip(rels, rels[1:]))
