@@ -61,7 +61,9 @@ int plan_levels(const gbmg_grid& g, int levels, int coarse_max, int dims[][3]) {
 }
 
 LevelView<double> v64(const Level& l) {
-  return LevelView<double>{l.nx, l.ny, l.nz, l.fx, l.fy, l.fz, l.cx, l.cy, l.cz, l.idiag, l.sol, l.src};
+  LevelView<double> v{l.nx, l.ny, l.nz, l.fx, l.fy, l.fz, l.cx, l.cy, l.cz, l.idiag, l.sol, l.src};
+  v.diag = l.diag;
+  return v;
 }
 LevelView<float> v32(const Level& l) {
   LevelView<float> v{l.nx, l.ny, l.nz, l.fx, l.fy, l.fz, l.cx32, l.cy32, l.cz32, nullptr,
@@ -317,7 +319,7 @@ int free_all(gbmg_handle* h) {
   reset_graphs(h);
   for (int l = 0; l < h->L; ++l) {
     Level& v = h->lv[l];
-    dfree(v.cx); dfree(v.cy); dfree(v.cz); dfree(v.idiag);
+    dfree(v.cx); dfree(v.cy); dfree(v.cz); dfree(v.idiag); dfree(v.diag);
     if (l > 0) { dfree(v.sol); dfree(v.src); }
     dfree(v.cx32); dfree(v.cy32); dfree(v.cz32); dfree(v.sol32); dfree(v.src32);
     dfree(v.alt); dfree(v.alt32);
@@ -515,6 +517,10 @@ int allocate(gbmg_handle* h) {
   if (h->mixed) setup_subcycle<float>(h);
   else setup_subcycle<double>(h);
   GB_TRY(setup_tiles(h));
+  // the restriction of the FP64 levels reads their diagonal
+  if (!h->mixed)
+    for (int l = 0; l < std::min(h->sub_lc, L - 1); ++l)
+      if (!h->lv[l].tile) GB_TRY(dmalloc(h, &h->lv[l].diag, h->lv[l].n));
   GB_CUDA(h, cudaEventCreate(&h->ev0));
   GB_CUDA(h, cudaStreamCreateWithFlags(&h->cstream, cudaStreamNonBlocking));
   for (int i = 0; i < 5; ++i) GB_CUDA(h, cudaEventCreateWithFlags(&h->cev[i], cudaEventDisableTiming));
@@ -538,7 +544,7 @@ int build_hierarchy(gbmg_handle* h) {
   }
   for (int l = 0; l < h->L; ++l) {
     Level& v = h->lv[l];
-    if (v.idiag) LAUNCH(h, GBMG_PROF_SETUP, launch_idiag(s, v64(v), v.idiag));
+    if (v.idiag) LAUNCH(h, GBMG_PROF_SETUP, launch_idiag(s, v64(v), v.idiag, v.diag));
     if (l == 0 && v.cx32 && !h->fine_copies) {
       LAUNCH(h, GBMG_PROF_SETUP, launch_to_float(s, v.cx, v.cx32, v.n));
       LAUNCH(h, GBMG_PROF_SETUP, launch_to_float(s, v.cy, v.cy32, v.n));

@@ -45,6 +45,7 @@ struct LevelView {
   // on the finest level alternate direction, so each starts on the planes the
   // previous one touched last, which are still in L2
   int zrev = 0;
+  const T* diag = nullptr;  // sum of a cell's face coefficients, where it is stored (FP64)
 };
 
 // Deterministic single-pass grid reduction scratch: per-block partial sums,
@@ -184,7 +185,8 @@ struct Float3Out {
 };
 void launch_coarsen(cudaStream_t s, const LevelView<double>& F, double* cx, double* cy,
                     double* cz, int cnx, int cny, int cnz, Float3Out c32 = Float3Out{});
-void launch_idiag(cudaStream_t s, const LevelView<double>& L, double* idiag);
+// 1/diagonal, and the diagonal itself (may be null)
+void launch_idiag(cudaStream_t s, const LevelView<double>& L, double* idiag, double* diag);
 void launch_to_float(cudaStream_t s, const double* a, float* b, size_t n);
 
 // ---- launchers (kernels_flow.cu) -------------------------------------------

@@ -18,7 +18,7 @@ struct Level {
   int nx = 0, ny = 0, nz = 0;
   int fx = 1, fy = 1, fz = 1;
   size_t n = 0;
-  double *cx = nullptr, *cy = nullptr, *cz = nullptr, *idiag = nullptr;
+  double *cx = nullptr, *cy = nullptr, *cz = nullptr, *idiag = nullptr, *diag = nullptr;
   double *sol = nullptr, *src = nullptr;  // owned on levels >= 1
   float *cx32 = nullptr, *cy32 = nullptr, *cz32 = nullptr;
   float *sol32 = nullptr, *src32 = nullptr;

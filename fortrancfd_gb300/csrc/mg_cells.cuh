@@ -43,6 +43,21 @@ __device__ __forceinline__ void stencil(const LevelView<T>& L, const T* __restri
   if (k < L.nz - 1) { c = L.cz[q + sz]; s += c * ldc<kCg>(p + q + sz); d += c; }
 }
 
+// The neighbour sum alone.
+template <typename T, bool kCg = false>
+__device__ __forceinline__ T neighbour_sum(const LevelView<T>& L, const T* __restrict__ p, int i,
+                                           int j, int k, size_t q) {
+  const size_t sy = (size_t)L.nx, sz = (size_t)L.nx * L.ny;
+  T s = T(0);
+  if (i > 0) s += L.cx[q] * ldc<kCg>(p + q - 1);
+  if (i < L.nx - 1) s += L.cx[q + 1] * ldc<kCg>(p + q + 1);
+  if (j > 0) s += L.cy[q] * ldc<kCg>(p + q - sy);
+  if (j < L.ny - 1) s += L.cy[q + sy] * ldc<kCg>(p + q + sy);
+  if (k > 0) s += L.cz[q] * ldc<kCg>(p + q - sz);
+  if (k < L.nz - 1) s += L.cz[q + sz] * ldc<kCg>(p + q + sz);
+  return s;
+}
+
 // Face coefficient k/(rho_a + rho_b) of the density form.  FP32 uses the
 // approximate reciprocal (within 1 ulp): these coefficients only drive the
 // FP32 smoother and restriction of the mixed-precision cycle, whose result is
@@ -174,7 +189,8 @@ __device__ __forceinline__ void smooth_cell(const LevelView<T>& L, int i, int j,
 // kHalf: the level's last colour launch relaxed the cells of colour 1, whose
 // residual is therefore zero up to the rounding of the update: only the
 // children of colour 0 are visited (half the arithmetic; 256^3 FP64, bound by
-// the FP64 pipe, 484 -> 261 us).  FP64 only: in FP32 that rounding reaches 1e-4
+// the FP64 pipe, 484 -> 261 us), with the diagonal read back where it is stored
+// (9 operations a child for 14: 164 us).  FP64 only: in FP32 that rounding reaches 1e-4
 // of the residual within a correction's four cycles, enough to move the mixed
 // loop's schedule and with it the error left at the tolerance.
 template <typename T, bool kRho, bool kHalf, bool kCg = false>
@@ -189,7 +205,12 @@ __device__ __forceinline__ void restrict_cell(const LevelView<T>& F, const Level
         if (F.fx == 1 && ((i + j + k) & 1)) continue;
         const size_t q = ((size_t)k * F.ny + j) * F.nx + i;
         T s, d;
-        stencil<T, kCg>(F, F.sol, i, j, k, q, s, d);
+        if (F.diag) {
+          s = neighbour_sum<T, kCg>(F, F.sol, i, j, k, q);
+          d = F.diag[q];  // (the same sum of the coefficients)
+        } else {
+          stencil<T, kCg>(F, F.sol, i, j, k, q, s, d);
+        }
         acc += ldc<kCg>(F.src + q) - (s - d * ldc<kCg>(F.sol + q));
       }
   } else if (F.fx == 2) {
@@ -290,6 +311,32 @@ __device__ __forceinline__ void prolong_cell(const LevelView<T>& F, const LevelV
   const size_t cq = (size_t)K * csz + (size_t)J * csy + I;
   const T* e = C.sol;
   const T ec = ldc<kCg>(e + cq);
+  if constexpr (sizeof(T) == 8) {
+    if (F.fx == 2 && live >= 0) {
+      // the same roundings in 17 FP64 operations for 22: halves and quarters are
+      // exact, so each slope is one fused multiply-add of a difference (256^3,
+      // bound by the FP64 pipe, 125 -> 70 us)
+      const T dx = (I < C.nx - 1 ? ldc<kCg>(e + cq + 1) : ec) - (I > 0 ? ldc<kCg>(e + cq - 1) : ec);
+      const T vx[2] = {fma(T(-0.125), dx, ec), fma(T(0.125), dx, ec)};
+      const T gy = F.fy == 2 ? (J < C.ny - 1 ? ldc<kCg>(e + cq + csy) : ec) -
+                                   (J > 0 ? ldc<kCg>(e + cq - csy) : ec)
+                             : T(0);
+      const T gz = F.fz == 2 ? (K < C.nz - 1 ? ldc<kCg>(e + cq + csz) : ec) -
+                                   (K > 0 ? ldc<kCg>(e + cq - csz) : ec)
+                             : T(0);
+      for (int dz = 0; dz < F.fz; ++dz)
+        for (int dy = 0; dy < F.fy; ++dy) {
+          const int j = F.fy * J + dy, k = F.fz * K + dz;
+          const int o = (j + k + live) & 1;  // the live child: x = 2I + o
+          T v = o ? vx[1] : vx[0];
+          if (F.fy == 2) v = fma(dy ? T(0.125) : T(-0.125), gy, v);
+          if (F.fz == 2) v = fma(dz ? T(0.125) : T(-0.125), gz, v);
+          T* pr = F.sol + ((size_t)k * F.ny + j) * F.nx + 2 * I + o;
+          *pr = ldc<kCg>(pr) + v;
+        }
+      return;
+    }
+  }
   T mx = T(0), my = T(0), mz = T(0);
   if (F.fx == 2)
     mx = T(0.5) * ((I < C.nx - 1 ? ldc<kCg>(e + cq + 1) : ec) - (I > 0 ? ldc<kCg>(e + cq - 1) : ec));
@@ -305,14 +352,7 @@ __device__ __forceinline__ void prolong_cell(const LevelView<T>& F, const LevelV
       T* row = F.sol + ((size_t)k * F.ny + j) * F.nx;
       const T ty = dy ? T(0.25) * my : -(T(0.25) * my);
       const T tz = dz ? T(0.25) * mz : -(T(0.25) * mz);
-      if (F.fx == 2 && live >= 0) {
-        const int o = (j + k + live) & 1;  // the live child: x = 2I + o
-        T v = ec + (o ? T(0.25) * mx : -(T(0.25) * mx));
-        if (F.fy == 2) v += ty;
-        if (F.fz == 2) v += tz;
-        T* pr = row + 2 * I + o;
-        *pr = ldc<kCg>(pr) + v;
-      } else if (F.fx == 2) {
+      if (F.fx == 2) {
         T v0 = ec + -(T(0.25) * mx), v1 = ec + T(0.25) * mx;
         if (F.fy == 2) { v0 += ty; v1 += ty; }
         if (F.fz == 2) { v0 += tz; v1 += tz; }
