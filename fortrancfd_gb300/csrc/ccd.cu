@@ -19,7 +19,7 @@
 //
 // A sweep is a chain of dependent operations, so what bounds it depends on the
 // number of lines.  Where they fill the GPU it is the FP64 pipe, and part of
-// the work runs on the integer pipes (k_ccd_lines: 21 FP64 operations per point
+// the work runs on the integer pipes (k_ccd_lines: 19 FP64 operations per point
 // for 53); where they do not (2D) it is the chain of one warp, which
 // k_ccd_lines4 shortens by giving a line four lanes.
 // k_ccd_bc fills the ghost layers by zero-gradient copies (bc), k_curvature
@@ -102,11 +102,15 @@ __device__ __forceinline__ void ccd_end(const CcdArgs& c, double f0, double f1, 
 }
 
 // Many lines: one line per thread, bound by the arithmetic pipes.  The back
-// substitution keeps its products in FP64: with the forward sweep's and all
-// quotients on the integer pipes the two kinds of pipe take about as long
-// (curvature of 192x128x256 cells 5.43 ms before, now 2.74; 3.04 with every
-// product on the integer pipes, 3.30 with none; 256^3 6.50, 6.45, 7.21).
-__global__ void __launch_bounds__(128) k_ccd_lines(CcdBatch batch) {
+// substitution keeps six of its eight products in FP64: with the forward sweep's,
+// the other two and all quotients on the integer pipes the two kinds of pipe take
+// about as long (curvature of 192x128x256 cells 5.43 ms before, now 2.32; 2.39 with
+// all eight in FP64, 2.82 with none).  Blocks of one warp, 28 to an SM: a block
+// lasts a whole line, and with 128 threads the last blocks left the SMs half idle
+// (2.47 ms).
+constexpr int kCcdThreads = 32;  // lines of a block
+
+__global__ void __launch_bounds__(kCcdThreads, 28) k_ccd_lines(CcdBatch batch) {
   const int pass = blockIdx.y;
   const CcdArgs& c = batch.c[pass];
   const double* __restrict__ table = batch.table[pass];
@@ -185,8 +189,8 @@ __global__ void __launch_bounds__(128) k_ccd_lines(CcdBatch batch) {
       const int i = i0 - u;
       if (i < 0) break;
       const double* t = table + (size_t)i * kCcdRec;
-      const double si = cs[u] - (__dmul_rn(__ldg(t + 4), sol) + __dmul_rn(__ldg(t + 5), sol2));
-      const double ssi = css[u] - (__dmul_rn(__ldg(t + 6), sol) + __dmul_rn(__ldg(t + 7), sol2));
+      const double si = cs[u] - (__dmul_rn(__ldg(t + 4), sol) + mul_int(__ldg(t + 5), sol2));
+      const double ssi = css[u] - (__dmul_rn(__ldg(t + 6), sol) + mul_int(__ldg(t + 7), sol2));
       sol = -ccd_det_int(t, __dmul_rn(__ldg(t + 9), ssi) - __dmul_rn(__ldg(t + 11), si));
       sol2 = ccd_det_int(t, __dmul_rn(__ldg(t + 8), ssi) - __dmul_rn(__ldg(t + 10), si));
       Sl[(int64_t)i * st] = sol;
@@ -544,7 +548,8 @@ void launch_ccd_lines(cudaStream_t s, const CcdBatch& b) {
     all += b.c[i].n1 * b.c[i].n2;
   }
   if (all >= kCcdManyLines)
-    k_ccd_lines<<<dim3((unsigned)((lines + 127) / 128), (unsigned)b.n), 128, 0, s>>>(b);
+    k_ccd_lines<<<dim3((unsigned)((lines + kCcdThreads - 1) / kCcdThreads), (unsigned)b.n),
+                  kCcdThreads, 0, s>>>(b);
   else  // one warp per block: the few warps spread over the SMs
     k_ccd_lines4<<<dim3((unsigned)((lines + 7) / 8), (unsigned)b.n), 32, 0, s>>>(b);
 }
