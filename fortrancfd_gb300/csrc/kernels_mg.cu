@@ -16,6 +16,7 @@
 #include "gbmg_internal.h"
 #include "idiv.h"
 #include "mg_cells.cuh"
+#include "pairs.cuh"
 #include "pdl.cuh"
 #include "reduce.cuh"
 
@@ -104,22 +105,29 @@ __global__ void __launch_bounds__(256) k_diag(LevelView<double> L, double* diag)
 // q = A d and (kDot) sum d.q (the Krylov matrix product): a warp per 128 cells
 // of a row, the diagonal read back instead of summed, 8 FP64 operations per
 // cell for 13 (bound by the FP64 pipe: 512^3, 3.5 ms before; a warp per whole
-// row left 1024^2 with 7 warps per SM)
+// row left 1024^2 with 7 warps per SM).  Rows by products with reciprocals, as an
+// integer division's conversions run on that pipe, and as many blocks as are
+// resident at once, with the registers for more loads in flight: with 8 per SM,
+// of which 5 fit, the last round left a third of the SM idle (512^3 2.31 -> 1.84
+// ms with 4 per SM, 1.91 with 6; 1024^2 without the sum 20.6 -> 17.2 us with 6,
+// 18.7 with 4).
 constexpr int kApplySeg = 128;
+template <bool kDot>
+constexpr int kApplyBlocks = kDot ? 4 : 6;  // per SM
 
 template <bool kDot>
-__global__ void __launch_bounds__(kRedThreads)
+__global__ void __launch_bounds__(kRedThreads, kApplyBlocks<kDot>)
     k_apply_diag(LevelView<double> L, const double* __restrict__ diag,
-                 const double* __restrict__ dvec, double* __restrict__ qvec, ReduceScratch R,
-                 int slot, int keep_rz) {
+                 const double* __restrict__ dvec, double* __restrict__ qvec, int segs,
+                 unsigned long long rsegs, unsigned long long rny, ReduceScratch R, int slot,
+                 int keep_rz) {
   double acc[1] = {0.0};
-  const int segs = (L.nx + kApplySeg - 1) / kApplySeg;
   const int items = L.ny * L.nz * segs;
   const int lane = threadIdx.x & 31, warps = kRedThreads / 32;
   const size_t sy = (size_t)L.nx, sz = (size_t)L.nx * L.ny;
   for (int it = blockIdx.x * warps + (threadIdx.x >> 5); it < items; it += gridDim.x * warps) {
-    const int row = it / segs, i0 = (it - row * segs) * kApplySeg;
-    const int j = row % L.ny, k = row / L.ny;
+    const int row = (int)div_by((unsigned long long)it, rsegs), i0 = (it - row * segs) * kApplySeg;
+    const int k = (int)div_by((unsigned long long)row, rny), j = row - k * L.ny;
     for (int i = i0 + lane; i < min(L.nx, i0 + kApplySeg); i += 32) {
       const size_t q = ((size_t)k * L.ny + j) * L.nx + i;
       double s = 0.0;
@@ -498,10 +506,16 @@ void launch_diag(cudaStream_t s, const LevelView<double>& L, double* diag) {
 void launch_apply_diag(cudaStream_t s, const LevelView<double>& L, const double* diag,
                        const double* d, double* q, const ReduceScratch& R, int slot,
                        bool keep_rz) {
-  const size_t items = (size_t)L.ny * L.nz * cdiv((size_t)L.nx, kApplySeg);
-  const int blocks = std::min(reduce_blocks_for(items * 32), R.max_blocks);
-  if (slot < 0) k_apply_diag<false><<<blocks, kRedThreads, 0, s>>>(L, diag, d, q, R, slot, 0);
-  else k_apply_diag<true><<<blocks, kRedThreads, 0, s>>>(L, diag, d, q, R, slot, keep_rz ? 1 : 0);
+  const int segs = (int)cdiv((size_t)L.nx, kApplySeg);
+  const size_t items = (size_t)L.ny * L.nz * segs;
+  const int most = 152 * (slot < 0 ? kApplyBlocks<false> : kApplyBlocks<true>);
+  const int blocks = std::min({reduce_blocks_for(items * 32), most, R.max_blocks});
+  const unsigned long long rsegs = div_rcp(segs), rny = div_rcp(L.ny);
+  if (slot < 0)
+    k_apply_diag<false><<<blocks, kRedThreads, 0, s>>>(L, diag, d, q, segs, rsegs, rny, R, slot, 0);
+  else
+    k_apply_diag<true><<<blocks, kRedThreads, 0, s>>>(L, diag, d, q, segs, rsegs, rny, R, slot,
+                                                      keep_rz ? 1 : 0);
 }
 
 template <typename T>

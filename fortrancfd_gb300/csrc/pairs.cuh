@@ -75,12 +75,15 @@ __device__ __forceinline__ void store_pair32(float* out, size_t m, double a, dou
   }
 }
 
+// the factor of div_by for a divisor
+inline unsigned long long div_rcp(int d) { return d == 1 ? 0ull : ~0ull / (unsigned)d + 1; }
+
 inline PairRows pair_rows(int nx, int ny) {
   PairRows P{};
   P.hx = (unsigned)std::max(nx / 2, 1);
   P.ny = (unsigned)ny;
-  P.rx = P.hx == 1 ? 0ull : ~0ull / P.hx + 1;
-  P.ry = P.ny == 1 ? 0ull : ~0ull / P.ny + 1;
+  P.rx = div_rcp((int)P.hx);
+  P.ry = div_rcp(ny);
   return P;
 }
 
