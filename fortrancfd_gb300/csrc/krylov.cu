@@ -31,6 +31,12 @@ namespace {
 
 constexpr int kGmThreads = 256, kGmWarps = kGmThreads / 32;
 constexpr int kGmVals = 32;  // sums of one launch
+// Blocks of the products and of the update that are resident on an SM, and all
+// that are launched (1024 blocks took two to four rounds, the last one part
+// empty: BEFORE).
+template <int G>
+constexpr int kDotsBlocks = G <= 4 ? 3 : 2;
+constexpr int kUpdateBlocks = 4;
 
 // sums of the lanes' a[0..NV-1]: sum v in a[0] of the lanes v * 32/NV and up
 template <int NV, int kOff = 16>
@@ -77,7 +83,7 @@ __device__ __forceinline__ bool gm_runs(const double* first) {
 
 // partials of V_i.w, i < cnt, and of w.w as the one after; 4 (G - 1) <= cnt < 4 G
 template <int G>
-__global__ void __launch_bounds__(kGmThreads, G <= 4 ? 3 : 2)
+__global__ void __launch_bounds__(kGmThreads, kDotsBlocks<G>)
     k_gm_dots(const double* __restrict__ V, size_t ld, int cnt, const double* __restrict__ w,
               size_t n, double* __restrict__ partials, const double* first) {
   pdl_enter();
@@ -156,7 +162,7 @@ __global__ void __launch_bounds__(kGmThreads) k_gm_finish(const double* __restri
 // than 0.7 of the length sqrt(*before) ("twice is enough"): a second pass that is
 // not needed takes the first one's norms
 template <bool kNorm>
-__global__ void __launch_bounds__(kGmThreads, 4)
+__global__ void __launch_bounds__(kGmThreads, kUpdateBlocks)
     k_gm_update(double* __restrict__ w, const double* __restrict__ V, size_t ld,
                 const double* __restrict__ coef, int cnt, double sign, size_t n, double* partials,
                 unsigned int* counter, double* nrm, const double* before, const double* first) {
@@ -321,28 +327,31 @@ unsigned gm_blocks(size_t items, unsigned most) {
 }  // namespace
 
 namespace {
+// (returns the number of blocks)
 template <int G>
-void dots_groups(cudaStream_t s, unsigned b, const double* V, size_t ld, int cnt, const double* w,
-                 size_t n, double* partials, const double* first) {
+int dots_groups(cudaStream_t s, const double* V, size_t ld, int cnt, const double* w, size_t n,
+                double* partials, const double* first) {
   if constexpr (G > 1)
-    if (cnt < 4 * (G - 1)) return dots_groups<G - 1>(s, b, V, ld, cnt, w, n, partials, first);
+    if (cnt < 4 * (G - 1)) return dots_groups<G - 1>(s, V, ld, cnt, w, n, partials, first);
+  const unsigned b = gm_blocks(n, 152 * kDotsBlocks<G>);
   launch_pdl(k_gm_dots<G>, dim3(b), dim3(kGmThreads), 0, s, V, ld, cnt, w, n, partials, first);
+  return (int)b;
 }
 }  // namespace
 
 void launch_gm_dots(cudaStream_t s, const double* V, size_t ld, int cnt, const double* w, size_t n,
                     double* partials, double* out, const double* first) {
   static_assert(kGmresRestart < kGmVals, "sums of one launch");
-  const unsigned b = gm_blocks(n, kGmresBlocks);
-  dots_groups<kGmVals / 4>(s, b, V, ld, cnt, w, n, partials, first);
+  const int b = dots_groups<kGmVals / 4>(s, V, ld, cnt, w, n, partials, first);
   launch_pdl(k_gm_finish, dim3((unsigned)cnt + 1u), dim3(kGmThreads), 0, s,
-             (const double*)partials, (int)b, out, first);
+             (const double*)partials, b, out, first);
 }
 
 void launch_gm_update(cudaStream_t s, double* w, const double* V, size_t ld, const double* coef,
                       int cnt, double sign, size_t n, double* partials, unsigned int* counter,
                       double* nrm, const double* before, const double* first) {
-  const dim3 b(gm_blocks(n, kGmresBlocks)), t(kGmThreads);
+  static_assert(152 * kUpdateBlocks <= kGmresBlocks && 152 * kDotsBlocks<1> <= kGmresBlocks, "partials");
+  const dim3 b(gm_blocks(n, 152 * kUpdateBlocks)), t(kGmThreads);
   if (nrm)
     launch_pdl(k_gm_update<true>, b, t, 0, s, w, V, ld, coef, cnt, sign, n, partials, counter, nrm, before, first);
   else
