@@ -329,7 +329,7 @@ void launch_apply_diag(cudaStream_t s, const LevelView<double>& L, const double*
 // Flexible GMRES passes (krylov.cu), basis V_i at V + i*ld; partials:
 // kGmresBlocks doubles per sum; counter as ReduceScratch::counter.
 constexpr int kGmresRestart = 30;   // restart length
-constexpr int kGmresBlocks = 1024;  // blocks of the products and the update
+constexpr int kGmresBlocks = 1024;  // blocks of the products and the update at most
 // the sum of z
 void launch_gm_sum(cudaStream_t s, const PcgVec& z, const ReduceScratch& R, int slot);
 // out[i] = V_i.w for i < cnt, out[cnt] = w.w.  first: null in a first Gram-Schmidt
