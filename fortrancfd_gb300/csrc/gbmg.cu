@@ -1307,6 +1307,8 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
       if (status == GBMG_OK && !(rel < rtol)) {
         status = std::isfinite(rel) ? GBMG_NOT_CONVERGED : GBMG_DIVERGED;
         if (status == GBMG_NOT_CONVERGED && cyc < h->prm.max_cycles) continue;
+      } else if (status == GBMG_NOT_CONVERGED && rel < rtol) {
+        status = GBMG_OK;  // at the cycle limit the recursion ended just above the tolerance
       }
     }
     // mean projection of p (compatibility_sol on the finest level)
