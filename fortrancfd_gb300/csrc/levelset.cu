@@ -33,6 +33,7 @@
 // before) and runs at 59% of the FP64 pipe and 46% of the issue slots: the
 // integer work that replaced the rest now takes about as long.
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <string>
@@ -845,7 +846,10 @@ int gbmg_ls_redistance(gbmg_ls* ls, gbmg_field phi, double ls_wid, double rdt, d
   int rc;
   if ((rc = ls_in(ls, phi, mem, ls->phi)) != GBMG_OK) return rc;
   // level_set_redis_init (+ level_set_redis_stable for btn = 0)
-  const LsWidth wid = ls_width(ls_wid);
+  // (a ratio so large, or a width so small, that lam's other factors or a quotient
+  // of the sums overflow makes lam * 0 a NaN: the formula decides in every cell)
+  LsWidth wid = ls_width(ls_wid);
+  if (std::fabs(rho_12) >= 0x1p200 || ls_wid < 0x1p-200) wid.out = 0x7fffffffffffffffll;
   LS_CUDA(ls, cudaMemsetAsync(ls->red + 1, 0, sizeof(unsigned long long), ls->stream));
   k_ls_sign<<<nb, 256, 0, ls->stream>>>(n, ls->phi, wid, btn, s);
   ls->launches += 1;
