@@ -174,6 +174,9 @@ void launch_prolong(cudaStream_t s, const LevelView<T>& F, const LevelView<T>& C
 template <typename TO>
 void launch_residual_norm(cudaStream_t s, const LevelView<double>& L, TO* r,
                           const ReduceScratch& R, int slot);
+// (src - A sol - rec)^2 summed over some of the rows into slot; returns their share
+double launch_residual_stray(cudaStream_t s, const LevelView<double>& L, const double* rec,
+                             const ReduceScratch& R, int slot);
 template <typename T>
 void launch_coarse_solve(cudaStream_t s, int n, const T* minv, const T* adense, const T* b, T* x);
 // work: 2 n^2 + n doubles of scratch (n = cells of the coarsest level)

@@ -8,8 +8,8 @@
 //   k_pcg_step       p += alpha d, r -= alpha q, |r|^2, and r rounded to float
 //                    for the next FP32 V-cycle
 // The residual follows the recursion and the solve loop restates it as
-// b - A p in FP64 before it accepts a solution (a tolerance near the FP64 floor
-// recomputes it every iteration: k_pcg_x, then the residual kernel).
+// b - A p in FP64 before it accepts a solution (near the accuracy that FP64
+// allows it is recomputed every iteration: k_pcg_x, then the residual kernel).
 // Recomputing it always, with one pass per vector operation, read and wrote
 // 208 bytes and issued 37 FP64 operations per cell and iteration: 10.6 of the 13.7
 // ms of a 512^3 iteration.  These passes move 152 bytes with 16 operations
