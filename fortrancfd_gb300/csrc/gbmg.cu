@@ -315,11 +315,18 @@ void enqueue_defect(gbmg_handle* h, int pc, const float* e, float* r32, int slot
   }
 }
 
+void free_spare(gbmg_handle* h) {
+  if (h->kdiag == h->lv[0].diag) h->kdiag = nullptr;
+  for (int l = 0; l < h->L; ++l) dfree(h->lv[l].diag);
+}
+
 int free_all(gbmg_handle* h) {
   reset_graphs(h);
+  free_spare(h);
+  dfree(h->kdiag);
   for (int l = 0; l < h->L; ++l) {
     Level& v = h->lv[l];
-    dfree(v.cx); dfree(v.cy); dfree(v.cz); dfree(v.idiag); dfree(v.diag);
+    dfree(v.cx); dfree(v.cy); dfree(v.cz); dfree(v.idiag);
     if (l > 0) { dfree(v.sol); dfree(v.src); }
     dfree(v.cx32); dfree(v.cy32); dfree(v.cz32); dfree(v.sol32); dfree(v.src32);
     dfree(v.alt); dfree(v.alt32);
@@ -328,7 +335,7 @@ int free_all(gbmg_handle* h) {
   dfree(h->pw[0]); dfree(h->pw[1]); dfree(h->bw); dfree(h->cxw); dfree(h->cyw); dfree(h->czw);
   for (int a = 0; a < 3; ++a) dfree(h->vel[a]);
   dfree(h->aux[0]); dfree(h->aux[1]); dfree(h->r0);
-  dfree(h->kdiag); dfree(h->kr); dfree(h->kz); dfree(h->kzold); dfree(h->kd); dfree(h->kq);
+  dfree(h->kr); dfree(h->kz); dfree(h->kzold); dfree(h->kd); dfree(h->kq);
   dfree(h->gmV); dfree(h->gmZ); dfree(h->gmPart); dfree(h->gmDev);
   if (h->gmHost) cudaFreeHost(h->gmHost);
   if (h->gmEv) cudaEventDestroy(h->gmEv);
@@ -474,7 +481,6 @@ int allocate(gbmg_handle* h) {
   // the FP64 increment rule keeps the previous cycle's p
   if (h->prm.stop_rule == GBMG_STOP_INCREMENT && !h->mixed) GB_TRY(dmalloc(h, &h->r0, h->n0));
   if (h->prm.krylov) {
-    GB_TRY(dmalloc(h, &h->kdiag, h->n0));
     GB_TRY(dmalloc(h, &h->kr, h->n0));
     if (!h->mixed) GB_TRY(dmalloc(h, &h->kz, h->n0));
     GB_TRY(dmalloc(h, &h->kzold, h->n0));
@@ -517,10 +523,13 @@ int allocate(gbmg_handle* h) {
   if (h->mixed) setup_subcycle<float>(h);
   else setup_subcycle<double>(h);
   GB_TRY(setup_tiles(h));
-  // the restriction of the FP64 levels reads their diagonal
+  // the restriction of the FP64 levels reads their diagonal and the Krylov matrix
+  // product the finest level's, or sum the coefficients where there is none
   if (!h->mixed)
     for (int l = 0; l < std::min(h->sub_lc, L - 1); ++l)
-      if (!h->lv[l].tile) GB_TRY(dmalloc(h, &h->lv[l].diag, h->lv[l].n));
+      if (!h->lv[l].tile) dmalloc_spare(h, &h->lv[l].diag, h->lv[l].n);
+  h->kdiag = h->prm.krylov ? h->lv[0].diag : nullptr;
+  if (h->prm.krylov && !h->kdiag) dmalloc_spare(h, &h->kdiag, h->n0);
   GB_CUDA(h, cudaEventCreate(&h->ev0));
   GB_CUDA(h, cudaStreamCreateWithFlags(&h->cstream, cudaStreamNonBlocking));
   for (int i = 0; i < 5; ++i) GB_CUDA(h, cudaEventCreateWithFlags(&h->cev[i], cudaEventDisableTiming));
@@ -553,7 +562,8 @@ int build_hierarchy(gbmg_handle* h) {
   }
   LAUNCH(h, GBMG_PROF_SETUP,
          launch_coarse_invert(s, v64(h->lv[h->L - 1]), h->minv, h->adense, h->minv32, h->adense32, h->cwork));
-  if (h->kdiag) LAUNCH(h, GBMG_PROF_SETUP, launch_diag(s, v64(h->lv[0]), h->kdiag));
+  if (h->kdiag && h->kdiag != h->lv[0].diag)
+    LAUNCH(h, GBMG_PROF_SETUP, launch_diag(s, v64(h->lv[0]), h->kdiag));
   if (h->mixed && !h->fine_copies) {
     const Level& f = h->lv[0];
     LAUNCH(h, GBMG_PROF_SETUP, launch_to_dw(s, f.cx, h->cxw, f.n));
@@ -1487,6 +1497,17 @@ int zero_walls(gbmg_handle* h, const gbmg_field dfield[3], bool has_w) {
 
 namespace gbmg {
 namespace host {
+
+// (between the launches of a call: captured graphs go, as they hold the arrays)
+bool release_spare(gbmg_handle* h) {
+  bool any = false;
+  for (int l = 0; l < h->L; ++l) any = any || h->lv[l].diag;
+  if (!any || cudaStreamSynchronize(h->stream) != cudaSuccess) return false;
+  reset_graphs(h);
+  free_spare(h);
+  return true;
+}
+
 
 // The projection on device face velocities (fields addressed at their face
 // (0,0,0)) with the initial pressure already in h->p: b = div(u*)/dt, the

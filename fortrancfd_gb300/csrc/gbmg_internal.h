@@ -324,7 +324,7 @@ void launch_pcg_x(cudaStream_t s, double* x, const double* d, size_t n,
 // x += alpha d, r -= alpha q, |r|^2; r32 (may be null): r rounded to float, in z's layout
 void launch_pcg_step(cudaStream_t s, double* x, const double* d, double* r, const double* q,
                      float* r32, const PcgVec& z, const ReduceScratch& R);
-// sum of the face coefficients of each cell, and q = A d with it, d.q into
+// sum of the face coefficients of each cell, and q = A d with it (null: summed), d.q into
 // slot (none when slot < 0); keep_rz: kSlotDot2+1 <- kSlotDot (kernels_mg.cu)
 void launch_diag(cudaStream_t s, const LevelView<double>& L, double* diag);
 void launch_apply_diag(cudaStream_t s, const LevelView<double>& L, const double* diag,

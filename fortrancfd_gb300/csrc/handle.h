@@ -63,7 +63,9 @@ struct gbmg_handle {
   // flexible CG recomputes b - A p every iteration (tight tolerances) instead
   // of following the recursion
   bool pcg_true = false;
-  double* kdiag = nullptr;  // sum of the finest level's face coefficients per cell
+  // sum of the finest level's face coefficients per cell: that level's own array where
+  // it has one, none where memory is short
+  double* kdiag = nullptr;
   // flexible GMRES (krylov = 2): basis V (restart + 1 vectors), preconditioned
   // vectors Z (restart), dot partials, device and pinned host coefficients
   // gmLd: stride of V and Z (n0 rounded up to even); gmEv: the step's coefficients copied
@@ -217,11 +219,32 @@ inline void prof_end(gbmg_handle* h, int cls) {
     prof_end(h, cls);        \
   } while (0)
 
+// Frees the arrays that the handle can do without; true if there were any (gbmg.cu).
+bool release_spare(gbmg_handle* h);
+
 template <typename T>
 inline int dmalloc(gbmg_handle* h, T** ptr, size_t n) {
   *ptr = nullptr;
-  GB_CUDA(h, cudaMalloc((void**)ptr, (n ? n : 1) * sizeof(T)));
+  const size_t bytes = (n ? n : 1) * sizeof(T);
+  cudaError_t e = cudaMalloc((void**)ptr, bytes);
+  if (e == cudaErrorMemoryAllocation && release_spare(h)) {
+    cudaGetLastError();
+    e = cudaMalloc((void**)ptr, bytes);
+  }
+  GB_CUDA(h, e);
   return GBMG_OK;
+}
+
+// An array that the handle can do without, where it is a small part of what is
+// free (an eighth: what the caller allocates beside the handle still fits).
+inline void dmalloc_spare(gbmg_handle* h, double** ptr, size_t n) {
+  size_t free_bytes = 0, total = 0;
+  *ptr = nullptr;
+  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || 8 * n * sizeof(double) > free_bytes ||
+      cudaMalloc((void**)ptr, n * sizeof(double)) != cudaSuccess) {
+    *ptr = nullptr;
+    cudaGetLastError();
+  }
 }
 
 template <typename T>

@@ -134,7 +134,8 @@ constexpr int kApplySeg = 128;
 template <bool kDot>
 constexpr int kApplyBlocks = kDot ? 4 : 6;  // per SM
 
-template <bool kDot>
+// (kStored false: no diagonal, where memory is short: summed, with the same bits)
+template <bool kDot, bool kStored>
 __global__ void __launch_bounds__(kRedThreads, kApplyBlocks<kDot>)
     k_apply_diag(LevelView<double> L, const double* __restrict__ diag,
                  const double* __restrict__ dvec, double* __restrict__ qvec, int segs,
@@ -149,14 +150,19 @@ __global__ void __launch_bounds__(kRedThreads, kApplyBlocks<kDot>)
     const int k = (int)div_by((unsigned long long)row, rny), j = row - k * L.ny;
     for (int i = i0 + lane; i < min(L.nx, i0 + kApplySeg); i += 32) {
       const size_t q = ((size_t)k * L.ny + j) * L.nx + i;
-      double s = 0.0;
-      if (i > 0) s += L.cx[q] * dvec[q - 1];
-      if (i < L.nx - 1) s += L.cx[q + 1] * dvec[q + 1];
-      if (j > 0) s += L.cy[q] * dvec[q - sy];
-      if (j < L.ny - 1) s += L.cy[q + sy] * dvec[q + sy];
-      if (k > 0) s += L.cz[q] * dvec[q - sz];
-      if (k < L.nz - 1) s += L.cz[q + sz] * dvec[q + sz];
-      const double a = s - diag[q] * dvec[q];
+      double s = 0.0, d = 0.0;
+      if constexpr (kStored) {
+        d = diag[q];
+        if (i > 0) s += L.cx[q] * dvec[q - 1];
+        if (i < L.nx - 1) s += L.cx[q + 1] * dvec[q + 1];
+        if (j > 0) s += L.cy[q] * dvec[q - sy];
+        if (j < L.ny - 1) s += L.cy[q + sy] * dvec[q + sy];
+        if (k > 0) s += L.cz[q] * dvec[q - sz];
+        if (k < L.nz - 1) s += L.cz[q + sz] * dvec[q + sz];
+      } else {
+        stencil(L, dvec, i, j, k, q, s, d);
+      }
+      const double a = s - d * dvec[q];
       qvec[q] = a;
       if (kDot) acc[0] += dvec[q] * a;
     }
@@ -542,11 +548,12 @@ void launch_apply_diag(cudaStream_t s, const LevelView<double>& L, const double*
   const int most = 152 * (slot < 0 ? kApplyBlocks<false> : kApplyBlocks<true>);
   const int blocks = std::min({reduce_blocks_for(items * 32), most, R.max_blocks});
   const unsigned long long rsegs = div_rcp(segs), rny = div_rcp(L.ny);
-  if (slot < 0)
-    k_apply_diag<false><<<blocks, kRedThreads, 0, s>>>(L, diag, d, q, segs, rsegs, rny, R, slot, 0);
-  else
-    k_apply_diag<true><<<blocks, kRedThreads, 0, s>>>(L, diag, d, q, segs, rsegs, rny, R, slot,
-                                                      keep_rz ? 1 : 0);
+  const auto go = [&](auto kernel) {
+    kernel<<<blocks, kRedThreads, 0, s>>>(L, diag, d, q, segs, rsegs, rny, R, slot,
+                                          slot >= 0 && keep_rz ? 1 : 0);
+  };
+  if (slot < 0) diag ? go(k_apply_diag<false, true>) : go(k_apply_diag<false, false>);
+  else diag ? go(k_apply_diag<true, true>) : go(k_apply_diag<true, false>);
 }
 
 template <typename T>
