@@ -1173,9 +1173,12 @@ int finish_mixed(gbmg_handle* h, bool shifted) {
   return check_launch(h, "mean");
 }
 
-// Flexible CG looks at how far its recursion has strayed below this many
-// tolerances, and is steered by b - A p from there on when it is more than this
-// part of the tolerance.
+// Flexible CG steers by b - A p in every iteration on grids of up to kPcgSmall
+// cells; on larger ones by the recursion, restated every kPcgRestate iterations and
+// looked at below kPcgCheck tolerances: where it has strayed by kPcgStray of the
+// tolerance, b - A p steers from there on (solve_internal).
+constexpr size_t kPcgSmall = (size_t)1 << 18;
+constexpr int kPcgRestate = 8;
 constexpr double kPcgCheck = 100.0, kPcgStray = 0.05;
 
 // Restarts of the stationary mixed loop after a failed FP64 certification.
@@ -1195,16 +1198,22 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
   if (h->prm.stop_rule == GBMG_STOP_RMS) tol = tol * std::sqrt((double)n) / scale;
   const double rtol = by_inc ? 0.0 : tol;  // threshold of the residual tests
   bool shifted = false;
-  // Below 1e-11 flexible CG recomputes its residual every iteration.  Above, it
-  // follows the recursion, which strays from b - A p by rounding that grows with
-  // |A||p|.  Near the accuracy that FP64 allows (2D, density ratio 1000, fine grids)
-  // that is as much as the tolerance, and the last iterations, steered by a
-  // residual so far off, go wrong: of 460 solves (512^2 to 4096^2 and 128^3, 1e-9 to
-  // 1.1e-11) 88 took one to ten iterations more, some thirty, than with b - A p in
-  // every iteration.  So the recursion is looked at once, at kPcgCheck tolerances,
-  // and left where it has strayed by kPcgStray of the tolerance (checked at 10
-  // tolerances 22 of the 460 took more); a start below that has no room for it.
-  h->pcg_true = rtol < 1e-11;
+  // Flexible CG and its recursion.  The recursion's residual strays from b - A p by
+  // rounding that grows with |A||p|, by the tolerance and more where that is near
+  // the accuracy that FP64 allows (fine 2D grids with a density ratio of 1000, 3D
+  // ones with 1e5).  Put right only at the end, the jump breaks the conjugacy of the
+  // directions: of 312 such solves (128^2 to 2048^2, 32^3 to 256^3, tolerances 1e-9 to
+  // 1.1e-11) 58 took one to ten iterations more than with b - A p in every
+  // iteration, or did not converge any more.  Restated every eight iterations the
+  // jumps are too small for that, and near the end every iteration's counts (without
+  // that 10 of the 312 differ, even restated every four); together 311 take the
+  // same iterations.  A start below the check has no room for the recursion, nor has
+  // a tolerance below 1e-11.  On small grids an iteration is bound by its launches
+  // and b - A p costs 0 to 7% of it (128^2, 64^3), less than the host's waits for the
+  // restating (64^3 10%); on large ones it costs more (1024^2 13%, 2048^2 25%) and the
+  // restating 5% (512^3 361 -> 381 ms).
+  h->pcg_true = rtol < 1e-11 || n <= kPcgSmall;
+  int restate = kPcgRestate;  // the iteration before which the recursion is restated
   // initial residual
   f.sol = h->p; f.src = h->b;
   if (pcg) {
@@ -1244,6 +1253,11 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
       const bool adapt = kind == kGraphMixed && h->adaptive && !h->stag_mode;
       int next = kind == kGraphMixed ? (h->stag_mode ? 1 : h->inner) : 1;
       while (cyc < h->prm.max_cycles) {
+        const bool recursion = pcg && !h->pcg_true;
+        if (recursion && cyc >= restate) {
+          GB_TRY(pcg_residual(h));
+          restate = cyc + kPcgRestate;
+        }
         // every iteration of full length but the first flexible-CG one: the
         // loop on the device
         if (!(pcg && cyc == 0) && next == (kind == kGraphMixed ? h->inner : 1)) {
@@ -1252,7 +1266,7 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
           c.tol = target;
           c.guard = 1e3 * std::max(1.0, st->res0);
           c.best = best;
-          c.max_cycles = h->prm.max_cycles;
+          c.max_cycles = recursion ? std::min(restate, h->prm.max_cycles) : h->prm.max_cycles;
           c.step = kind == kGraphMixed ? h->inner : 1;
           c.by_inc = by_inc ? 1 : 0;
           c.flat_stop = (kind == kGraphMixed && h->prm.certify) ? 1 : 0;
@@ -1279,6 +1293,7 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
             // ended by a test, by the predicted last correction (run below),
             // or with too few cycles left for a whole iteration (run below)
             if (status != GBMG_NOT_CONVERGED || stalled || cyc >= h->prm.max_cycles) break;
+            if (recursion && cyc >= restate) continue;
             if (c.tail > 0) next = c.tail;
           }
         }

@@ -7,9 +7,10 @@
 //   k_apply_diag     q = A d and d.q
 //   k_pcg_step       p += alpha d, r -= alpha q, |r|^2, and r rounded to float
 //                    for the next FP32 V-cycle
-// The residual follows the recursion and the solve loop restates it as
-// b - A p in FP64 before it accepts a solution (near the accuracy that FP64
-// allows it is recomputed every iteration: k_pcg_x, then the residual kernel).
+// The residual follows the recursion; the solve loop restates it as b - A p in
+// FP64 every few iterations and before it accepts a solution.  On small grids and
+// near the accuracy that FP64 allows it is recomputed every iteration (k_pcg_x,
+// then the residual kernel).
 // Recomputing it always, with one pass per vector operation, read and wrote
 // 208 bytes and issued 37 FP64 operations per cell and iteration: 10.6 of the 13.7
 // ms of a 512^3 iteration.  These passes move 152 bytes with 16 operations
@@ -119,7 +120,8 @@ __global__ void __launch_bounds__(kRedThreads)
           [&](size_t q, double2 v) { x[q] = v.x + alpha * v.y; });
 }
 
-// r32 (K = kZ32, kZSplit): the new residual rounded to float
+// r32 (K = kZ32, kZSplit): the new residual rounded to float.  n is even: an odd grid
+// has no coarser level and at most kMaxCoarse cells, too few for the recursion.
 template <int K>
 __global__ void __launch_bounds__(kRedThreads)
     k_pcg_step(double* x, const double* __restrict__ d, double* r, const double* __restrict__ q,
@@ -148,14 +150,6 @@ __global__ void __launch_bounds__(kRedThreads)
     one(m + step, xb, db, rb, qb);
   }
   if (m < pairs) one(m, x2[m], d2[m], r2[m], q2[m]);
-  if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
-    const size_t e = n - 1;
-    x[e] += alpha * d[e];
-    const double a = r[e] - alpha * q[e];
-    r[e] = a;
-    acc[0] += a * a;
-    if (K != kZ64) r32[e] = (float)a;
-  }
   grid_sum_finish<1>(acc, R, kSlotNorm);
 }
 
