@@ -256,19 +256,44 @@ int enqueue_vcycle(gbmg_handle* h, bool reverse_post, bool zero_fine) {
   return check_launch(h, "v-cycle");
 }
 
-// Algorithmic HBM bytes of one V-cycle (each array touched once per kernel).
-double vcycle_bytes(const gbmg_handle* h, int w) {
+// Algorithmic HBM bytes of one V-cycle (each array touched once per kernel; w
+// bytes per value).  zero_fine as enqueue_vcycle.
+double vcycle_bytes(const gbmg_handle* h, int w, bool zero_fine) {
   double bytes = 0.0;
   const bool idiag = (w == 8);
+  const int top = std::min(h->sub_lc, h->L - 1);
   for (int l = 0; l < h->L - 1; ++l) {
-    const double n = (double)h->lv[l].n, nc = (double)h->lv[l + 1].n;
+    const Level& v = h->lv[l];
+    const double n = (double)v.n, nc = (double)h->lv[l + 1].n;
+    const bool zero = l > 0 || zero_fine;
+    if (l < top && by_tiles(h, l, zero)) {
+      // a launch: p read (not the first from zero) and written, b, the
+      // coefficients (cx, cy, 1/diag; split: rho); coarse b written by the last
+      // launch down, coarse e read by the first one up
+      const int launches = tile_launches(h->prm.nu1) + tile_launches(h->prm.nu2);
+      const double coef = v.split ? 1.0 : (idiag ? 3.0 : 2.0);
+      bytes += (launches * (3.0 + coef) - (zero ? 1.0 : 0.0)) * w * n + 2.0 * w * nc;
+      continue;
+    }
     const double sweep = (idiag ? 7.0 : 6.0) * w * n;  // p r/w, b, cx, cy, cz (+ 1/diag)
     bytes += (h->prm.nu1 + h->prm.nu2) * sweep;
-    bytes += 5.0 * w * n + 2.0 * w * nc;  // restrict: p, b, cx, cy, cz -> coarse b, sol
+    // restrict: p, b, cx, cy, cz (+ diag) -> coarse b, sol
+    bytes += (v.diag ? 6.0 : 5.0) * w * n + 2.0 * w * nc;
     bytes += 2.0 * w * n + w * nc;        // prolong: p r/w, coarse e
   }
   bytes += 2.0 * w * h->nc + (double)w * h->nc * h->nc;
   return bytes;
+}
+
+// The same per cell of the Krylov iterations' kernels on the finest level: the V-cycle's
+// result, the matrix product (cx, cy, cz, d, diag -> q), and b - A p (b, p, cx, cy,
+// cz -> r, and r -> its FP32 copy).
+struct KrylovBytes {
+  double z, product, residual;
+};
+KrylovBytes krylov_bytes(const gbmg_handle* h) {
+  return KrylovBytes{h->mixed ? 4.0 : 8.0, h->kdiag ? 48.0 : 40.0,
+                     h->mixed && h->prm.krylov == 1 ? 60.0 : 48.0};
 }
 
 int reset_graphs(gbmg_handle* h) {
@@ -1007,7 +1032,8 @@ int gm_vcycle(gbmg_handle* h) {
 // step of 1024^2 left it idle for 50 of 345 us with two waits per step).  At each
 // restart and at the end the true FP64 residual b - A p is recomputed.  On entry kr holds r0 = b - A p and host_res[kSlotNorm] its
 // squared norm.
-int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles, int* status) {
+int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles, int* status,
+           double* bytes) {
   const cudaStream_t s = h->stream;
   Level& f = h->lv[0];
   const size_t n = h->n0;
@@ -1026,6 +1052,8 @@ int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles
   double rel = *rel_io, factor = 0.2;  // factor: last reduction of the residual
   int total = 0;
   *status = GBMG_NOT_CONVERGED;
+  const KrylovBytes kb = krylov_bytes(h);
+  double per_cell = 0.0;
   while (total < h->prm.max_cycles) {
     const double beta = std::sqrt(r2);
     if (!(beta > 0.0)) { *status = GBMG_OK; break; }
@@ -1063,6 +1091,10 @@ int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles
       const double hn = std::sqrt(norms[0]);
       if (norms[4] != 0.0)
         for (int i = 0; i <= j; ++i) col[i] += h->gmHost[(m + 2) + i];
+      // sum of z, z_j, w = A z_j; a pass: the basis and w for the products, the basis
+      // and w r/w for the update; v_{j+1} twice from w
+      per_cell += kb.z + (kb.z + 8.0) + kb.product +
+                  (norms[4] != 0.0 ? 2.0 : 1.0) * (16.0 * (j + 1) + 24.0) + (16.0 + kb.z);
       col[j + 1] = hn;
       for (int i = 0; i < j; ++i) {
         const double t = cs[i] * col[i] + sn[i] * col[i + 1];
@@ -1090,6 +1122,7 @@ int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles
       for (int k = i + 1; k < j; ++k) t -= H[(size_t)i * m + k] * y[k];
       y[i] = H[(size_t)i * m + i] != 0.0 ? t / H[(size_t)i * m + i] : 0.0;
     }
+    per_cell += (16.0 + kb.z) + (8.0 * j + 16.0) + kb.residual;  // v_0, p += Z y, b - A p
     std::copy(y.begin(), y.begin() + j, h->gmHost);
     GB_CUDA(h, cudaMemcpyAsync(h->gmDev, h->gmHost, j * sizeof(double), cudaMemcpyHostToDevice, s));
     LAUNCH(h, VC, launch_gm_update(s, h->p, h->gmZ, ld, h->gmDev, j, 1.0, n, nullptr, nullptr, nullptr,
@@ -1105,6 +1138,7 @@ int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles
   }
   *rel_io = rel;
   *cycles = total;
+  *bytes = per_cell * (double)n;
   return GBMG_OK;
 }
 
@@ -1233,6 +1267,9 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
   int status = GBMG_NOT_CONVERGED;
   int cyc = 0;
   double target = tol;  // where flexible CG stops next
+  int rec = 0;          // its iterations by the recursion
+  double krylov = 0.0;  // bytes of the Krylov iterations' kernels but those of every iteration
+  const KrylovBytes kb = krylov_bytes(h);
   if (h->prm.krylov == 1 && !h->pcg_true) {
     if (rel < kPcgCheck * tol) h->pcg_true = true;
     else target = kPcgCheck * tol;
@@ -1240,7 +1277,7 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
   if (rel < rtol || r2 == 0.0) {
     status = GBMG_OK;
   } else if (h->prm.krylov == 2) {
-    GB_TRY(fgmres(h, tol, scale, &rel, &cyc, &status));
+    GB_TRY(fgmres(h, tol, scale, &rel, &cyc, &status, &krylov));
     r2 = rel * scale * rel * scale;
   }
   for (int restart = 0;; ++restart) {
@@ -1256,6 +1293,7 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
         const bool recursion = pcg && !h->pcg_true;
         if (recursion && cyc >= restate) {
           GB_TRY(pcg_residual(h));
+          krylov += kb.residual * n;
           restate = cyc + kPcgRestate;
         }
         // every iteration of full length but the first flexible-CG one: the
@@ -1280,6 +1318,7 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
             if (kind == kGraphMixed) h->pcur ^= c.iters & 1;
             st->device_loop = 1;
             if (c.iters > 0) {
+              if (recursion) rec += c.cyc - cyc;
               cyc = c.cyc;
               r2 = c.r2;
               rel = c.rel;
@@ -1300,6 +1339,7 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
         const int step = kind == kGraphMixed ? std::min(next, h->prm.max_cycles - cyc) : 1;
         const double prev = rel;
         cyc += step;
+        if (recursion) rec += step;
         GB_TRY(run_iteration(h, kind, pcg && cyc == 1, step));
         if (kind == kGraphMixed) h->pcur ^= 1;
         GB_CUDA(h, cudaStreamSynchronize(s));
@@ -1356,6 +1396,7 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
         target = tol;
         double d2 = 0.0;
         GB_TRY(pcg_strayed(h, &d2));
+        krylov += (kb.residual + 8.0) / 17.0 * n;
         if (std::sqrt(d2) / scale <= kPcgStray * tol) continue;
         h->pcg_true = true;
       }
@@ -1363,6 +1404,7 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
       // tolerance (also where, at the cycle limit, the recursion ended just above
       // it), else the iteration goes on from it
       GB_TRY(pcg_residual(h));
+      krylov += kb.residual * n;
       GB_TRY(read_result(h, kSlotNorm, &r2));
       rel = std::sqrt(r2) / scale;
       if (status != GBMG_DIVERGED && rel < rtol) {
@@ -1454,17 +1496,25 @@ int solve_internal(gbmg_handle* h, double tol, double bnorm, gbmg_stats* st) {
   st->coarse_n = h->nc;
   st->rel_residual = rel;
   st->rms_residual = std::sqrt(r2 / (double)n);
-  // algorithmic bytes per cycle: the V-cycle, plus the residual of each
-  // iteration (FP64: p, b, cx, cy, cz; or the defect with its e read, p write,
-  // r32 write and zeroed e)
+  // algorithmic bytes: the V-cycles, the kernels of the loop, the first residual and
+  // the mean projection
   const int w = h->mixed ? 4 : 8;
-  double per = vcycle_bytes(h, w);
-  if (kind == kGraphMixed) per += (40.0 * n + 16.0 * n + 4.0 * n) / h->inner;
-  else if (h->prm.krylov == 1) per += (h->mixed ? 156.0 : 160.0) * n;  // pcg.cu's passes
-  else per += 40.0 * n + (h->mixed ? 20.0 * n : 0.0);
-  if (h->prm.krylov == 2)
-    per += (h->mixed ? 24.0 : 8.0) * n + 16.0 * n + 32.0 * n + 48.0 * n + 24.0 * n + 8.0 * n;
-  st->bytes = per * cyc + 40.0 * n + 32.0 * n;
+  double bytes = vcycle_bytes(h, w, kind != kGraphFp64 && h->prm.nu1 > 0) * cyc;
+  if (h->prm.krylov == 2) {
+    bytes += krylov + kb.residual * n;
+  } else if (pcg) {
+    // sum of z; z - mean, r.z and r.z_old; d; A d; then p and r by the recursion
+    // (with its FP32 copy), or p and b - A p
+    const double each = kb.z + (kb.z + 24.0) + 24.0 + kb.product;
+    bytes += (each * cyc + (h->mixed ? 52.0 : 48.0) * rec + (24.0 + kb.residual) * (cyc - rec)) * n;
+    bytes += krylov + kb.residual * n;
+  } else if (kind == kGraphMixed) {
+    // the defect: p, b, cx, cy, cz and e read, p and r32 written
+    bytes += (40.0 * n + 16.0 * n + 4.0 * n) / h->inner * cyc + 40.0 * n;
+  } else {
+    bytes += 40.0 * n * cyc + 40.0 * n;  // b - A p: p, b, cx, cy, cz
+  }
+  st->bytes = bytes + 32.0 * n;
   return status;
 }
 
