@@ -712,6 +712,14 @@ int read_result(gbmg_handle* h, int slot, double* v) {
   return GBMG_OK;
 }
 
+// The finest FP32 unknown to zero (both colour halves where it is split).
+int zero_fine32(gbmg_handle* h) {
+  const Level& f = h->lv[0];
+  const size_t n = f.split ? f.n / 2 + f.hstride : f.n;
+  GB_CUDA(h, cudaMemsetAsync(f.sol32, 0, n * sizeof(float), h->stream));
+  return GBMG_OK;
+}
+
 // kr = b - A p in FP64 and its norm (flexible CG: at the start, and where the
 // recursion's residual is about to be believed), with the FP32 copy that the
 // next mixed iteration's V-cycle reads.
@@ -768,7 +776,7 @@ int enqueue_iteration(gbmg_handle* h, int kind, bool first, bool to_host = true,
   } else if (kind == kGraphMixed) {
     // e = V-cycles(r) in FP32 (the first from zero, the others continuing
     // from e); p += e and r = b - A p in double-word
-    if (!zg) GB_CUDA(h, cudaMemsetAsync(f.sol32, 0, n * sizeof(float), s));
+    if (!zg) GB_TRY(zero_fine32(h));
     GB_TRY(enqueue_vcycle<float>(h, false, zg));
     for (int c = 1; c < cycles; ++c) GB_TRY(enqueue_vcycle<float>(h, false, false));
     // the increment rule: the cycle's correction e is p_k - p_(k-1)
@@ -784,7 +792,7 @@ int enqueue_iteration(gbmg_handle* h, int kind, bool first, bool to_host = true,
       GB_TRY(enqueue_vcycle<double>(h, true, zg));
     } else {
       // (src32 holds r: pcg_residual or the last iteration's step wrote it)
-      if (!zg) GB_CUDA(h, cudaMemsetAsync(f.sol32, 0, (f.split ? n / 2 + f.hstride : n) * sizeof(float), s));
+      if (!zg) GB_TRY(zero_fine32(h));
       GB_TRY(enqueue_vcycle<float>(h, true, zg));
     }
     const bool z64 = kind == kGraphPcg64;
@@ -984,8 +992,7 @@ int gm_vcycle(gbmg_handle* h) {
       f.sol = h->p; f.src = h->b;
       GB_TRY(rc);
     } else {
-      if (!zg)
-        GB_CUDA(h, cudaMemsetAsync(f.sol32, 0, (f.split ? h->n0 / 2 + f.hstride : h->n0) * sizeof(float), s));
+      if (!zg) GB_TRY(zero_fine32(h));
       GB_TRY(enqueue_vcycle<float>(h, true, zg));
     }
     LAUNCH(h, GBMG_PROF_VECTOR, launch_gm_sum(s, gm_vec(h), h->red, kSlotSum));
