@@ -127,16 +127,17 @@ __global__ void __launch_bounds__(256) k_diag(LevelView<double> L, double* diag)
 // row left 1024^2 with 7 warps per SM).  Rows by products with reciprocals, as an
 // integer division's conversions run on that pipe, and as many blocks as are
 // resident at once, with the registers for more loads in flight: with 8 per SM,
-// of which 5 fit, the last round left a third of the SM idle (512^3 2.31 -> 1.84
-// ms with 4 per SM, 1.91 with 6; 1024^2 without the sum 20.6 -> 17.2 us with 6,
-// 18.7 with 4).
+// of which 5 fit, the last round left a third of the SM idle.  Four per SM, against
+// six: with the sum 64^3 10.5 for 12.9 us, 128^3 36.4 for 43.2, 1024^2 24.8 for 25.9,
+// 4096^2 255 for 267, 512^3 1839 for 1838 (384^3 785 for 772); without 64^3 5.7 for
+// 6.4, 128^3 28.8 for 31.2, 2048^2 58.9 for 64.4, 256^3 204 for 225, 512^3 1604 for
+// 1709 (1024^2 18.4 for 17.9).
 constexpr int kApplySeg = 128;
-template <bool kDot>
-constexpr int kApplyBlocks = kDot ? 4 : 6;  // per SM
+constexpr int kApplyBlocks = 4;  // per SM
 
 // (kStored false: no diagonal, where memory is short: summed, with the same bits)
 template <bool kDot, bool kStored>
-__global__ void __launch_bounds__(kRedThreads, kApplyBlocks<kDot>)
+__global__ void __launch_bounds__(kRedThreads, kApplyBlocks)
     k_apply_diag(LevelView<double> L, const double* __restrict__ diag,
                  const double* __restrict__ dvec, double* __restrict__ qvec, int segs,
                  unsigned long long rsegs, unsigned long long rny, ReduceScratch R, int slot,
@@ -545,7 +546,7 @@ void launch_apply_diag(cudaStream_t s, const LevelView<double>& L, const double*
                        bool keep_rz) {
   const int segs = (int)cdiv((size_t)L.nx, kApplySeg);
   const size_t items = (size_t)L.ny * L.nz * segs;
-  const int most = 152 * (slot < 0 ? kApplyBlocks<false> : kApplyBlocks<true>);
+  const int most = 152 * kApplyBlocks;
   const int blocks = std::min({reduce_blocks_for(items * 32), most, R.max_blocks});
   const unsigned long long rsegs = div_rcp(segs), rny = div_rcp(L.ny);
   const auto go = [&](auto kernel) {
