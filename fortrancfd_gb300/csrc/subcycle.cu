@@ -518,7 +518,7 @@ __device__ void subcycle_body(const SubCycle<T>& S, T* base) {
 template <typename T>
 __global__ void __launch_bounds__(kSubThreads, 1) k_subcycle(SubCycle<T> S) {
   pdl_launch();
-  extern __shared__ unsigned char sub_raw[];
+  extern __shared__ __align__(16) unsigned char sub_raw[];
   subcycle_body(S, reinterpret_cast<T*>(sub_raw));
 }
 
