@@ -40,23 +40,11 @@ __device__ __forceinline__ dw dw_add(dw a, dw b) {
 
 __device__ __forceinline__ dw dw_neg(dw a) { return dw{-a.hi, -a.lo}; }
 
-__device__ __forceinline__ dw dw_sub(dw a, dw b) { return dw_add(a, dw_neg(b)); }
-
 __device__ __forceinline__ dw dw_add_f(dw a, float b) {
   dw s = two_sum(a.hi, b);
   s.lo += a.lo;
   return fast_two_sum(s.hi, s.lo);
 }
-
-__device__ __forceinline__ dw dw_mul(dw a, dw b) {
-  const float p = a.hi * b.hi;
-  float e = fmaf(a.hi, b.hi, -p);
-  e = fmaf(a.hi, b.lo, e);
-  e = fmaf(a.lo, b.hi, e);
-  return fast_two_sum(p, e);
-}
-
-__device__ __forceinline__ float dw_to_float(dw a) { return a.hi + a.lo; }
 
 __device__ __forceinline__ dw dw_from_double(double x) {
   const float hi = __double2float_rn(x);
@@ -166,16 +154,9 @@ struct residual_acc {
   __device__ __forceinline__ float value_f() const { return hi + lo; }
 };
 
-__device__ __forceinline__ dw dw_load(const float2* p) {
-  const float2 v = *p;
-  return dw{v.x, v.y};
-}
-
 __device__ __forceinline__ dw dw_ldg(const float2* p) {
   const float2 v = __ldg(p);
   return dw{v.x, v.y};
 }
-
-__device__ __forceinline__ void dw_store(float2* p, dw a) { *p = make_float2(a.hi, a.lo); }
 
 }  // namespace gbmg

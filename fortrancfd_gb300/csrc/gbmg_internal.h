@@ -302,7 +302,6 @@ int sum_blocks(size_t n, const ReduceScratch& R);  // its blocks
 // y = x - result[slot]/n ; result[slot2] <- sum y^2 (slot2 < 0: no norm)
 void launch_shift_by_mean(cudaStream_t s, const double* x, double* y, size_t n,
                           const ReduceScratch& R, int slot, int slot2);
-void launch_add_float(cudaStream_t s, double* p, const float* e, size_t n);
 // Flexible-CG passes (pcg.cu).  Slots: kSlotSum = sum z, kSlotDot = r.z,
 // kSlotDot+1 = r.z_old, kSlotDot2 = d.(A d), kSlotDot2+1 = r.z of the previous
 // iteration, kSlotNorm = |r|^2.

@@ -315,6 +315,13 @@ inline long long ls_outside_bits(double ls_wid) {
   return (long long)idiv_bits(ls_wid * (1.0 - 1e-12) * (1.0 + 1e-15));
 }
 
+// whether |b| lies in 2^-60..2^60, so that quotients of ordinary values by it stay
+// in the normal range
+inline bool divisor_ok(double b) {
+  const double m = b < 0 ? -b : b;
+  return m >= 0x1p-60 && m <= 0x1p60;
+}
+
 // ---- division by a constant known on the host --------------------------------
 // kDivExact: h is a power of two, x / h adds to the exponent.
 // kDivPair:  x / h = fma(x, y, x yl) with y + yl = 1/h to 106 bits, two FP64
@@ -325,8 +332,12 @@ inline long long ls_outside_bits(double ls_wid) {
 //            only go wrong for an x whose quotient lies that close to a
 //            midpoint; const_div finds all such x (at most a few, from a
 //            linear congruence) and tests them.
-// kDivKnown: some such x fails (or h is negative): Markstein's two correction
-//            steps (fdiv.cuh), five operations.
+// kDivKnown: some such x fails (or h is negative): with y = 1/h rounded to nearest,
+//            q0 = x y is within two ulps of the quotient, one correction by the
+//            remainder, q1 = q0 + (x - h q0) y, brings it within one, and a second
+//            one rounds correctly (P. Markstein, "Computation of elementary
+//            functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
+//            34(1), 1990): five operations.
 // kDivIeee:  h out of range: the division itself.
 enum : int { kDivIeee = 0, kDivExact = 1, kDivPair = 2, kDivKnown = 3 };
 
@@ -376,7 +387,7 @@ inline ConstDiv const_div_i(double h) {
 
 inline ConstDiv const_div(double h) {
   ConstDiv c = const_div_i(h);
-  if (c.mode == kDivExact || !(std::fabs(h) >= 0x1p-60 && std::fabs(h) <= 0x1p60)) return c;
+  if (c.mode == kDivExact || !divisor_ok(h)) return c;
   int ex;
   c.mode = kDivKnown;
   if (!(h > 0)) return c;

@@ -383,11 +383,6 @@ __global__ void __launch_bounds__(kRedThreads) k_shift_by_mean(const double* __r
   if (slot2 >= 0) grid_sum_finish<1>(acc, R, slot2);
 }
 
-__global__ void k_add_float(double* p, const float* __restrict__ e, size_t n) {
-  stride4(n, [&](size_t q) { return make_double2(p[q], (double)e[q]); },
-          [&](size_t q, double2 v) { p[q] = v.x + v.y; });
-}
-
 __global__ void k_d2f(const double* __restrict__ a, float* b, size_t n) {
   stride4(n, [&](size_t q) { return a[q]; }, [&](size_t q, double v) { b[q] = (float)v; });
 }
@@ -587,10 +582,6 @@ void launch_shift_by_mean(cudaStream_t s, const double* x, double* y, size_t n,
                           const ReduceScratch& R, int slot, int slot2) {
   const unsigned b = std::min<unsigned>(stride_blocks(n), (unsigned)R.max_blocks);
   k_shift_by_mean<<<b, kRedThreads, 0, s>>>(x, y, n, R, slot, slot2);
-}
-
-void launch_add_float(cudaStream_t s, double* p, const float* e, size_t n) {
-  k_add_float<<<stride_blocks(n) * 2, kRedThreads, 0, s>>>(p, e, n);
 }
 
 void launch_double_to_float(cudaStream_t s, const double* a, float* b, size_t n) {

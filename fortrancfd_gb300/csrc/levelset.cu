@@ -39,7 +39,6 @@
 #include <string>
 
 #include "gbmg.h"
-#include "fdiv.cuh"
 #include "gbmg_internal.h"
 #include "idiv.h"
 

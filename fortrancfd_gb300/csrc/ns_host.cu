@@ -14,7 +14,6 @@
 #include <string>
 #include <vector>
 
-#include "fdiv.cuh"
 #include "handle.h"
 
 using namespace gbmg;
@@ -109,11 +108,11 @@ int ns_prepare(gbmg_handle* h, const gbmg_ns_params* prm, const gbmg_ns_fields* 
   for (int i = 0; i < 3; ++i) {
     a.h[i] = const_div_i(hs[i]);
     a.h2[i] = const_div_i(hs[i] * hs[i]);
-    if (!fdiv_divisor_ok(hs[i])) a.band = 0;
+    if (!divisor_ok(hs[i])) a.band = 0;
   }
   a.rediv = const_div_i(prm->re);
-  if (!fdiv_divisor_ok(prm->re) || !(std::fabs(prm->mu_12) < 0x1p60) ||
-      !(std::fabs(prm->btn_sf) < 0x1p60) || (prm->btn_sf != 0 && !fdiv_divisor_ok(prm->we)))
+  if (!divisor_ok(prm->re) || !(std::fabs(prm->mu_12) < 0x1p60) ||
+      !(std::fabs(prm->btn_sf) < 0x1p60) || (prm->btn_sf != 0 && !divisor_ok(prm->we)))
     a.band = 0;
   a.scheme = prm->adv_scheme;
   if (a.scheme != 0 && a.scheme != 1) {

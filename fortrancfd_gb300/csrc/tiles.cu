@@ -21,7 +21,7 @@
 // wrote them from the cycle.
 //
 // Time per cycle, separate launches -> tiles: FP64 128^2 79.6 -> 49.3 us, 512^2
-// 175 -> 119; mixed 128 x 256 53.2 -> 33.0, 512^2 77.5 -> 47.2, 1024^2 (from level
+// 175 -> 119; mixed 128 x 256 53.2 -> 31.0, 512^2 77.5 -> 47.2, 1024^2 (from level
 // 512^2 down) 110.6 -> 83.6.  Tiles of 16 x 8 cells with 256 threads: more
 // threads than cells of a colour, since a phase is one chain of latencies (FP64
 // 128^2 with 128 threads 63, with 16 x 16 and 32 x 16 tiles 59 and 63 us).  The
@@ -243,10 +243,13 @@ void tile_pick(cudaStream_t s, const LevelView<T>& F, const LevelView<T>& C, con
 
 // 2D levels of at most 512 x 512 cells, both axes halved (so that the halo is made
 // of whole coarse cells and rows are even).  Larger levels are bound by their
-// arithmetic and traffic, which the halos double: the split level of 1024^2 makes
-// its FP32 cycle 97 us in tiles, 84 in separate launches.  3D halos cost more: 32^3
-// in tiles of 8^3 leaves the 256^3 cycle as it was (463.5 for 465.6 us), 64^3 in
-// tiles of 16 x 8 x 8, a sweep a launch, makes it 474.
+// arithmetic and traffic, which the halos double.  Time of a solve per cycle with
+// the finest level in separate launches -> in tiles (all below it in tiles): 1024^2 FP64 237 ->
+// 272 us, colour-split FP32 89.5 -> 102.8, FP32 with stored coefficients 96.0 -> 96.0;
+// 768^2 178.5 -> 187.1, 74.4 -> 73.5, 74.3 -> 74.1; below that tiles are ahead (768 x
+// 512 177 -> 145, 70.4 -> 64.6, 68.3 -> 68.3), so the line is on the safe side.  3D
+// halos cost more: 32^3 in tiles of 8^3 leaves the 256^3 cycle as it was (463.5 for
+// 465.6 us), 64^3 in tiles of 16 x 8 x 8, a sweep a launch, makes it 474.
 bool tile_level(int nx, int ny, int nz, int fx, int fy) {
   return nz == 1 && fx == 2 && fy == 2 && (size_t)nx * ny <= (size_t)1 << 18;
 }
