@@ -20,13 +20,13 @@
 // wait for the preceding kernel: ordinary launches separate the set-up that
 // wrote them from the cycle.
 //
-// Time per cycle, separate launches -> tiles: FP64 128^2 79.6 -> 49.3 us, 512^2
-// 175 -> 119; mixed 128 x 256 53.2 -> 31.0, 512^2 77.5 -> 47.2, 1024^2 (from level
-// 512^2 down) 110.6 -> 83.6.  Tiles of 16 x 8 cells with 256 threads: more
-// threads than cells of a colour, since a phase is one chain of latencies (FP64
-// 128^2 with 128 threads 63, with 16 x 16 and 32 x 16 tiles 59 and 63 us).  The
-// split level takes 32 x 16 with 512 (512^2: 47.2 us, with 16 x 8 52.2): its blocks
-// also form their coefficients.
+// Time of a solve per cycle, separate launches -> tiles: FP64 128^2 75.1 -> 48.4 us,
+// 512^2 166 -> 119; mixed 128 x 256 52.9 -> 35.4, 512^2 79.5 -> 50.5, 1024^2 (from level
+// 512^2 down) 114.5 -> 89.5.  Tiles of 16 x 8 cells with 256 threads: more threads than
+// cells of a colour, since a phase is one chain of latencies (FP64 128^2 a third slower
+// with 128 threads, a fifth to a third with 16 x 16 and 32 x 16 tiles).  The split level
+// takes 32 x 16 with 512 (16 x 8 is a tenth slower): its blocks also form their
+// coefficients.
 #include <algorithm>
 
 #include "gbmg_internal.h"

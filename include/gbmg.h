@@ -435,14 +435,18 @@ int64_t gbmg_kernel_launches(gbmg_handle* h);
  * 75,167-168).  With profiling on, graphs are bypassed and every launch is
  * bracketed by CUDA events on the handle's stream.  Classes: GBMG_PROF_*. */
 enum {
-  GBMG_PROF_SMOOTH_FINE = 0,   /* smoother on the finest level */
-  GBMG_PROF_SMOOTH_COARSE = 1, /* smoother on the other levels */
+  /* Smoother launches.  A 2D level of at most 512 x 512 cells restricts and prolongs
+   * inside them (one launch holds two sweeps and the transfer), so its transfers are
+   * timed and counted here and not under RESTRICT and PROLONG. */
+  GBMG_PROF_SMOOTH_FINE = 0,   /* on the finest level */
+  GBMG_PROF_SMOOTH_COARSE = 1, /* on the other levels above the bottom block */
   GBMG_PROF_RESTRICT_FINE = 2, /* residual + restriction out of the finest level */
   GBMG_PROF_RESTRICT_COARSE = 3,
   GBMG_PROF_PROLONG_FINE = 4,  /* prolongation + correction into the finest level */
   GBMG_PROF_PROLONG_COARSE = 5,
-  GBMG_PROF_COARSE_SOLVE = 6,
-  GBMG_PROF_RESIDUAL = 7,      /* FP64 (or double-word) residual + norm on the finest level */
+  GBMG_PROF_COARSE_SOLVE = 6,  /* the bottom block: the smallest levels and the dense solve */
+  GBMG_PROF_RESIDUAL = 7,      /* FP64 (or double-word) residual + norm on the finest level,
+                                  Krylov matrix product */
   GBMG_PROF_VECTOR = 8,        /* mean projection, p += e, Krylov vector kernels */
   GBMG_PROF_SETUP = 9,         /* coefficients, coarse operators, coarse inverse */
   GBMG_PROF_CERTIFY = 10,      /* native FP64 residual after a mixed-precision solve */
