@@ -204,7 +204,7 @@ void tile_leg(gbmg_handle* h, int l, bool up, int first, bool zero) {
     else if (!up && start && zero) e = last ? kTileZeroRestrict : kTileZero;
     else if (!up && last) e = kTileRestrict;
     const int to = left & 1 ? 0 : 1;
-    LAUNCH(h, cs, launch_tile<T>(h->stream, F, C, buf[1 - to], buf[to], m, first, e));
+    LAUNCH(h, cs, launch_tile<T>(h->stream, F, C, buf[1 - to], buf[to], m, first, e, zero));
   }
 }
 
@@ -225,8 +225,9 @@ int enqueue_vcycle(gbmg_handle* h, bool reverse_post, bool zero_fine) {
       continue;
     }
     for (int it = 0; it < h->prm.nu1; ++it) sweep<T>(h, l, 0, it == 0 && zero);
+    // (the half restriction where the unknown is a correction, see restrict_cell)
     LAUNCH(h, l == 0 ? GBMG_PROF_RESTRICT_FINE : GBMG_PROF_RESTRICT_COARSE,
-           launch_restrict<T>(s, view_next<T>(h->lv[l]), view<T>(h->lv[l + 1]), !pre, pre));
+           launch_restrict<T>(s, view_next<T>(h->lv[l]), view<T>(h->lv[l + 1]), !pre, pre && zero));
   }
   if (h->sub_lc < L) {
     LAUNCH(h, GBMG_PROF_COARSE_SOLVE, launch_subcycle<T>(s, make_subcycle<T>(h, reverse_post)));

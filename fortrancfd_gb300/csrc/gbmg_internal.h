@@ -150,10 +150,11 @@ enum TileEnds { kTilePlain, kTileZero, kTileRestrict, kTileZeroRestrict, kTilePr
 constexpr int kTileSweeps = 2;
 // whether a level may run in tiles
 bool tile_level(int nx, int ny, int nz, int fx, int fy);
-// `sweeps` red-black sweeps of level F, in -> out (distinct arrays); C: the next level
+// `sweeps` red-black sweeps of level F, in -> out (distinct arrays); C: the next
+// level; half (FP64): as launch_restrict
 template <typename T>
 void launch_tile(cudaStream_t s, const LevelView<T>& F, const LevelView<T>& C, const T* in, T* out,
-                 int sweeps, int first, TileEnds e);
+                 int sweeps, int first, TileEnds e, bool half);
 
 // ---- launchers (kernels_mg.cu) ---------------------------------------------
 // zero_guess: the level's current values are taken as zero (first colour of
@@ -162,7 +163,7 @@ template <typename T>
 void launch_smooth(cudaStream_t s, const LevelView<T>& L, int color, bool zero_guess = false);
 // zero_sol: also set the coarse unknown to zero (not needed when its first
 // sweep starts from a zero guess); half (FP64): the fine level's last colour
-// launch relaxed colour 1, whose residual is taken as zero
+// launch relaxed colour 1, whose residual is taken as zero (restrict_cell)
 template <typename T>
 void launch_restrict(cudaStream_t s, const LevelView<T>& F, const LevelView<T>& C, bool zero_sol,
                      bool half);

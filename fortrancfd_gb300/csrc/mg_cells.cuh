@@ -187,12 +187,17 @@ __device__ __forceinline__ void smooth_cell(const LevelView<T>& L, int i, int j,
 // (src - A sol) on the fine level; coarse sol = 0.  One thread per coarse
 // cell; the children are summed in the order z, y, x (the oracle's).
 // kHalf: the level's last colour launch relaxed the cells of colour 1, whose
-// residual is therefore zero up to the rounding of the update: only the
-// children of colour 0 are visited (half the arithmetic; 256^3 FP64, bound by
-// the FP64 pipe, 484 -> 261 us), with the diagonal read back where it is stored
-// (9 operations a child for 14: 164 us).  FP64 only: in FP32 that rounding reaches 1e-4
-// of the residual within a correction's four cycles, enough to move the mixed
-// loop's schedule and with it the error left at the tolerance.
+// residual is therefore zero up to the rounding of the update: only the children of
+// colour 0 are visited (half the arithmetic; 256^3 FP64, bound by the FP64 pipe, 484
+// -> 261 us), with the diagonal read back where it is stored (9 operations a child
+// for 14: 164 us, all children 300).  Only where the unknown is a correction: that
+// rounding is relative to the unknown, and left out of the mean it acts as a source.
+// On the finest level of the stationary FP64 cycle, where the unknown is p, the
+// residual that the solve can reach rose with the density ratio and the size (one
+// bubble: 64^3 at 1e4 1.5-fold, 128^3 and 256^3 at 1e5 3-fold, none at 1000; 2D 320 x
+// 512 at 1e4 1.4-fold), so that level takes all children (256^3 solve 41.7 -> 44.4 ms).  FP64 only: in
+// FP32 that rounding reaches 1e-4 of the residual within a correction's four cycles,
+// enough to move the mixed loop's schedule and with it the error left at the tolerance.
 template <typename T, bool kRho, bool kHalf, bool kCg = false>
 __device__ __forceinline__ void restrict_cell(const LevelView<T>& F, const LevelView<T>& C, int I,
                                               int J, int K, int zero_sol) {
@@ -257,25 +262,49 @@ __device__ __forceinline__ void restrict_cell(const LevelView<T>& F, const Level
           czm = *reinterpret_cast<const V2*>(F.cz + q);
           czp = zr ? *reinterpret_cast<const V2*>(F.cz + q + sz) : zero2;
         }
+        // the diagonal read back where it is stored (FP64; the same sum)
+        const bool stored = sizeof(T) == 8 && F.diag;
+        V2 dg = zero2;
+        if (stored) dg = *reinterpret_cast<const V2*>(F.diag + q);
         // child x = i0: neighbours x- (pl, cx[i0]), x+ (p.y, cx[i0+1]); same order as stencil()
         {
-          T s = T(0), d = T(0), c;
-          if (xl) { c = cxp.x; s += c * pl; d += c; }
-          c = cxp.y; s += c * p.y; d += c;
-          if (yl) { c = cym.x; s += c * pym.x; d += c; }
-          if (yr) { c = cyp.x; s += c * pyp.x; d += c; }
-          if (zl) { c = czm.x; s += c * pzm.x; d += c; }
-          if (zr) { c = czp.x; s += c * pzp.x; d += c; }
+          T s = T(0), d = T(0);
+          if (xl) s += cxp.x * pl;
+          s += cxp.y * p.y;
+          if (yl) s += cym.x * pym.x;
+          if (yr) s += cyp.x * pyp.x;
+          if (zl) s += czm.x * pzm.x;
+          if (zr) s += czp.x * pzp.x;
+          if (stored) {
+            d = dg.x;
+          } else {
+            if (xl) d += cxp.x;
+            d += cxp.y;
+            if (yl) d += cym.x;
+            if (yr) d += cyp.x;
+            if (zl) d += czm.x;
+            if (zr) d += czp.x;
+          }
           acc += b.x - (s - d * p.x);
         }
         {
-          T s = T(0), d = T(0), c;
-          c = cxp.y; s += c * p.x; d += c;
-          if (xr) { c = cxr; s += c * pr; d += c; }
-          if (yl) { c = cym.y; s += c * pym.y; d += c; }
-          if (yr) { c = cyp.y; s += c * pyp.y; d += c; }
-          if (zl) { c = czm.y; s += c * pzm.y; d += c; }
-          if (zr) { c = czp.y; s += c * pzp.y; d += c; }
+          T s = T(0), d = T(0);
+          s += cxp.y * p.x;
+          if (xr) s += cxr * pr;
+          if (yl) s += cym.y * pym.y;
+          if (yr) s += cyp.y * pyp.y;
+          if (zl) s += czm.y * pzm.y;
+          if (zr) s += czp.y * pzp.y;
+          if (stored) {
+            d = dg.y;
+          } else {
+            d += cxp.y;
+            if (xr) d += cxr;
+            if (yl) d += cym.y;
+            if (yr) d += cyp.y;
+            if (zl) d += czm.y;
+            if (zr) d += czp.y;
+          }
           acc += b.y - (s - d * p.y);
         }
       }

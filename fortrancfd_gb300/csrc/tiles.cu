@@ -38,13 +38,14 @@ namespace gbmg {
 namespace {
 
 // kM: colours relaxed; kRes: followed by the restriction; kSplit: the colour-split
-// finest level, coefficients from the density
-template <typename T, int kTx, int kTy, int kM, bool kRes, int kThr, bool kSplit = false>
+// finest level, coefficients from the density; kHalf (FP64): restrict_cell's half
+template <typename T, int kTx, int kTy, int kM, bool kRes, int kThr, bool kSplit = false,
+          bool kHalf = false>
 struct Tile {
   using Value = T;
   static constexpr int H = kM + (kRes ? 1 : 0);  // even in front of a prolongation
   static constexpr int TX = kTx, TY = kTy, M = kM, THREADS = kThr;
-  static constexpr bool RES = kRes, SPLIT = kSplit, IDIAG = sizeof(T) == 8;
+  static constexpr bool RES = kRes, SPLIT = kSplit, HALF = kHalf, IDIAG = sizeof(T) == 8;
   static constexpr int LX = kTx + 2 * H, LY = kTy + 2 * H, N = LX * LY;
   static constexpr size_t BYTES = (size_t)(IDIAG ? 5 : 4) * N * sizeof(T);
 };
@@ -186,13 +187,13 @@ __global__ void __launch_bounds__(P::THREADS)
     if (inside(x, y)) sol_out[at(x, y)] = sol[(ty + H) * LX + tx + H];
   }
   if (!P::RES) return;
-  // residuals in place of the right-hand side, which only their own cells read.
-  // FP64: the children of the colour relaxed last (1) have none (restrict_cell)
-  constexpr int SX = P::IDIAG ? 2 : 1, RX = P::TX / SX;
+  // residuals in place of the right-hand side, which only their own cells read
+  // (HALF: the children of the colour relaxed last, 1, have none)
+  constexpr int SX = P::HALF ? 2 : 1, RX = P::TX / SX;
   for (int t = tid; t < RX * P::TY; t += P::THREADS) {
     const int y = t / RX;
     int x = t - y * RX;
-    if (P::IDIAG) x = 2 * x + (y & 1);
+    if (P::HALF) x = 2 * x + (y & 1);
     const int q = (y + H) * LX + x + H;
     T s, d;
     neighbours(q, s, d);
@@ -211,7 +212,7 @@ __global__ void __launch_bounds__(P::THREADS)
     for (int dy = 0; dy < 2; ++dy)
 #pragma unroll
       for (int dx = 0; dx < 2; ++dx)
-        if (!P::IDIAG || dx == dy) acc += r[dy * LX + dx];
+        if (!P::HALF || dx == dy) acc += r[dy * LX + dx];
     C.src[(size_t)J * C.nx + I] = acc * T(0.25);
   }
 }
@@ -225,7 +226,7 @@ void tile_launch(cudaStream_t s, const LevelView<typename P::Value>& F,
   launch_pdl(k_tile<P>, grd, dim3(P::THREADS), P::BYTES, s, F, C, in, out, A);
 }
 
-template <typename T, bool R>
+template <typename T, bool R, bool kHalf>
 void tile_pick(cudaStream_t s, const LevelView<T>& F, const LevelView<T>& C, const T* in, T* out,
                int sweeps, const TileArgs& A) {
   if constexpr (sizeof(T) == 4) {
@@ -235,8 +236,8 @@ void tile_pick(cudaStream_t s, const LevelView<T>& F, const LevelView<T>& C, con
       return;
     }
   }
-  if (sweeps == 2) tile_launch<Tile<T, 16, 8, 4, R, 256>>(s, F, C, in, out, A);
-  else tile_launch<Tile<T, 16, 8, 2, R, 256>>(s, F, C, in, out, A);
+  if (sweeps == 2) tile_launch<Tile<T, 16, 8, 4, R, 256, false, kHalf>>(s, F, C, in, out, A);
+  else tile_launch<Tile<T, 16, 8, 2, R, 256, false, kHalf>>(s, F, C, in, out, A);
 }
 
 }  // namespace
@@ -256,15 +257,20 @@ bool tile_level(int nx, int ny, int nz, int fx, int fy) {
 
 template <typename T>
 void launch_tile(cudaStream_t s, const LevelView<T>& F, const LevelView<T>& C, const T* in, T* out,
-                 int sweeps, int first, TileEnds e) {
+                 int sweeps, int first, TileEnds e, bool half) {
   const TileArgs A{first, e == kTileZero || e == kTileZeroRestrict, e == kTileProlong};
-  if (e == kTileRestrict || e == kTileZeroRestrict) tile_pick<T, true>(s, F, C, in, out, sweeps, A);
-  else tile_pick<T, false>(s, F, C, in, out, sweeps, A);
+  if (e == kTileRestrict || e == kTileZeroRestrict) {
+    if constexpr (sizeof(T) == 8)
+      if (half) return tile_pick<T, true, true>(s, F, C, in, out, sweeps, A);
+    tile_pick<T, true, false>(s, F, C, in, out, sweeps, A);
+  } else {
+    tile_pick<T, false, false>(s, F, C, in, out, sweeps, A);
+  }
 }
 
 template void launch_tile<float>(cudaStream_t, const LevelView<float>&, const LevelView<float>&,
-                                 const float*, float*, int, int, TileEnds);
+                                 const float*, float*, int, int, TileEnds, bool);
 template void launch_tile<double>(cudaStream_t, const LevelView<double>&, const LevelView<double>&,
-                                  const double*, double*, int, int, TileEnds);
+                                  const double*, double*, int, int, TileEnds, bool);
 
 }  // namespace gbmg
