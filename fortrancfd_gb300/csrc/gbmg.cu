@@ -1031,9 +1031,9 @@ int gm_vcycle(gbmg_handle* h) {
 // Saad's FGMRES): the residual norm falls monotonically, where conjugate
 // gradients can first raise it many-fold on a smooth right-hand side (the
 // adjoint of a smooth objective).  Per Arnoldi step: z_j = M v_j (the V-cycle one
-// captured graph) and w = A z_j, classical Gram-Schmidt with a second pass only
-// when the first removed most of w, decided on the device, one copy of the
-// coefficients to the host for the Givens rotations, and w scaled into v_{j+1}
+// captured graph) and w = A z_j, classical Gram-Schmidt with a second pass when the
+// first removed most of w (nearly every step, see krylov.cu), decided on the device,
+// one copy of the coefficients to the host for the Givens rotations, and w scaled into v_{j+1}
 // meanwhile.  Where the last reduction of the residual does not promise that this
 // step is the last, the next step's V-cycle is launched before the host waits: it
 // reads the device's data alone, and the GPU has work while the host rotates (a
@@ -1076,7 +1076,7 @@ int fgmres(gbmg_handle* h, double tol, double scale, double* rel_io, int* cycles
       if (!ahead) GB_TRY(gm_vcycle(h));
       LAUNCH(h, VC, launch_gm_z(s, z, zj, h->red.result + kSlotSum));
       LAUNCH(h, GBMG_PROF_RESIDUAL, launch_apply_diag(s, v64(f), h->kdiag, zj, w, h->red, -1, false));
-      // classical Gram-Schmidt; a second pass only when the first removed most
+      // classical Gram-Schmidt; a second pass when the first removed most
       // of w (|w| fell below 0.7 of its length: "twice is enough")
       LAUNCH(h, VC, launch_gm_dots(s, h->gmV, ld, j + 1, w, n, h->gmPart, h1, nullptr));
       LAUNCH(h, VC, launch_gm_update(s, w, h->gmV, ld, h1, j + 1, -1.0, n, h->gmPart,

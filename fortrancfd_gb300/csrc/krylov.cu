@@ -12,9 +12,11 @@
 // everything beside the one operation is kept off it: w is read once for all
 // vectors, and the sums of a warp are folded together (9 additions for eight
 // sums, 40 one by one, which with four elements per thread were more than the
-// products).  1024^2, 12 vectors on average: products 33 + 4 us, mean 18, v 8;
-// before, 65 + 2 x 31 (a pass per vector, separate norms), 31 with two conversions,
-// and two copies of 6.
+// products).  Both passes run twice in nearly every step: with a good preconditioner
+// A M v is nearly v, and the first one takes most of w away (1024^2: 45 of 45 steps,
+// 128^3: 15 of 15).  1024^2 in the stream of a step: products 26, 34 and 42 us with up
+// to 7, 11 and 15 vectors, the update 48 on average, z 6, v 7, the mean 10; with a pass per
+// vector, separate norms and two conversions 65 + 2 x 31 + 31 and two copies of 6.
 // The sums keep a fixed order (thread: stride of the grid; warp: halves;
 // block: warps in order; then blocks the same way), whatever is summed together.
 // The basis is one array of vectors of n doubles

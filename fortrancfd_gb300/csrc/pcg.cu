@@ -13,9 +13,10 @@
 // then the residual kernel).
 // Recomputing it always, with one pass per vector operation, read and wrote
 // 208 bytes and issued 37 FP64 operations per cell and iteration: 10.6 of the 13.7
-// ms of a 512^3 iteration.  These passes move 152 bytes with 16 operations
-// (the FP64 pipe runs 2 lanes per clock and SM, so an operation per cell costs
-// as much as 11 bytes): 512^3, 47 iterations, 645 ms before.
+// ms of a 512^3 iteration.  These passes move 156 bytes with 15 operations (mixed;
+// FP64 160 with 16; the FP64 pipe runs 2 lanes per clock and SM, so an operation
+// per cell costs as much as 11 bytes); with b - A p in place of the recursion 188 with
+// 28 (FP64 184 with 29).
 // z is read straight from the V-cycle's result: FP64, FP32, or FP32 in the
 // colour-split layout (cell q in half (i+j+k)&1 at q/2).  All passes work on
 // pairs of cells (2m, 2m+1), which share a row when nx is even.

@@ -11,7 +11,7 @@
 // summed in z, y, x order, slopes added x, y, z), so the cycle is the same cycle.
 //
 // One block is bound by the instructions and the latency of its phases (from
-// 16^3 down 68,000 cycles at first, 35 us), so:
+// 16^3 down it had been 68,000 cycles, 35 us), so:
 //   - the coefficients and matrices, which no kernel of the cycle writes, are
 //     staged before the wait for the preceding kernel;
 //   - arrays are padded with zeros by a plane (2D: a row) and a wall's
